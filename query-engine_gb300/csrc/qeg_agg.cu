@@ -2324,17 +2324,18 @@ void AggState::finish(uint64_t* nrows_out) {
   }
   const uint64_t out_cap = (mode == 0) ? 1 : std::max<uint64_t>(inserted + 2 + ntails, 1);
   const int ncolsout = static_cast<int>(keys.size() + aggs.size());
-  out_vals.clear();
-  out_valid.clear();
-  out_vals.resize(ncolsout);
-  out_valid.resize(ncolsout);
+  // One allocation for all output columns.
+  const size_t val_bytes = (out_cap * 8 + 255) / 256 * 256, ok_bytes = (out_cap + 255) / 256 * 256;
+  out_slab.alloc((val_bytes + ok_bytes) * ncolsout, ctx->stream);
+  out_vals.assign(ncolsout, nullptr);
+  out_valid.assign(ncolsout, nullptr);
   FinK F{};
   F.naggs = static_cast<int>(aggs.size());
   for (int c = 0; c < ncolsout; ++c) {
-    out_vals[c].alloc(out_cap * 8, ctx->stream);
-    out_valid[c].alloc(out_cap, ctx->stream);
-    F.vals[c] = out_vals[c].get();
-    F.valid[c] = out_valid[c].get<uint8_t>();
+    out_vals[c] = out_slab.get<uint8_t>() + val_bytes * c;
+    out_valid[c] = out_slab.get<uint8_t>() + val_bytes * ncolsout + ok_bytes * c;
+    F.vals[c] = out_vals[c];
+    F.valid[c] = out_valid[c];
     F.rtype[c] = rtypes[c];
   }
   for (size_t a = 0; a < aggs.size(); ++a) {
@@ -2342,9 +2343,8 @@ void AggState::finish(uint64_t* nrows_out) {
     F.vfield[a] = vfield[a];
     F.nfield[a] = nfield[a];
   }
-  DevBuf cnt(8, ctx->stream);
-  QEG_CUDA(cudaMemsetAsync(cnt.get(), 0, 8, ctx->stream));
-  F.out_count = cnt.get<unsigned long long>();
+  F.out_count = counters.get<unsigned long long>() + 5;
+  QEG_CUDA(cudaMemsetAsync(F.out_count, 0, 8, ctx->stream));
   F.out_cap = out_cap;
   F.packed_width = packed ? bucket_width : 0;
   AggK P = kparams_base();
@@ -2368,11 +2368,7 @@ void AggState::finish(uint64_t* nrows_out) {
   else finalize_kernel<2><<<g, 1024, 0, ctx->stream>>>(P, F);
   ctx->launches++;
   QEG_CUDA(cudaGetLastError());
-  unsigned long long n = 0;
-  QEG_CUDA(cudaMemcpyAsync(&n, cnt.get(), 8, cudaMemcpyDeviceToHost, ctx->stream));
-  QEG_CUDA(cudaStreamSynchronize(ctx->stream));
-  check_device_error(ctx);
-  nout = n;
+  read_words_and_error(ctx, F.out_count, 1, &nout);  // one synchronisation
   finished = true;
   *nrows_out = nout;
 }
@@ -2381,8 +2377,10 @@ void AggState::fetch(uint64_t first, uint64_t count, const qeg_out_column* outs)
   require(finished, "fetch() before finish()");
   require(first <= nout && count <= nout - first, "fetch range outside the result");
   require(outs != nullptr, "outs is NULL");
+  std::vector<FetchCol> cols;
   for (size_t c = 0; c < out_vals.size(); ++c)
-    fetch_column(ctx, out_vals[c].get(), out_valid[c].get<uint8_t>(), type_width(rtypes[c]), first, count, outs[c]);
+    cols.push_back(FetchCol{out_vals[c], out_valid[c], type_width(rtypes[c])});
+  fetch_columns(ctx, cols.data(), static_cast<int>(cols.size()), first, count, outs);
 }
 
 }  // namespace qeg

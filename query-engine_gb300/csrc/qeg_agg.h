@@ -189,7 +189,8 @@ struct AggState {
 
   bool finished = false;
   uint64_t nout = 0;
-  std::vector<DevBuf> out_vals, out_valid;
+  DevBuf out_slab;  // every output column's values, then every column's valid bytes
+  std::vector<uint8_t*> out_vals, out_valid;
 
   void plan(const int32_t* col_types, int ncols, const uint32_t* key_cols, int nk, const qeg_agg_spec* aggs,
             int na);

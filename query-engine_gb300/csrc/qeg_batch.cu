@@ -751,9 +751,10 @@ qeg_status qeg_batch_fetch(qeg_batch* b, uint32_t query, const qeg_out_column* o
     }
     Round& R = S.rounds[S.where_round[query]];
     const BatchQ& Q = R.qs[S.where_local[query]];
+    std::vector<FetchCol> cols;
     for (size_t c = 0; c < S.plan.rtypes.size(); ++c)
-      fetch_column(ctx, R.out_vals[c].get(), R.out_valid[c].get<uint8_t>(), type_width(S.plan.rtypes[c]),
-                   Q.out_off, S.group_counts[query], outs[c]);
+      cols.push_back(FetchCol{R.out_vals[c].get(), R.out_valid[c].get<uint8_t>(), type_width(S.plan.rtypes[c])});
+    fetch_columns(ctx, cols.data(), static_cast<int>(cols.size()), Q.out_off, S.group_counts[query], outs);
   });
 }
 

@@ -9,22 +9,79 @@ namespace qeg {
 
 namespace {
 
-// Packs one byte per row (1 = valid) into 64-bit validity words, LSB-first
-// (core/validity.h:21-40). Padding bits of the last word are set to 1, the
-// reference's canonical representation (core/validity.h:53-58).
-__global__ void pack_validity_kernel(const uint8_t* __restrict__ valid, uint64_t n,
-                                     uint64_t* __restrict__ words, uint32_t* __restrict__ any_null) {
+// Output columns of one fetch (qeg::fetch_columns): at most every key and
+// aggregate of a GROUP BY.
+struct FetchK {
+  const uint8_t* vals[kMaxFetchCols];
+  const uint8_t* valid[kMaxFetchCols];
+  uint8_t* dst[kMaxFetchCols];      // nullptr: the values go by a copy of their own, or are not wanted
+  uint64_t* words[kMaxFetchCols];   // nullptr: no validity words wanted
+  uint32_t* null_flags;          // page-locked host memory, one per column, zeroed: 1 when it holds a NULL
+  uint64_t count;
+  uint8_t width[kMaxFetchCols];
+  uint8_t unit[kMaxFetchCols];  // bytes per copied element: 16, or at most the width, as both ends are aligned
+};
+
+// Copies `n` elements of type T.
+template <typename T>
+__device__ __forceinline__ void copy_elems(uint8_t* dst, const uint8_t* src, uint64_t n, uint64_t i, uint64_t step) {
+#pragma unroll 4
+  for (; i < n; i += step) reinterpret_cast<T*>(dst)[i] = __ldg(reinterpret_cast<const T*>(src) + i);
+}
+
+// One launch for a whole fetch, blockIdx.y = column: packs one byte per row (1
+// = valid) into 64-bit validity words, LSB-first (core/validity.h:21-40;
+// padding bits of the last word set, core/validity.h:53-58), and copies the
+// values. Small results are bound by the launch and the synchronisation that
+// follows, so the columns share both; large ones by the copy (16-byte loads
+// and stores where both ends allow). Per column a copy, an allocation, a
+// memset, a pack kernel, two more copies and a synchronisation took 45-55 us
+// (fetch of 6 small columns: 290 us into device buffers, 330 us into host
+// arrays); packing with one thread per word read the valid bytes 64 apart
+// (35 us per 16.6M-row column), a warp per word reads them side by side.
+__global__ void __launch_bounds__(256) fetch_kernel(const FetchK P) {
+  const int c = blockIdx.y;
+  const uint64_t n = P.count;
+  const unsigned lane = threadIdx.x & 31u;
+  uint64_t* words = P.words[c];
+  const uint8_t* valid = P.valid[c];
   const uint64_t nw = (n + 63) / 64;
-  for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nw;
-       w += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t bits = ~0ull;
-    const uint64_t base = w * 64;
-    for (int b = 0; b < 64; ++b) {
-      const uint64_t r = base + b;
-      if (r < n && !valid[r]) bits &= ~(1ull << b);
+  bool nulls = false;
+  constexpr int kU = 4;  // words per warp and step, their loads independent
+  for (uint64_t w0 = (blockIdx.x * 8ull + (threadIdx.x >> 5)) * kU; w0 < nw; w0 += gridDim.x * 8ull * kU) {
+    bool lo[kU], hi[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint64_t r = (w0 + u) * 64 + lane;
+      lo[u] = r >= n || valid[r] != 0;
+      hi[u] = r + 32 >= n || valid[r + 32] != 0;
     }
-    words[w] = bits;
-    if (bits != ~0ull) atomicOr(any_null, 1u);
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint64_t bits = __ballot_sync(0xffffffffu, lo[u]) |
+                            (static_cast<uint64_t>(__ballot_sync(0xffffffffu, hi[u])) << 32);
+      if (w0 + u < nw) {
+        nulls |= bits != ~0ull;
+        if (words && lane == 0) words[w0 + u] = bits;
+      }
+    }
+  }
+  if (nulls && lane == 0) P.null_flags[c] = 1u;
+  uint8_t* dst = P.dst[c];
+  if (!dst) return;
+  const uint8_t* src = P.vals[c];
+  const uint64_t i = blockIdx.x * 256ull + threadIdx.x, step = gridDim.x * 256ull;
+  const uint64_t bytes = n * P.width[c];
+  const int unit = P.unit[c];
+  if (unit == 16) {
+    copy_elems<uint4>(dst, src, bytes / 16, i, step);
+    for (uint64_t b = bytes / 16 * 16 + i; b < bytes; b += step) dst[b] = src[b];
+  } else if (unit == 8) {
+    copy_elems<uint64_t>(dst, src, bytes / 8, i, step);
+  } else if (unit == 4) {
+    copy_elems<uint32_t>(dst, src, bytes / 4, i, step);
+  } else {
+    copy_elems<uint8_t>(dst, src, bytes, i, step);
   }
 }
 
@@ -177,33 +234,95 @@ void raise_device_error(qeg_ctx* ctx, uint32_t e) {
   throw Error(QEG_ERR_CUDA, "device error word " + std::to_string(e));
 }
 
-void fetch_column(qeg_ctx* ctx, const void* dev_vals, const uint8_t* dev_valid, size_t width,
-                  uint64_t first, uint64_t count, const qeg_out_column& out) {
+void fetch_columns(qeg_ctx* ctx, const FetchCol* cols, int ncols, uint64_t first, uint64_t count,
+                   const qeg_out_column* outs) {
+  require(ncols <= kMaxFetchCols, "too many output columns in one fetch");
   if (count == 0) {
-    if (out.all_valid) *out.all_valid = 1;
+    for (int c = 0; c < ncols; ++c)
+      if (outs[c].all_valid) *outs[c].all_valid = 1;
     return;
   }
-  const bool dev_out = is_device_ptr(out.data);
-  const auto kind = dev_out ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-  if (out.data)
-    QEG_CUDA(cudaMemcpyAsync(out.data, static_cast<const uint8_t*>(dev_vals) + first * width,
-                             count * width, kind, ctx->stream));
   const uint64_t nw = (count + 63) / 64;
-  DevBuf words(nw * 8 + 8, ctx->stream);
-  QEG_CUDA(cudaMemsetAsync(words.get<uint8_t>() + nw * 8, 0, 4, ctx->stream));
-  uint32_t* any_null = reinterpret_cast<uint32_t*>(words.get<uint8_t>() + nw * 8);
-  pack_validity_kernel<<<grid_for(ctx, nw, 256, 4), 256, 0, ctx->stream>>>(dev_valid + first, count,
-                                                                         words.get<uint64_t>(), any_null);
+  const size_t flag_bytes = static_cast<size_t>(kMaxFetchCols) * 4;
+  // Where each column's values and words go. Host destinations of a small
+  // result are written by the kernel into the context's page-locked buffer
+  // and copied from there by the host (no device-to-host copy commands); those
+  // of a large one by a copy per array, at the host link's speed when the
+  // destination is page-locked. The line: a copy command into pageable memory
+  // costs about 10 us of host time whatever its size, the host's own copy of
+  // kSmallFetch bytes about as much in all.
+  constexpr size_t kSmallFetch = 256 << 10;
+  // Device words go straight to the caller when they are 8-byte aligned.
+  std::vector<bool> dev_data(ncols), dev_words(ncols), copy_words(ncols);
+  size_t host_bytes = 0;
+  for (int c = 0; c < ncols; ++c) {
+    dev_data[c] = outs[c].data && is_device_ptr(outs[c].data);
+    dev_words[c] = outs[c].validity && is_device_ptr(outs[c].validity);
+    if (outs[c].data && !dev_data[c]) host_bytes += (count * cols[c].width + 15) / 16 * 16;
+    if (outs[c].validity && !dev_words[c]) host_bytes += (nw * 8 + 15) / 16 * 16;
+  }
+  const bool small = host_bytes <= kSmallFetch;
+  bool any_copy = false;
+  for (int c = 0; c < ncols; ++c) {
+    copy_words[c] = outs[c].validity &&
+                    (dev_words[c] ? reinterpret_cast<uintptr_t>(outs[c].validity) % 8 != 0 : !small);
+    any_copy = any_copy || copy_words[c];
+  }
+  uint8_t* pin = static_cast<uint8_t*>(ctx->pinned_in.reserve(flag_bytes + (small ? host_bytes : 0)));
+  std::memset(pin, 0, flag_bytes);
+  DevBuf staged;  // validity words that go by a copy
+  if (any_copy) staged.alloc(nw * 8 * ncols, ctx->stream);
+  FetchK P{};
+  P.count = count;
+  P.null_flags = reinterpret_cast<uint32_t*>(pin);
+  std::vector<uint8_t*> pin_data(ncols, nullptr), pin_words(ncols, nullptr);
+  uint8_t* at = pin + flag_bytes;
+  for (int c = 0; c < ncols; ++c) {
+    const size_t bytes = count * cols[c].width;
+    P.vals[c] = static_cast<const uint8_t*>(cols[c].vals) + first * cols[c].width;
+    P.valid[c] = cols[c].valid + first;
+    P.width[c] = static_cast<uint8_t>(cols[c].width);
+    if (dev_data[c]) {
+      P.dst[c] = static_cast<uint8_t*>(outs[c].data);
+    } else if (outs[c].data && small) {
+      P.dst[c] = pin_data[c] = at;
+      at += (bytes + 15) / 16 * 16;
+    } else if (outs[c].data) {
+      QEG_CUDA(cudaMemcpyAsync(outs[c].data, P.vals[c], bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    }
+    if (copy_words[c]) {
+      P.words[c] = staged.get<uint64_t>() + nw * c;
+    } else if (dev_words[c]) {
+      P.words[c] = outs[c].validity;
+    } else if (outs[c].validity) {
+      pin_words[c] = at;
+      P.words[c] = reinterpret_cast<uint64_t*>(at);
+      at += (nw * 8 + 15) / 16 * 16;
+    }
+    const uintptr_t ends = reinterpret_cast<uintptr_t>(P.vals[c]) | reinterpret_cast<uintptr_t>(P.dst[c]);
+    P.unit[c] = ends % 16 == 0 ? 16 : ends % cols[c].width == 0 ? P.width[c] : 1;
+  }
+  // About 1024 rows per block, at most eight blocks per SM over all columns.
+  const uint64_t gx = std::min<uint64_t>((count + 1023) / 1024,
+                                         std::max<uint64_t>(1, static_cast<uint64_t>(ctx->sms) * 8 / ncols));
+  fetch_kernel<<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(ncols)), 256, 0, ctx->stream>>>(P);
   ctx->launches++;
   QEG_CUDA(cudaGetLastError());
-  uint32_t has_null = 0;
-  if (out.validity) {
-    const auto vk = is_device_ptr(out.validity) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    QEG_CUDA(cudaMemcpyAsync(out.validity, words.get(), nw * 8, vk, ctx->stream));
-  }
-  QEG_CUDA(cudaMemcpyAsync(&has_null, any_null, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  for (int c = 0; c < ncols; ++c)
+    if (copy_words[c])
+      QEG_CUDA(cudaMemcpyAsync(outs[c].validity, P.words[c], nw * 8, cudaMemcpyDefault, ctx->stream));
   QEG_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (out.all_valid) *out.all_valid = has_null ? 0 : 1;
+  for (int c = 0; c < ncols; ++c) {
+    if (pin_data[c]) std::memcpy(outs[c].data, pin_data[c], count * cols[c].width);
+    if (pin_words[c]) std::memcpy(outs[c].validity, pin_words[c], nw * 8);
+    if (outs[c].all_valid) *outs[c].all_valid = P.null_flags[c] ? 0 : 1;
+  }
+}
+
+void fetch_column(qeg_ctx* ctx, const void* dev_vals, const uint8_t* dev_valid, size_t width,
+                  uint64_t first, uint64_t count, const qeg_out_column& out) {
+  const FetchCol col{dev_vals, dev_valid, width};
+  fetch_columns(ctx, &col, 1, first, count, &out);
 }
 
 }  // namespace qeg

@@ -210,9 +210,19 @@ inline unsigned grid_for(qeg_ctx* ctx, uint64_t work_items, int block, int block
   return static_cast<unsigned>(g == 0 ? 1 : g);
 }
 
-// Copies `count` rows starting at `first` of a device column (values `width`
-// bytes, validity as one byte per row) into a caller output column (host or
-// device), packing validity into 64-bit words.
+// Copies rows [first, first + count) of device columns (values `width` bytes,
+// validity as one byte per row) into caller output columns (host or device),
+// packing validity into 64-bit words: one kernel and one stream
+// synchronisation for all columns.
+struct FetchCol {
+  const void* vals;
+  const uint8_t* valid;
+  size_t width;
+};
+constexpr int kMaxFetchCols = 40;  // 8 keys and 32 aggregates
+void fetch_columns(qeg_ctx* ctx, const FetchCol* cols, int ncols, uint64_t first, uint64_t count,
+                   const qeg_out_column* outs);
+// The same for one column.
 void fetch_column(qeg_ctx* ctx, const void* dev_vals, const uint8_t* dev_valid, size_t width,
                   uint64_t first, uint64_t count, const qeg_out_column& out);
 
