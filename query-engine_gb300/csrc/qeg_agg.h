@@ -44,12 +44,10 @@ struct AggK {
   const uint32_t* sel;
   uint64_t nrows;  // rows to process (sel length, or len when dense)
   uint64_t len;    // physical column length
-  int smem_slots;  // power of two, 0 = no private table
+  int smem_slots;  // composite private tables: slots (power of two)
   int smem_insert; // 1: first-come insertion into the private table
-  int smem_probe;
   const uint64_t* hot;  // heavy hitters preloaded into the private table
   int nhot;
-  int warp_hot;  // the first warp_hot heavy hitters also get warp-private rows
   int probe_limit;
   uint32_t* spill_rows;
   uint64_t spill_cap;
@@ -60,27 +58,10 @@ struct AggK {
   uint32_t* full_flag;           // NULL: no table-full signal
   uint64_t full_at;              // running insert count that raises the flag
   uint32_t* err;
-  // Partitioned strategy, first pass (pool_key != nullptr): a row whose key is
-  // not in its CTA's private table (read-only: the sketch's heavy hitters) is
-  // appended to the region of its key's hash partition (key word + each value
-  // column's 8-byte value) instead of going to the global table. Region p
-  // holds rows [part_off[p], part_off[p + 1]) of the pool.
-  uint64_t* pool_key;
-  uint64_t* pool_val[kMaxVals];
-  unsigned long long* part_fill;  // rows appended per partition
-  const uint64_t* part_off;       // [nparts + 1] region starts (exact: a histogram pass sized them)
-  int part_shift;                 // partition of a key = key_hash1(key) >> part_shift
 };
 
-// Parameter block of the partitioned strategy's second pass (part_agg_kernel):
-// one CTA aggregates one partition's pool rows at a time in a shared-memory
-// table and appends its groups, as table rows, to `tails`.
+// Second pass of the partitioned strategy: where the groups go.
 struct PartB {
-  const uint64_t* pool_key;
-  const uint64_t* pool_val[kMaxVals];
-  const uint64_t* part_off;       // [nparts + 1]
-  uint32_t nparts;
-  int slots;                      // shared-memory table slots (power of two)
   uint64_t* tails;                // row_words words per group
   uint64_t tails_cap;
   unsigned long long* counters;   // [0] groups appended (may pass tails_cap), [1] failed partitions
@@ -99,6 +80,7 @@ struct FinK {
   unsigned long long* out_count;
   uint64_t out_cap;
   int64_t packed_width;  // > 0: single-key rows hold packed (partition key, bucket index) words
+  int32_t packed_pair;   // 1: single-key rows hold two packed 4-byte keys
   // Single key: a second table of the same row format (nullptr: none). A row
   // whose key is also there is merged into that row and not emitted; the
   // second table is finalized after this one.
@@ -115,16 +97,14 @@ struct SketchResult {
   double total_rows = 0;
   double null_frac = 0;
   double top_share[16] = {};  // share of sampled rows in the top 2^i candidates
-  std::vector<uint64_t> heavy;  // candidate heavy-hitter key words, most frequent first
 };
-
-// Perfect hash of the first n heavy-hitter key words (qeg_agg.cu): 2^lgT
-// slots, 2^lgB buckets, packed into `words` for the partitioned passes.
-void hot_phf_build(const uint64_t* keys, int n, int* lgT, int* lgB, std::vector<uint64_t>& words);
 
 // Builds the sketch of one key column (qeg_sketch.cu).
 void sketch_key_column(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uint64_t nrows, uint64_t len,
-                       uint64_t sample_target, int want_heavy, SketchResult& out);
+                       uint64_t sample_target, SketchResult& out);
+// The `want` most frequent key words of a sample, most frequent first.
+std::vector<uint64_t> sample_heavy(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uint64_t nrows, uint64_t len,
+                                   uint64_t sample_target, int want);
 // Sketches every query [offsets[q], offsets[q+1]) of a batch's key column in
 // one launch (one CTA per query); `d_offsets` is the device copy of `offsets`.
 void batch_sketch(qeg_ctx* ctx, const DevCol& key, const uint64_t* d_offsets, const std::vector<uint64_t>& offsets,
@@ -154,6 +134,7 @@ struct AggState {
   DevBuf table;
   uint64_t cap = 0;
   DevBuf counters, spill_rows, spill_parts, hot_keys_dev;
+  DevBuf priv_sums;  // F64 sums of the CTA-private tables (qeg_privagg.cuh)
   uint64_t spill_cap = 0, part_cap = 0;
   int smem_slots = 0, smem_insert = 0, nhot = 0;
   int probe_limit = 128;
@@ -166,25 +147,20 @@ struct AggState {
   // as its bucket's lower edge with this width; 0 for a plain GROUP BY.
   int64_t bucket_width = 0;
   // A window with one I32 partition key may pack (key, bucket index) into one
-  // key word and take the single-key path while every batch allows it (no
-  // NULLs in either column, bucket indexes within int32); a batch that does
-  // not converts the table to composite rows.
+  // key word, a GROUP BY of two keys of at most 4 bytes both of them, and take
+  // the single-key path while every batch allows it (no NULLs in either
+  // column, bucket indexes within int32); a batch that does not converts the
+  // table to composite rows.
   bool packable = false, packed = false;
   int64_t pack_qmin = 0, pack_qmax = 0;  // bucket-index range of the first packed batch
 
-  // Partitioned strategy (QEG_AGG_PARTITIONED, single key): the first pass
-  // aggregates each CTA's first-come keys in its private table and appends
-  // every other row to its key-hash partition's region of the pool; the second
-  // pass aggregates one partition per CTA in shared memory into `tails`, rows
-  // of the table format. The global table holds the private tables' flushes,
-  // spilled rows and partitions whose groups did not fit; finish() merges tail
-  // rows whose key is also there and emits both.
+  // Partitioned strategy (QEG_AGG_PARTITIONED, single key): heavy hitters go
+  // through private tables into the global table, every other row through the
+  // pool into `tails`, rows of the table format. The global table also holds
+  // the rows of partitions whose groups did not fit; finish() merges tail rows
+  // whose key is in both and emits both.
   int part_bits = 0;
-  int pb_slots = 0;
-  DevBuf phf_dev;  // the heavy hitters' perfect hash (hot_phf_build)
-  int phf_lgT = 6, phf_lgB = 3, phf_words = 0;
-  DevBuf pool_key, part_fill, part_off, part_hist, part_failed, tails, part_counters;
-  std::vector<DevBuf> pool_vals;
+  DevBuf pool, part_words, part_failed, tails, part_counters;
   uint64_t ntails = 0, tails_cap = 0;
 
   bool finished = false;
@@ -201,22 +177,26 @@ struct AggState {
   void unpack();
   void alloc_table(uint64_t new_cap);
   size_t smem_bytes(int block) const;
-  int warp_hot() const;
   int block_threads() const;
+  uint32_t null_field(int c) const;
+  int priv_max_slots(uint32_t skip) const;
   void set_field_columns(AggK& P) const;
   uint32_t field_spec(const AggK& P) const;  // qeg_warpagg.cuh field-set code
   void launch(const AggK& P, uint64_t nrows);
   void launch_private(const AggK& P, uint64_t nrows);  // composite keys, CTA-private tables
+  void launch_private1(const AggK& P, uint64_t nrows);  // single key, CTA-private tables
   void read_counters(uint64_t out[3]);
   void grow(uint64_t new_cap);
   void first_consume(const std::vector<StagedCol>& staged, uint64_t nrows, uint64_t len, const uint32_t* dsel);
+  void find_heavy(const std::vector<StagedCol>& staged, uint64_t nrows, uint64_t len, const uint32_t* dsel);
   double estimate_groups(const std::vector<StagedCol>& staged, uint64_t nrows, uint64_t len, const uint32_t* dsel);
   void settle(const std::vector<StagedCol>& staged, uint64_t len);
   bool part_eligible(const std::vector<StagedCol>& staged) const;
-  int part_table_slots() const;
+  int part_table_slots(uint32_t skip) const;
+  std::vector<uint64_t> hot_table(int want, int S, int* count) const;
+  void priv_sums_for(struct PrivK& A, uint64_t grid);
   void setup_partitioned(uint64_t nrows);
   void consume_partitioned(const std::vector<StagedCol>& staged, uint64_t nrows, uint64_t len, const uint32_t* dsel);
-  void part_second_pass();
   void merge_tails();
   void consume(const qeg_column* cols, int ncols, const uint32_t* sel, uint64_t sel_len);
   void finish(uint64_t* nrows_out);

@@ -21,6 +21,8 @@ enum ColType : int32_t { kI32 = 0, kI64 = 1, kF64 = 2, kBOOL = 3, kTS = 4, kSTR 
 // Internal key type (never a column type): a tumbling window's I32 partition
 // key and bucket index packed into one key word (see key_word).
 constexpr int32_t kPackedKey = 16;
+// Likewise: two keys of at most 4 bytes packed into one key word.
+constexpr int32_t kPackedPair = 17;
 
 constexpr uint64_t kCanonNaN = 0x7ff8000000000000ull;
 constexpr uint64_t kHashSeed = 0x51E57A11AB1E5EEDull;
@@ -40,8 +42,10 @@ struct DevCol {
   // kPackedKey: `data` is the partition key (type `type1`), `data2` the time
   // column (type `type2`); the key word is (key << 32) | (t / bucket), both
   // halves as 32-bit integers (no NULLs, key values and bucket indexes within
-  // int32).
+  // int32). kPackedPair: the key word is the two columns' 4-byte key words,
+  // (data << 32) | data2 (no NULLs).
   const void* data2;
+  const int32_t* code_map2;  // of data2, when it is a STR column
   int32_t type2;
   int32_t type1;
 };
@@ -62,6 +66,13 @@ __host__ __device__ __forceinline__ uint64_t hash_fold(uint64_t acc, uint64_t w)
 __device__ __forceinline__ bool col_valid(const DevCol& c, uint64_t p) {
   if (c.all_valid) return true;
   return (__ldg(c.validity + (p >> 6)) >> (p & 63)) & 1ull;
+}
+
+// 4-byte key word of row p of an I32, STR or BOOL column.
+__device__ __forceinline__ uint32_t key_word32(const void* data, const int32_t* code_map, int32_t type, uint64_t p) {
+  if (type == kBOOL) return __ldg(static_cast<const uint8_t*>(data) + p);
+  const int32_t v = __ldg(static_cast<const int32_t*>(data) + p);
+  return static_cast<uint32_t>(type == kSTR && code_map ? __ldg(code_map + v) : v);
 }
 
 // Canonical 64-bit key word of row p (valid rows only).
@@ -92,6 +103,9 @@ __device__ __forceinline__ uint64_t key_word(const DevCol& c, uint64_t p) {
       return (static_cast<uint64_t>(static_cast<uint32_t>(a)) << 32) |
              static_cast<uint32_t>(static_cast<int32_t>(q));
     }
+    case kPackedPair:
+      return (static_cast<uint64_t>(key_word32(c.data, c.code_map, c.type1, p)) << 32) |
+             key_word32(c.data2, c.code_map2, c.type2, p);
     case kF64: {
       const uint64_t b = static_cast<uint64_t>(__ldg(static_cast<const long long*>(c.data) + p));
       const uint64_t mag = b & 0x7fffffffffffffffull;

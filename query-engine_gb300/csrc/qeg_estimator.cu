@@ -114,7 +114,7 @@ qeg_status qeg_sketch(qeg_ctx* ctx, const qeg_column* key, uint64_t sample_rows,
     StagedCol s;
     stage_column(ctx, *key, s);
     SketchResult r;
-    sketch_key_column(ctx, s.dev, nullptr, key->len, key->len, sample_rows ? sample_rows : (1u << 20), 0, r);
+    sketch_key_column(ctx, s.dev, nullptr, key->len, key->len, sample_rows ? sample_rows : (1u << 20), r);
     for (int i = 0; i < kSketchFeatures; ++i) features[i] = r.features[i];
     if (classic_groups) *classic_groups = classic_estimate(r);
     if (top_share) *top_share = r.top_share[11];

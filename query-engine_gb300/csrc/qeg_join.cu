@@ -2195,7 +2195,7 @@ void JoinState::finish_build() {
       // Table size from the estimated distinct build keys (the learned
       // estimator, or the classic one without weights).
       SketchResult sk;
-      sketch_key_column(ctx, store_key(0), nullptr, nbuild, nbuild, 1u << 20, 0, sk);
+      sketch_key_column(ctx, store_key(0), nullptr, nbuild, nbuild, 1u << 20, sk);
       double g = 0, share = 0;
       if (!learned_estimate(ctx, sk, &g, &share)) g = classic_estimate(sk);
       if (const char* e = getenv("QEG_JOIN_EST_SCALE")) g *= atof(e);  // (tests: force a misestimate)

@@ -202,20 +202,27 @@ double hll_estimate(const std::vector<uint32_t>& regs) {
   return e;
 }
 
-}  // namespace
-
-void sketch_key_column(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uint64_t nrows, uint64_t len,
-                       uint64_t sample_target, int want_heavy, SketchResult& out) {
-  out = SketchResult{};
-  out.total_rows = static_cast<double>(nrows);
+// Sample blocks of kSampleBlock rows, `stride` rows apart, of about
+// `sample_target` rows in all.
+void sample_blocks(uint64_t nrows, uint64_t sample_target, uint64_t& stride, uint64_t& nblocks) {
   const uint64_t target_blocks = std::max<uint64_t>(1, sample_target / kSampleBlock);
-  uint64_t stride = kSampleBlock;
-  uint64_t nblocks = (nrows + kSampleBlock - 1) / kSampleBlock;
+  stride = kSampleBlock;
+  nblocks = (nrows + kSampleBlock - 1) / kSampleBlock;
   if (nblocks > target_blocks) {
     stride = ((nrows / target_blocks) / kSampleBlock) * kSampleBlock;
     if (stride < kSampleBlock) stride = kSampleBlock;
     nblocks = (nrows + stride - 1) / stride;
   }
+}
+
+}  // namespace
+
+void sketch_key_column(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uint64_t nrows, uint64_t len,
+                       uint64_t sample_target, SketchResult& out) {
+  out = SketchResult{};
+  out.total_rows = static_cast<double>(nrows);
+  uint64_t stride, nblocks;
+  sample_blocks(nrows, sample_target, stride, nblocks);
   const size_t words = kHllM + kCmsDepth * kCmsWidth;
   DevBuf buf(words * 4 + kCandGlobal * 16 + 16, ctx->stream);
   QEG_CUDA(cudaMemsetAsync(buf.get(), 0, buf.bytes(), ctx->stream));
@@ -292,9 +299,16 @@ void sketch_key_column(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uin
   f[77] = out.total_rows > 0 ? static_cast<float>(out.sample_rows / out.total_rows) : 1.f;
   f[78] = static_cast<float>(out.null_frac);
   f[79] = nonnull > 0 ? static_cast<float>(std::min(1.0, out.hll_estimate / nonnull)) : 0.f;
+}
 
-  if (want_heavy <= 0 || nblocks == 0) return;
-  // Heavy hitters: the sample's want_heavy most frequent keys, by exact counts.
+// Heavy hitters: the sample's `want` most frequent keys, by exact counts.
+std::vector<uint64_t> sample_heavy(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uint64_t nrows, uint64_t len,
+                                   uint64_t sample_target, int want) {
+  std::vector<uint64_t> out;
+  uint64_t stride, nblocks;
+  sample_blocks(nrows, sample_target, stride, nblocks);
+  if (nblocks == 0) return out;
+  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(nblocks, ctx->sms * 8ull));
   HeavyK H{};
   H.key = key;
   H.sel = sel;
@@ -304,7 +318,7 @@ void sketch_key_column(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uin
   H.nblocks = nblocks;
   H.cap = 1;
   while (H.cap < 2 * nblocks * kSampleBlock) H.cap <<= 1;
-  H.out_cap = static_cast<uint32_t>(4 * want_heavy);
+  H.out_cap = static_cast<uint32_t>(4 * want);
   const size_t head = H.cap * 12 + kHeavyBins * 4 + 16;
   DevBuf hb(head + static_cast<size_t>(H.out_cap) * 16, ctx->stream);
   QEG_CUDA(cudaMemsetAsync(hb.get(), 0, head, ctx->stream));
@@ -313,7 +327,7 @@ void sketch_key_column(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uin
   H.hist = H.cnt + H.cap;
   H.nout = H.hist + kHeavyBins;
   H.out = reinterpret_cast<unsigned long long*>(hb.get<uint8_t>() + head);
-  H.err = P.err;
+  H.err = static_cast<uint32_t*>(ctx->dev_err.get());
   heavy_count_kernel<<<grid, kSampleBlock, 0, ctx->stream>>>(H);
   heavy_hist_kernel<<<grid_for(ctx, H.cap, 256, 4), 256, 0, ctx->stream>>>(H);
   std::vector<uint32_t> hist(kHeavyBins);
@@ -344,8 +358,9 @@ void sketch_key_column(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uin
   std::sort(top.begin(), top.end(), [](const auto& a, const auto& b) {
     return a.first != b.first ? a.first > b.first : a.second < b.second;
   });
-  const size_t nh = std::min<size_t>(top.size(), static_cast<size_t>(want_heavy));
-  for (size_t i = 0; i < nh; ++i) out.heavy.push_back(top[i].second);
+  const size_t nh = std::min<size_t>(top.size(), static_cast<size_t>(want));
+  for (size_t i = 0; i < nh; ++i) out.push_back(top[i].second);
+  return out;
 }
 
 // ---------------------------------------------------------------------------
@@ -607,24 +622,19 @@ double AggState::estimate_groups(const std::vector<StagedCol>& staged, uint64_t 
     return static_cast<double>(std::min<uint64_t>(std::max<uint64_t>(nrows, 1), 1ull << 22));
   }
   SketchResult s;
-  // Heavy hitters are wanted for preloading (hot_keys > 0) and by the
-  // partitioned strategy, which the estimate may choose.
-  const bool part_possible = (cfg.strategy == QEG_AGG_AUTO || cfg.strategy == QEG_AGG_PARTITIONED) &&
-                             part_eligible(staged);
-  const int want_heavy = (cfg.hot_keys > 0 || part_possible) ? 4096 : 0;
-  if (packed) {
+  if (packed && bucket_width > 0) {
     // A packed window's (partition key, bucket) words are clustered by time,
     // which a strided sample cannot extrapolate: estimate the partition key's
     // distinct count instead and multiply by the buckets the time range
     // spans (at most one group per row).
-    sketch_key_column(ctx, staged[keys[0]].dev, dsel, nrows, len, 1u << 20, 0, s);
+    sketch_key_column(ctx, staged[keys[0]].dev, dsel, nrows, len, 1u << 20, s);
     double keys_est = 0, share = 0;
     if (!learned_estimate(ctx, s, &keys_est, &share)) keys_est = classic_estimate(s);
     hot_share = 0;
     const double buckets = static_cast<double>(pack_qmax - pack_qmin + 1);
     return std::max(1.0, std::min(static_cast<double>(nrows), std::max(keys_est, 1.0) * buckets));
   }
-  sketch_key_column(ctx, key_col(staged, 0), dsel, nrows, len, 1u << 20, want_heavy, s);
+  sketch_key_column(ctx, key_col(staged, 0), dsel, nrows, len, 1u << 20, s);
   double groups = 0, share = 0;
   if (learned_estimate(ctx, s, &groups, &share)) {
     hot_share = share;
@@ -632,8 +642,12 @@ double AggState::estimate_groups(const std::vector<StagedCol>& staged, uint64_t 
     groups = classic_estimate(s);
     hot_share = s.top_share[11];
   }
-  heavy_candidates = s.heavy;
   return std::max(groups, 1.0);
+}
+
+// The most frequent keys of a sample of the batch, most frequent first.
+void AggState::find_heavy(const std::vector<StagedCol>& staged, uint64_t nrows, uint64_t len, const uint32_t* dsel) {
+  heavy_candidates = sample_heavy(ctx, key_col(staged, 0), dsel, nrows, len, 1u << 20, 4096);
 }
 
 }  // namespace qeg
