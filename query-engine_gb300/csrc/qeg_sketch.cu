@@ -6,6 +6,7 @@
 // overflowing table is grown and the affected rows replayed).
 #include <algorithm>
 #include <cmath>
+#include <functional>
 
 #include "qeg_agg.h"
 
@@ -37,7 +38,13 @@ struct SketchK {
 
 __device__ __forceinline__ uint64_t sketch_hash(uint64_t w) { return mix64(w ^ 0x243F6A8885A308D3ull); }
 
-__global__ void __launch_bounds__(kSampleBlock) sketch_kernel(const SketchK P) {
+// The registers and the sketch take 140 KB of shared memory, so one CTA runs
+// per SM: kSketchThreads of them, several sample blocks at a time, hide the
+// latency of the loads and shared-memory atomics (256 threads: 67 us for 1M
+// sampled rows).
+constexpr int kSketchThreads = 1024;
+
+__global__ void __launch_bounds__(kSketchThreads) sketch_kernel(const SketchK P) {
   extern __shared__ uint32_t sh[];
   uint32_t* hll = sh;                                  // kHllM
   uint32_t* cms = hll + kHllM;                         // kCmsDepth * kCmsWidth
@@ -52,8 +59,10 @@ __global__ void __launch_bounds__(kSampleBlock) sketch_kernel(const SketchK P) {
   if (threadIdx.x == 0) s_rows = s_nulls = 0;
   __syncthreads();
   unsigned long long rows = 0, nulls = 0;
-  for (uint64_t b = blockIdx.x; b < P.nblocks; b += gridDim.x) {
-    const uint64_t i = b * P.stride + threadIdx.x;
+  constexpr int kBlocks = kSketchThreads / kSampleBlock;  // sample blocks per CTA at a time
+  for (uint64_t b = blockIdx.x * static_cast<uint64_t>(kBlocks) + threadIdx.x / kSampleBlock; b < P.nblocks;
+       b += gridDim.x * static_cast<uint64_t>(kBlocks)) {
+    const uint64_t i = b * P.stride + threadIdx.x % kSampleBlock;
     if (i >= P.nrows) continue;
     uint64_t p = i;
     if (P.sel) {
@@ -188,14 +197,12 @@ __global__ void heavy_compact_kernel(const HeavyK P) {
   }
 }
 
-double hll_estimate(const std::vector<uint32_t>& regs) {
+// HyperLogLog estimate from the number of registers of each value.
+double hll_estimate(const uint32_t (&regs)[65]) {
   const double m = kHllM;
   double sum = 0;
-  int zeros = 0;
-  for (uint32_t r : regs) {
-    sum += std::ldexp(1.0, -static_cast<int>(r));
-    if (r == 0) ++zeros;
-  }
+  for (int r = 0; r <= 64; ++r) sum += regs[r] * std::ldexp(1.0, -r);
+  const uint32_t zeros = regs[0];
   const double alpha = 0.7213 / (1.0 + 1.079 / m);
   double e = alpha * m * m / sum;
   if (e <= 2.5 * m && zeros > 0) e = m * std::log(m / zeros);  // linear counting
@@ -241,20 +248,22 @@ void sketch_key_column(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uin
   P.err = static_cast<uint32_t*>(ctx->dev_err.get());
   const size_t sb = words * 4 + kCandLocal * 12;
   raise_dynamic_smem(reinterpret_cast<const void*>(sketch_kernel), sb);
-  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(nblocks, ctx->sms * 2ull));
+  constexpr uint64_t kPer = kSketchThreads / kSampleBlock;
+  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((nblocks + kPer - 1) / kPer, ctx->sms));
   if (nblocks > 0) {
-    sketch_kernel<<<grid, kSampleBlock, sb, ctx->stream>>>(P);
+    sketch_kernel<<<grid, kSketchThreads, sb, ctx->stream>>>(P);
     ctx->launches++;
     QEG_CUDA(cudaGetLastError());
   }
-  std::vector<uint32_t> regs(words);
-  std::vector<unsigned long long> cand(2 * kCandGlobal + 2);
-  QEG_CUDA(cudaMemcpyAsync(regs.data(), buf.get(), words * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  QEG_CUDA(cudaMemcpyAsync(cand.data(), P.cand_key, cand.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
-  QEG_CUDA(cudaStreamSynchronize(ctx->stream));
-  check_device_error(ctx);
+  // Registers, sketch, candidates and totals lie back to back: one copy into
+  // page-locked memory, with the error word.
+  std::vector<uint64_t> host((words * 4 + kCandGlobal * 16 + 16) / 8);
+  read_words_and_error(ctx, buf.get(), host.size(), host.data());
+  const uint32_t* regs = reinterpret_cast<const uint32_t*>(host.data());
+  const uint64_t* cand = host.data() + words / 2;
 
-  const std::vector<uint32_t> hll(regs.begin(), regs.begin() + kHllM);
+  uint32_t hll[65] = {};  // registers by value
+  for (int i = 0; i < kHllM; ++i) ++hll[std::min<uint32_t>(regs[i], 64)];
   out.sample_rows = static_cast<double>(cand[2 * kCandGlobal]);
   const double nulls = static_cast<double>(cand[2 * kCandGlobal + 1]);
   out.null_frac = out.sample_rows > 0 ? nulls / out.sample_rows : 0;
@@ -271,20 +280,20 @@ void sketch_key_column(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uin
     }
     return best;
   };
-  std::vector<std::pair<uint32_t, uint64_t>> ranked;
+  std::vector<uint32_t> ranked;
   for (int i = 0; i < kCandGlobal; ++i)
-    if (cand[i]) ranked.push_back({cms_est(cand[i] - 1), cand[i] - 1});
-  std::sort(ranked.begin(), ranked.end(), [](auto& a, auto& b) { return a.first > b.first; });
+    if (cand[i]) ranked.push_back(cms_est(cand[i] - 1));
+  std::sort(ranked.begin(), ranked.end(), std::greater<uint32_t>());
 
   // Features: 64 normalised HLL register-value bins, then 16 frequency features.
   float* f = out.features;
   for (int i = 0; i < kSketchFeatures; ++i) f[i] = 0;
-  for (uint32_t r : hll) f[std::min<uint32_t>(r, 63)] += 1.0f / kHllM;
+  for (uint32_t r = 0; r <= 64; ++r) f[std::min<uint32_t>(r, 63)] += static_cast<float>(hll[r]) / kHllM;
   double cum = 0;
   size_t k = 0;
   for (int i = 0; i < 12; ++i) {
     const size_t upto = size_t(1) << i;
-    while (k < ranked.size() && k < upto) cum += ranked[k++].first;
+    while (k < ranked.size() && k < upto) cum += ranked[k++];
     out.top_share[i] = nonnull > 0 ? std::min(1.0, cum / nonnull) : 0;
   }
   for (int i = 0; i < 10; ++i) f[64 + i] = static_cast<float>(out.top_share[i]);
