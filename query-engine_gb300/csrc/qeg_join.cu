@@ -36,11 +36,13 @@ namespace qeg {
 namespace {
 
 constexpr uint32_t kNullRow = 0xffffffffu;  // ops/join_internal.h:31
-// Hashed single-key tables of at least this many bytes (too large to stay in
-// L2 beside the probe stream) get a Bloom filter of kBloomBitsPerKey bits per
-// build row: 16 bits and four bits per key in one 64-bit word give a false
-// positive rate of about 0.5%, in 32 MB for 16M build rows.
-constexpr uint64_t kBloomMinTableBytes = 32ull << 20;
+// Hashed single-key tables of at least this many bytes get a Bloom filter of
+// kBloomBitsPerKey bits per build row: 16 bits and four bits per key in one
+// 32-bit word give a false positive rate of about 0.8%, in 32 MB for 16M build
+// rows. The line: 128M random 32-byte reads beside the 2 GB probe stream take
+// 0.54 ms from a 64 MB table (all L2 hits), 1.03 ms from 96 MB, 1.32 ms from
+// 128 MB, while the filter's own read of every row costs 0.52 ms.
+constexpr uint64_t kBloomMinTableBytes = 96ull << 20;
 constexpr uint64_t kBloomBitsPerKey = 16;
 // Learned sizing of hashed single-key builds (QEG_SIZE_LEARNED): build sides
 // of at least kJoinSketchMinRows rows are sketched, and the table gets
@@ -64,10 +66,10 @@ struct JTable {
   const uint32_t* rows;
   const uint64_t* bitmap;  // dense and unique: one bit per slot
   int unique;
-  int shift;  // hash, single key: home slot = hash >> shift (64 - log2 cap)
+  int shift;  // hash, single key: home_slot(hash, shift), shift = 64 - log2 cap
   // Hash, single key: a blocked Bloom filter of the build keys (nullptr: none).
   // Key hash h selects word h >> bshift and sets the four bits bloom_mask(h).
-  const uint64_t* bloom;
+  const uint32_t* bloom;
   int bshift;
 };
 
@@ -86,15 +88,33 @@ __device__ __forceinline__ uint64_t ld_acquire64(const uint64_t* p) {
 }
 
 // Loads the key tuple of row p. Returns false when any key column is NULL.
-// Slot hash of a key tuple: one splitmix64 round for a single key word, the
-// seeded fold of every word for composite keys.
-__device__ __forceinline__ uint64_t single_key_hash(uint64_t k) { return mix64(k ^ kHashSeed); }
+// Slot hash of a single key word: two multiplies, a bijection (splitmix64's
+// finaliser takes about three times the instructions, and the sinks are bound
+// by them). Composite keys take the seeded fold of every word.
+__device__ __forceinline__ uint64_t single_key_hash(uint64_t k) {
+  uint64_t x = k * 0x9E3779B97F4A7C15ull;
+  x ^= x >> 32;
+  return x * 0xD1342543DE82EF95ull;
+}
 
-// Bits of a key in its Bloom filter word: four positions from the low 24 bits
-// of the key hash (the word is chosen by its top bits, the table's home slot by
-// its top bits too, so the positions are independent of both).
-__device__ __forceinline__ uint64_t bloom_mask(uint64_t h) {
-  return (1ull << (h & 63)) | (1ull << ((h >> 6) & 63)) | (1ull << ((h >> 12) & 63)) | (1ull << ((h >> 18) & 63));
+// Home slot of a single key: the first of a four-slot bucket (one 32-byte
+// sector) picked by the top bits of the hash. Buckets fill in order, so one
+// load answers a lookup unless the bucket is full of other keys.
+__device__ __forceinline__ uint64_t home_slot(uint64_t h, int shift) { return (h >> shift) & ~3ull; }
+
+// Bits of a key in its Bloom filter word: four positions from the low half of
+// the key hash (the word is chosen by its top bits, as the home slot is).
+__device__ __forceinline__ uint32_t bloom_mask(uint64_t h) {
+  const uint32_t x = static_cast<uint32_t>(h) >> 8;
+  return __funnelshift_l(1u, 1u, x) | __funnelshift_l(1u, 1u, x >> 5) | __funnelshift_l(1u, 1u, x >> 10) |
+         __funnelshift_l(1u, 1u, x >> 15);
+}
+
+// One bucket of a single-key table.
+__device__ __forceinline__ void load_bucket(const uint64_t* keys, uint64_t s, uint64_t (&c)[4]) {
+  asm volatile("ld.global.nc.L1::no_allocate.v4.b64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(c[0]), "=l"(c[1]), "=l"(c[2]), "=l"(c[3])
+               : "l"(keys + s));
 }
 
 __device__ __forceinline__ bool load_key(const DevCol* kc, int nk, uint64_t p, uint64_t* w, uint64_t& h) {
@@ -119,7 +139,7 @@ __device__ __forceinline__ int64_t hash_slot(const JTable& T, const uint64_t* w,
   if (T.nkeys == 1) {
     const uint64_t k = w[0];
     if (k == 0) return static_cast<int64_t>(T.cap);
-    uint64_t s = h >> T.shift;  // home slot: the top bits of the hash
+    uint64_t s = home_slot(h, T.shift);
     // (`limit`: an insert into a table sized from an estimate gives up after
     // that many slots; the build is then redone at full size.)
     for (uint64_t t = 0; t < T.cap && t < limit; ++t) {
@@ -185,7 +205,7 @@ struct BuildK {
   uint32_t* dup;
   unsigned long long* distinct;
   uint32_t* err;
-  unsigned long long* bloom;  // single key: the Bloom filter to fill (nullptr: none)
+  unsigned int* bloom;  // single key: the Bloom filter to fill (nullptr: none)
   // Single key, table sized from an estimate: inserts give up after
   // probe_limit slots and raise *ovf (nullptr: full-size table, no limit).
   uint32_t* ovf;
@@ -199,7 +219,7 @@ __global__ void build_count_kernel(BuildK P) {
     uint64_t w[kMaxKeys], h;
     bool existed = false;
     if (!load_key(P.key, P.nkeys, r, w, h)) continue;
-    if (P.bloom) atomicOr(P.bloom + (h >> P.T.bshift), static_cast<unsigned long long>(bloom_mask(h)));
+    if (P.bloom) atomicOr(P.bloom + (h >> P.T.bshift), bloom_mask(h));
     int64_t s;
     if (P.T.strategy == QEG_JOIN_DENSE) {
       s = dense_value(P.key[0], r) - P.T.dmin;
@@ -227,6 +247,81 @@ __global__ void build_count_kernel(BuildK P) {
   if ((threadIdx.x & 31) == 0) {
     if (fresh) atomicAdd(P.distinct, fresh);
     if (dup) *P.dup = 1;
+  }
+}
+
+// Hashed single key with deferred counts (P.presence): kInsertU rows per
+// thread, every step's loads and claims of all rows issued together. (One row
+// at a time left the inserts waiting on one random access each: 8M rows took
+// 396 us.)
+constexpr int kInsertU = 4;
+__global__ void __launch_bounds__(256) build_insert1_kernel(const __grid_constant__ BuildK P) {
+  unsigned long long fresh = 0;
+  uint32_t dup = 0;
+  const uint64_t step = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  for (uint64_t r0 = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; r0 < P.n; r0 += step * kInsertU) {
+    uint64_t k[kInsertU], s[kInsertU], cur[kInsertU];
+    bool look[kInsertU], any = false;
+#pragma unroll
+    for (int u = 0; u < kInsertU; ++u) {
+      const uint64_t r = r0 + u * step;
+      look[u] = r < P.n && col_valid(P.key[0], r);
+      k[u] = look[u] ? key_word(P.key[0], r) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < kInsertU; ++u) {
+      const uint64_t h = single_key_hash(k[u]);
+      if (look[u] && P.bloom) atomicOr(P.bloom + (h >> P.T.bshift), bloom_mask(h));
+      s[u] = home_slot(h, P.T.shift);
+      if (look[u] && k[u] == 0) {
+        look[u] = false;
+        if (!P.no_count) {
+          if (atomicAdd(&P.T.cnt[P.T.cap], 1u) != 0) dup = 1;
+          else ++fresh;
+        }
+      }
+      any |= look[u];
+    }
+    const uint64_t limit = P.ovf ? min(P.probe_limit, P.T.cap) : P.T.cap;
+    for (uint64_t t = 0; any && t < limit; ++t) {
+#pragma unroll
+      for (int u = 0; u < kInsertU; ++u) cur[u] = look[u] ? ld_relaxed64(P.T.keys + s[u]) : 1;
+      bool claim[kInsertU];
+#pragma unroll
+      for (int u = 0; u < kInsertU; ++u) {
+        claim[u] = look[u] && cur[u] == 0;
+        if (claim[u])
+          cur[u] = atomicCAS(reinterpret_cast<unsigned long long*>(P.T.keys + s[u]), 0ull,
+                             static_cast<unsigned long long>(k[u]));
+      }
+      any = false;
+#pragma unroll
+      for (int u = 0; u < kInsertU; ++u) {
+        if (!look[u]) continue;
+        if (claim[u] && cur[u] == 0) {
+          ++fresh;
+          look[u] = false;
+        } else if (cur[u] == k[u]) {
+          dup = 1;
+          look[u] = false;
+        } else {
+          s[u] = (s[u] + 1) & (P.T.cap - 1);
+          any = true;
+        }
+      }
+    }
+    if (any) {
+      if (P.ovf) atomicExch(P.ovf, 1u);  // the table is too small: the host rebuilds it
+      else atomicOr(P.err, kDevSpillOverflow);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    fresh += __shfl_down_sync(0xffffffffu, fresh, o);
+    dup |= __shfl_down_sync(0xffffffffu, dup, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (fresh && !P.no_count) atomicAdd(P.distinct, fresh);
+    if (dup && !P.no_count) *P.dup = 1;
   }
 }
 
@@ -326,11 +421,32 @@ struct ProbeK {
   int left;
   uint32_t* counts;    // per probe row output rows
   const uint64_t* starts;
+  uint32_t* match;     // per probe row: build row (unique build keys) or slot
   uint32_t* out_probe;
   uint32_t* out_build;
   unsigned long long* acc;  // sink: [0] count, [1] sum, [2] any payload
   uint32_t* err;
 };
+
+// Hashed single-key lookup of key word k (nonzero) whose home bucket g the
+// caller has loaded into c: match multiplicity. Walks on while buckets are
+// full of other keys.
+template <bool UNIQUE>
+__device__ __forceinline__ uint64_t hashed_resolve(const JTable& T, uint64_t k, uint64_t g, uint64_t (&c)[4]) {
+  for (uint64_t t = 0; t < T.cap; t += 4) {
+    if (UNIQUE) {
+      if (c[0] == k || c[1] == k || c[2] == k || c[3] == k) return 1;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (c[i] == k) return __ldg(T.cnt + g + i);
+    }
+    if (c[3] == 0) return 0;  // (buckets fill in order)
+    g = (g + 4) & (T.cap - 1);
+    load_bucket(T.keys, g, c);
+  }
+  return 0;
+}
 
 // Read-only lookup of one key in the finished table: match multiplicity.
 template <typename KT, int STRAT, bool UNIQUE>
@@ -344,41 +460,18 @@ __device__ __forceinline__ uint64_t sink_lookup(const JTable& T, KT key) {
     const uint64_t k = sizeof(KT) == 4 ? static_cast<uint64_t>(static_cast<uint32_t>(key))
                                        : static_cast<uint64_t>(key);
     if (k == 0) return __ldg(T.cnt + T.cap);
-    // Linear probing read four slots (one 32-byte sector) at a time: the
-    // aligned group holding the home slot, then the following groups. Slots
-    // before the home slot in the first group are not part of the probe.
-    const uint64_t home = single_key_hash(k) >> T.shift;
-    uint64_t g = home & ~3ull;
-    int skip = static_cast<int>(home & 3);
-    const ulonglong2* base = reinterpret_cast<const ulonglong2*>(T.keys);
-    for (uint64_t t = 0; t < T.cap; t += 4) {
-      const ulonglong2 a = __ldg(base + (g >> 1));
-      const ulonglong2 b = __ldg(base + (g >> 1) + 1);
-      const uint64_t c[4] = {a.x, a.y, b.x, b.y};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (i < skip) continue;
-        if (c[i] == k) return UNIQUE ? 1 : __ldg(T.cnt + g + i);
-        if (c[i] == 0) return 0;
-      }
-      skip = 0;
-      g = (g + 4) & (T.cap - 1);
-    }
-    return 0;
+    const uint64_t g = home_slot(single_key_hash(k), T.shift);
+    uint64_t c[4];
+    load_bucket(T.keys, g, c);
+    return hashed_resolve<UNIQUE>(T, k, g, c);
   }
 }
 
-// Loads a 64-bit word with an L2 evict-last policy: the Bloom filter (and
-// optionally the table) keeps its lines in L2 while the probe stream, loaded
-// evict-first, passes through.
-__device__ __forceinline__ uint64_t ld_keep_l2(const uint64_t* p, uint64_t pol) {
-  uint64_t v;
-  asm volatile("ld.global.nc.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(v) : "l"(p), "l"(pol));
-  return v;
-}
-__device__ __forceinline__ ulonglong2 ld_keep_l2x2(const ulonglong2* p, uint64_t pol) {
-  ulonglong2 v;
-  asm volatile("ld.global.nc.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;" : "=l"(v.x), "=l"(v.y) : "l"(p), "l"(pol));
+// Loads a Bloom filter word with an L2 evict-last policy: the filter keeps its
+// lines in L2 while the probe stream, loaded evict-first, passes through.
+__device__ __forceinline__ uint32_t ld_keep_l2(const uint32_t* p, uint64_t pol) {
+  uint32_t v;
+  asm volatile("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ uint64_t evict_last_policy() {
@@ -387,41 +480,14 @@ __device__ __forceinline__ uint64_t evict_last_policy() {
   return pol;
 }
 
-// Hashed single-key lookup of key word k (nonzero, home slot `home`) whose
-// first 32-byte slot group {a, b} (the aligned group holding the home slot) the
-// caller has already loaded: resolves within it when it can, else walks on.
-template <bool UNIQUE>
-__device__ __forceinline__ uint64_t hashed_resolve(const JTable& T, uint64_t k, uint64_t home, ulonglong2 a,
-                                                   ulonglong2 b) {
-  uint64_t g = home & ~3ull;
-  int skip = static_cast<int>(home & 3);
-  const ulonglong2* base = reinterpret_cast<const ulonglong2*>(T.keys);
-  for (uint64_t t = 0; t < T.cap; t += 4) {
-    if (t) {
-      a = __ldg(base + (g >> 1));
-      b = __ldg(base + (g >> 1) + 1);
-    }
-    const uint64_t c[4] = {a.x, a.y, b.x, b.y};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (i < skip) continue;
-      if (c[i] == k) return UNIQUE ? 1 : __ldg(T.cnt + g + i);
-      if (c[i] == 0) return 0;
-    }
-    skip = 0;
-    g = (g + 4) & (T.cap - 1);
-  }
-  return 0;
-}
-
 // Match multiplicities of two probe keys against a hashed single-key table,
 // with every memory access of the two rows issued before any is consumed: the
-// two Bloom filter words (when the table has a filter), then the first slot
-// group of each row that passed it. kv: the key is non-NULL.
+// two Bloom filter words (when the table has a filter), then the home bucket
+// of each row that passed it. kv: the key is non-NULL.
 template <typename KT, bool UNIQUE, bool BLOOM>
 __device__ __forceinline__ void hashed_lookup2(const JTable& T, const KT (&key)[2], const bool (&kv)[2],
-                                               uint64_t (&m)[2], uint64_t keep_pol, int keep_table) {
-  uint64_t k[2], h[2];
+                                               uint64_t (&m)[2], uint64_t keep_pol) {
+  uint64_t k[2], h[2], g[2], c[2][4];
   bool go[2];
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
@@ -430,39 +496,24 @@ __device__ __forceinline__ void hashed_lookup2(const JTable& T, const KT (&key)[
     go[j] = kv[j];
   }
   if (BLOOM) {
-    uint64_t fw[2];
+    uint32_t fw[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) fw[j] = go[j] ? ld_keep_l2(T.bloom + (h[j] >> T.bshift), keep_pol) : 0;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const uint64_t bm = bloom_mask(h[j]);
-      go[j] = go[j] && (fw[j] & bm) == bm;
-    }
+    for (int j = 0; j < 2; ++j) go[j] = go[j] && (~fw[j] & bloom_mask(h[j])) == 0;
   }
-  const ulonglong2* base = reinterpret_cast<const ulonglong2*>(T.keys);
-  ulonglong2 a[2], b[2];
-  uint64_t home[2];
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
-    home[j] = h[j] >> T.shift;
-    a[j] = make_ulonglong2(0, 0);
-    b[j] = make_ulonglong2(0, 0);
-    if (go[j] && k[j] != 0) {
-      const uint64_t g = home[j] & ~3ull;
-      if (keep_table) {
-        a[j] = ld_keep_l2x2(base + (g >> 1), keep_pol);
-        b[j] = ld_keep_l2x2(base + (g >> 1) + 1, keep_pol);
-      } else {
-        a[j] = __ldg(base + (g >> 1));
-        b[j] = __ldg(base + (g >> 1) + 1);
-      }
-    }
+    g[j] = home_slot(h[j], T.shift);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[j][i] = 0;
+    if (go[j]) load_bucket(T.keys, g[j], c[j]);
   }
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     if (!go[j]) m[j] = 0;
     else if (k[j] == 0) m[j] = __ldg(T.cnt + T.cap);
-    else m[j] = hashed_resolve<UNIQUE>(T, k[j], home[j], a[j], b[j]);
+    else m[j] = hashed_resolve<UNIQUE>(T, k[j], g[j], c[j]);
   }
 }
 
@@ -474,7 +525,6 @@ struct SinkK {
   uint64_t n;
   JTable T;
   unsigned long long* acc;  // [0] count, [1] sum, [2] any non-null payload matched
-  int keep_table;           // hashed table reads also evict-last in L2 (QEG_JOIN_TABLE_KEEP_L2=1)
 };
 
 template <typename T>
@@ -616,8 +666,6 @@ __global__ void __launch_bounds__(kSweepThreads, 6) probe_sink_sweep_kernel(cons
   const unsigned lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
   const uint32_t ntiles = static_cast<uint32_t>(P.n / kRows);
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const ulonglong2* tab = reinterpret_cast<const ulonglong2*>(P.T.keys);
-  const uint64_t mask = P.T.cap - 1;
   using Cnt = typename std::conditional<UNIQUE, uint32_t, unsigned long long>::type;
   Cnt cnt = 0;
   uint32_t seen = 0;
@@ -625,23 +673,10 @@ __global__ void __launch_bounds__(kSweepThreads, 6) probe_sink_sweep_kernel(cons
   // Match multiplicity of key word k (hash h) in the table.
   auto lookup = [&](uint64_t k, uint64_t h) -> uint64_t {
     if (k == 0) return __ldg(P.T.cnt + P.T.cap);
-    const uint64_t home = h >> P.T.shift;
-    uint64_t g = home & ~3ull;
-    int skip = static_cast<int>(home & 3);
-    for (uint64_t t = 0; t <= mask; t += 4) {
-      const ulonglong2 a = __ldg(tab + (g >> 1));
-      const ulonglong2 b = __ldg(tab + (g >> 1) + 1);
-      const uint64_t c[4] = {a.x, a.y, b.x, b.y};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (i < skip) continue;
-        if (c[i] == k) return UNIQUE ? 1 : __ldg(P.T.cnt + g + i);
-        if (c[i] == 0) return 0;
-      }
-      skip = 0;
-      g = (g + 4) & mask;
-    }
-    return 0;
+    const uint64_t g = home_slot(h, P.T.shift);
+    uint64_t c[4];
+    load_bucket(P.T.keys, g, c);
+    return hashed_resolve<UNIQUE>(P.T, k, g, c);
   };
   for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntiles; t += nwarps) {
     const uint64_t base = static_cast<uint64_t>(t) * kRows;
@@ -849,7 +884,7 @@ __global__ void __launch_bounds__(256, MINB) probe_sink_lean_kernel(const SinkK 
       for (int c = 0; c < U; ++c) {
         const bool kv[2] = {((ckw[c] >> (2 * lane)) & 1ull) != 0, ((ckw[c] >> (2 * lane + 1)) & 1ull) != 0};
         uint64_t m[2];
-        hashed_lookup2<KT, UNIQUE, BLOOM>(P.T, ck[c], kv, m, keep_pol, P.keep_table);
+        hashed_lookup2<KT, UNIQUE, BLOOM>(P.T, ck[c], kv, m, keep_pol);
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           cnt += static_cast<Cnt>(m[j]);
@@ -1104,7 +1139,7 @@ struct PartK {
   unsigned long long* cursor;  // [P] next free row of each partition (pass 2)
   uint64_t* okey;              // key words, partition order
   int64_t* oval;               // payloads, partition order
-  const uint64_t* bloom;       // the table's Bloom filter: rows that miss it are dropped (nullptr: none)
+  const uint32_t* bloom;       // the table's Bloom filter: rows that miss it are dropped (nullptr: none)
   int bshift;
 };
 
@@ -1112,10 +1147,7 @@ struct PartK {
 // rules the key out.
 __device__ __forceinline__ int probe_part(const PartK& P, uint64_t k, uint64_t pol) {
   const uint64_t h = single_key_hash(k);
-  if (P.bloom) {
-    const uint64_t bm = bloom_mask(h);
-    if ((ld_keep_l2(P.bloom + (h >> P.bshift), pol) & bm) != bm) return -1;
-  }
+  if (P.bloom && (~ld_keep_l2(P.bloom + (h >> P.bshift), pol) & bloom_mask(h)) != 0) return -1;
   return static_cast<int>(h >> (64 - P.bits));
 }
 
@@ -1460,28 +1492,205 @@ __global__ void __launch_bounds__(512) probe_count_sum_kernel(const ProbeK P) {
   }
 }
 
-__global__ void probe_count_kernel(const ProbeK P) {
-  for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < P.n; p += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t w[kMaxKeys], h;
-    uint32_t m = 0;
-    if (load_key(P.key, P.nkeys, p, w, h)) {
-      const int64_t s = probe_slot(P.T, P.key, p, w, h, P.err);
-      if (s >= 0) m = P.T.cnt[s];
+// Slots of U probe rows in the finished table, read-only, or -1 (a NULL key,
+// or a key the table does not hold). NK is the number of key columns (0: any);
+// the U rows' loads are issued together, and so are those of each probe step.
+template <int NK, int U>
+__device__ __forceinline__ void find_slots(const JTable& T, const DevCol* key, int nkeys, const uint64_t (&p)[U],
+                                           const bool (&live)[U], int64_t (&slot)[U]) {
+  if constexpr (NK == 1) {
+    uint64_t k[U];
+    bool look[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      slot[u] = -1;
+      look[u] = live[u] && col_valid(key[0], p[u]);
+      k[u] = look[u] ? (T.strategy == QEG_JOIN_DENSE ? static_cast<uint64_t>(dense_value(key[0], p[u]))
+                                                     : key_word(key[0], p[u]))
+                     : 0;
     }
-    if (m == 0 && P.left) m = 1;
-    P.counts[p] = m;
+    if (T.strategy == QEG_JOIN_DENSE) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint64_t s = k[u] - static_cast<uint64_t>(T.dmin);
+        if (look[u] && static_cast<int64_t>(k[u]) >= T.dmin && s < T.cap) slot[u] = static_cast<int64_t>(s);
+      }
+      return;
+    }
+    uint64_t g[U];
+    bool any = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (look[u] && k[u] == 0) {
+        slot[u] = static_cast<int64_t>(T.cap);
+        look[u] = false;
+      }
+      g[u] = home_slot(single_key_hash(k[u]), T.shift);
+      any |= look[u];
+    }
+    for (uint64_t t = 0; any && t < T.cap; t += 4) {
+      uint64_t c[U][4];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        c[u][3] = 0;
+        if (look[u]) load_bucket(T.keys, g[u], c[u]);
+      }
+      any = false;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (!look[u]) continue;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (c[u][i] == k[u]) slot[u] = static_cast<int64_t>(g[u] + i);
+        look[u] = slot[u] < 0 && c[u][3] != 0;
+        g[u] = (g[u] + 4) & (T.cap - 1);
+        any |= look[u];
+      }
+    }
+  } else {
+    // Composite keys: rows of [tag][key words] (every row is published).
+    constexpr int KW = NK == 0 ? kMaxKeys : NK;
+    const int nk = NK == 0 ? nkeys : NK;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      slot[u] = -1;
+      uint64_t w[KW], h = kHashSeed;
+      bool look = live[u];
+#pragma unroll
+      for (int j = 0; j < KW; ++j) {
+        w[j] = 0;
+        if (j < nk && look) {
+          look = col_valid(key[j], p[u]);
+          if (look) w[j] = key_word(key[j], p[u]);
+          h = hash_fold(h, w[j]);
+        }
+      }
+      const uint64_t tag = (h >> 32) | 2ull;
+      uint64_t s = h & (T.cap - 1);
+      for (uint64_t t = 0; look && t < T.cap; ++t) {
+        const uint64_t* r = T.keys + s * (1 + nk);
+        const uint64_t st = __ldg(r);
+        if (st == 0) break;
+        if (st == tag) {
+          bool eq = true;
+#pragma unroll
+          for (int j = 0; j < KW; ++j)
+            if (j < nk) eq &= __ldg(r + 1 + j) == w[j];
+          if (eq) {
+            slot[u] = static_cast<int64_t>(s);
+            break;
+          }
+        }
+        s = (s + 1) & (T.cap - 1);
+      }
+    }
   }
 }
 
-__global__ void probe_emit_kernel(const ProbeK P) {
+constexpr int kProbeU = 2;  // probe rows per thread in flight (a bucket of 32 bytes each)
+
+// Unique build keys: the build row of every key, by slot (filled with
+// kNullRow before). A probe then reads the row of its slot, with no row counts
+// and no row lists.
+template <int NK>
+__global__ void __launch_bounds__(256) build_rows_kernel(const __grid_constant__ BuildK P) {
+  const uint64_t step = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  for (uint64_t r0 = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; r0 < P.n; r0 += step * kProbeU) {
+    uint64_t p[kProbeU];
+    bool live[kProbeU];
+    int64_t slot[kProbeU];
+#pragma unroll
+    for (int u = 0; u < kProbeU; ++u) {
+      p[u] = r0 + u * step;
+      live[u] = p[u] < P.n;
+    }
+    find_slots<NK, kProbeU>(P.T, P.key, P.nkeys, p, live, slot);
+#pragma unroll
+    for (int u = 0; u < kProbeU; ++u)
+      if (slot[u] >= 0) P.rows_out[slot[u]] = static_cast<uint32_t>(p[u]);
+  }
+}
+
+// One lookup per probe row. Unique build keys (P.T.unique): match[p] is the
+// build row or kNullRow, and an inner join counts the matches of every
+// kProbeChunk rows (chunk c: rows of one warp, in order). Repeated keys:
+// counts[p] output rows and the slot in match[p] (kNullRow: none).
+constexpr int kProbeChunk = 32 * kProbeU;  // (64)
+template <int NK>
+__global__ void __launch_bounds__(256) probe_match_kernel(const __grid_constant__ ProbeK P) {
+  const unsigned lane = threadIdx.x & 31u;
+  const uint64_t nchunks = (P.n + kProbeChunk - 1) / kProbeChunk;
+  const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (uint64_t c = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; c < nchunks; c += nwarps) {
+    uint64_t p[kProbeU];
+    bool live[kProbeU];
+    int64_t slot[kProbeU];
+#pragma unroll
+    for (int u = 0; u < kProbeU; ++u) {
+      p[u] = c * kProbeChunk + u * 32 + lane;
+      live[u] = p[u] < P.n;
+    }
+    find_slots<NK, kProbeU>(P.T, P.key, P.nkeys, p, live, slot);
+    if (P.T.unique) {
+      uint32_t m[kProbeU];
+      unsigned found = 0;
+#pragma unroll
+      for (int u = 0; u < kProbeU; ++u) m[u] = slot[u] >= 0 ? __ldg(P.T.rows + slot[u]) : kNullRow;
+#pragma unroll
+      for (int u = 0; u < kProbeU; ++u) {
+        if (live[u]) P.match[p[u]] = m[u];
+        found += __popc(__ballot_sync(0xffffffffu, m[u] != kNullRow));
+      }
+      if (!P.left && lane == 0) P.counts[c] = found;
+    } else {
+      uint32_t n[kProbeU];
+#pragma unroll
+      for (int u = 0; u < kProbeU; ++u) n[u] = slot[u] >= 0 ? __ldg(P.T.cnt + slot[u]) : 0;
+#pragma unroll
+      for (int u = 0; u < kProbeU; ++u) {
+        if (!live[u]) continue;
+        P.match[p[u]] = n[u] ? static_cast<uint32_t>(slot[u]) : kNullRow;
+        P.counts[p[u]] = n[u] == 0 && P.left ? 1 : n[u];
+      }
+    }
+  }
+}
+
+// Inner join, unique build keys: the matches of chunk c go to output rows
+// starts[c]..., in probe order.
+__global__ void __launch_bounds__(256) probe_compact_kernel(const __grid_constant__ ProbeK P) {
+  const unsigned lane = threadIdx.x & 31u;
+  const uint64_t nchunks = (P.n + kProbeChunk - 1) / kProbeChunk;
+  const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (uint64_t c = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; c < nchunks; c += nwarps) {
+    uint64_t o = P.starts[c];
+    uint32_t m[kProbeU];
+#pragma unroll
+    for (int u = 0; u < kProbeU; ++u) {
+      const uint64_t p = c * kProbeChunk + u * 32 + lane;
+      m[u] = p < P.n ? P.match[p] : kNullRow;
+    }
+#pragma unroll
+    for (int u = 0; u < kProbeU; ++u) {
+      const unsigned hits = __ballot_sync(0xffffffffu, m[u] != kNullRow);
+      if (m[u] != kNullRow) {
+        const uint64_t at = o + __popc(hits & ((1u << lane) - 1u));
+        P.out_probe[at] = static_cast<uint32_t>(c * kProbeChunk + u * 32 + lane);
+        P.out_build[at] = m[u];
+      }
+      o += __popc(hits);
+    }
+  }
+}
+
+// Repeated build keys: every probe row's output rows from its slot's row list.
+__global__ void probe_emit_kernel(const __grid_constant__ ProbeK P) {
   for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < P.n; p += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t m = P.counts[p];
     if (m == 0) continue;
-    uint64_t o = P.starts[p];
-    uint64_t w[kMaxKeys], h;
-    int64_t s = -1;
-    if (load_key(P.key, P.nkeys, p, w, h)) s = probe_slot(P.T, P.key, p, w, h, P.err);
-    if (s < 0 || P.T.cnt[s] == 0) {  // LEFT join, unmatched: one row, build side NULL
+    const uint64_t o = P.starts[p];
+    const uint32_t s = P.match[p];
+    if (s == kNullRow) {  // LEFT join, unmatched: one row, build side NULL
       P.out_probe[o] = static_cast<uint32_t>(p);
       P.out_build[o] = kNullRow;
       continue;
@@ -1492,6 +1701,12 @@ __global__ void probe_emit_kernel(const ProbeK P) {
       P.out_build[o + t] = P.T.rows[b + t];
     }
   }
+}
+
+// out[k] = k.
+__global__ void iota_kernel(uint32_t* __restrict__ out, uint64_t n) {
+  for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
+    out[k] = static_cast<uint32_t>(k);
 }
 
 // ---- as-of join (tsx/asof.cpp) ---------------------------------------------
@@ -1703,7 +1918,6 @@ __global__ void __launch_bounds__(256) asof_probe_kernel(const AsofProbeK P) {
       }
     }
     if (P.left) {
-      P.out_probe[p] = static_cast<uint32_t>(p);
       P.out_build[p] = m;
     } else {
       P.match[p] = m;
@@ -1797,7 +2011,10 @@ __global__ void gather_out_kernel(const void* __restrict__ src, const uint64_t* 
 // All output columns in one pass: a warp loads the probe and build row
 // indices of its 64 output rows once, then writes every column's values and
 // validity word for them (the per-column kernel above re-reads the indices
-// once per column).
+// once per column). With a packed row store of the build side (pack_rows_kernel;
+// RW words per row) each output row reads its build row with one or two
+// 32-byte loads: column by column, every value and validity byte is a random
+// access of its own (7 of them: 20M rows of 20 bytes took 1.17 ms).
 constexpr int kMaxGatherCols = 32;
 
 struct GatherCol {
@@ -1810,14 +2027,19 @@ struct GatherCol {
   int width;
   int side;  // 0 probe, 1 build
   int flag;  // index of the column's NULL flag
+  int off;   // build side: byte offset in the packed row, and the validity bit
+  int bit;
 };
 
 struct GatherK {
   GatherCol c[kMaxGatherCols];
   int ncols;
-  const uint32_t* idx[2];
+  const uint32_t* idx[2];  // idx[0] == nullptr: output row k is probe row first + k
+  uint64_t first;
   uint64_t n;
   unsigned int* flags;  // per column: set when a NULL was written
+  const uint64_t* packed;  // packed build rows
+  int mask_off;            // byte offset of the validity bits (4 bytes)
 };
 
 __device__ __forceinline__ bool gather_one(const GatherCol& c, uint32_t r, uint64_t k) {
@@ -1841,31 +2063,126 @@ __device__ __forceinline__ bool gather_one(const GatherCol& c, uint32_t r, uint6
   return ok;
 }
 
-__global__ void __launch_bounds__(256) gather_cols_kernel(const GatherK P) {
+// The 8 bytes that hold byte `off` of a packed row, shifted down to it (an
+// aligned value of up to 8 bytes). The word is picked by selects: an array
+// indexed at run time would live in local memory.
+template <int RW>
+__device__ __forceinline__ uint64_t packed_at(const uint64_t (&w)[RW], int off) {
+  uint64_t x = w[0];
+#pragma unroll
+  for (int i = 1; i < RW; ++i)
+    asm("{.reg .pred p; setp.eq.s32 p, %1, %2; selp.b64 %0, %3, %0, p;}"
+        : "+l"(x)
+        : "r"(off >> 3), "r"(i), "l"(w[i]));
+  return x >> ((off & 7) * 8);
+}
+
+template <int RW>
+__device__ __forceinline__ void packed_load(const uint64_t* rows, uint32_t r, uint64_t (&w)[RW]) {
+#pragma unroll
+  for (int i = 0; i < RW; ++i) w[i] = 0;
+  if (r == kNullRow) return;
+  const uint64_t* p = rows + static_cast<uint64_t>(r) * RW;
+#pragma unroll
+  for (int i = 0; i < RW; i += 4)
+    asm volatile("ld.global.L1::no_allocate.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(w[i]), "=l"(w[i + 1]), "=l"(w[i + 2]), "=l"(w[i + 3])
+                 : "l"(p + i));
+}
+
+// RW: words of a packed build row (0: the build columns are gathered one by one).
+template <int RW>
+__global__ void __launch_bounds__(256) gather_cols_kernel(const __grid_constant__ GatherK P) {
+  constexpr int RWS = RW ? RW : 1;
   const unsigned lane = threadIdx.x & 31u;
   const uint64_t nw = (P.n + 63) / 64;
   const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
+  uint32_t nulls = 0;  // columns this warp wrote a NULL to
   for (uint64_t w = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < nw; w += nwarps) {
     const uint64_t k0 = w * 64 + lane, k1 = k0 + 32;
     const bool in0 = k0 < P.n, in1 = k1 < P.n;
     uint32_t r[2][2];
-#pragma unroll
-    for (int sd = 0; sd < 2; ++sd) {
-      r[sd][0] = in0 ? P.idx[sd][k0] : kNullRow;
-      r[sd][1] = in1 ? P.idx[sd][k1] : kNullRow;
+    r[0][0] = in0 ? (P.idx[0] ? P.idx[0][k0] : static_cast<uint32_t>(P.first + k0)) : kNullRow;
+    r[0][1] = in1 ? (P.idx[0] ? P.idx[0][k1] : static_cast<uint32_t>(P.first + k1)) : kNullRow;
+    r[1][0] = in0 ? P.idx[1][k0] : kNullRow;
+    r[1][1] = in1 ? P.idx[1][k1] : kNullRow;
+    uint64_t row0[RWS], row1[RWS];
+    uint32_t mask0 = 0, mask1 = 0;
+    if constexpr (RW > 0) {
+      packed_load<RW>(P.packed, r[1][0], row0);
+      packed_load<RW>(P.packed, r[1][1], row1);
+      mask0 = static_cast<uint32_t>(packed_at<RW>(row0, P.mask_off));
+      mask1 = static_cast<uint32_t>(packed_at<RW>(row1, P.mask_off));
     }
     for (int c = 0; c < P.ncols; ++c) {
       const GatherCol& col = P.c[c];
-      const int sd = col.side;
-      const bool ok0 = in0 ? gather_one(col, r[sd][0], k0) : true;
-      const bool ok1 = in1 ? gather_one(col, r[sd][1], k1) : true;
-      const unsigned b0 = __ballot_sync(0xffffffffu, ok0), b1 = __ballot_sync(0xffffffffu, ok1);
-      if (lane == 0) {
-        const uint64_t word = static_cast<uint64_t>(b0) | (static_cast<uint64_t>(b1) << 32);
-        if (col.words) col.words[w] = word;
-        if (word != ~0ull) atomicOr(P.flags + col.flag, 1u);
+      bool ok0 = true, ok1 = true;  // padding rows count as valid
+      if (RW > 0 && col.side == 1) {
+        const uint64_t x0 = packed_at<RWS>(row0, col.off), x1 = packed_at<RWS>(row1, col.off);
+        if (in0) {
+          ok0 = (mask0 >> col.bit) & 1u;
+          if (col.width == 8) static_cast<uint64_t*>(col.out)[k0] = x0;
+          else if (col.width == 4) static_cast<uint32_t*>(col.out)[k0] = static_cast<uint32_t>(x0);
+          else static_cast<uint8_t*>(col.out)[k0] = static_cast<uint8_t>(x0);
+        }
+        if (in1) {
+          ok1 = (mask1 >> col.bit) & 1u;
+          if (col.width == 8) static_cast<uint64_t*>(col.out)[k1] = x1;
+          else if (col.width == 4) static_cast<uint32_t*>(col.out)[k1] = static_cast<uint32_t>(x1);
+          else static_cast<uint8_t*>(col.out)[k1] = static_cast<uint8_t>(x1);
+        }
+      } else {
+        const int sd = col.side;
+        if (in0) ok0 = gather_one(col, r[sd][0], k0);
+        if (in1) ok1 = gather_one(col, r[sd][1], k1);
       }
+      const unsigned b0 = __ballot_sync(0xffffffffu, ok0), b1 = __ballot_sync(0xffffffffu, ok1);
+      const uint64_t word = static_cast<uint64_t>(b0) | (static_cast<uint64_t>(b1) << 32);
+      if (lane == 0 && col.words) col.words[w] = word;
+      if (word != ~0ull) nulls |= 1u << c;
     }
+  }
+  // One flag write per warp and column: a write per word (every word of a
+  // LEFT join's build columns) would queue up at one L2 address.
+  if (lane < static_cast<unsigned>(P.ncols) && ((nulls >> lane) & 1u)) P.flags[P.c[lane].flag] = 1u;
+}
+
+// The build columns side by side: row r's values at their columns' offsets
+// and one validity bit per column, RW words of 8 bytes.
+template <int RW>
+__global__ void __launch_bounds__(256) pack_rows_kernel(const __grid_constant__ GatherK P, uint64_t n,
+                                                        uint64_t* __restrict__ out) {
+  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
+    uint64_t w[RW];
+#pragma unroll
+    for (int i = 0; i < RW; ++i) w[i] = 0;
+    uint64_t mask = 0;
+    for (int c = 0; c <= P.ncols; ++c) {
+      uint64_t v;
+      int off;
+      if (c < P.ncols) {
+        const GatherCol& col = P.c[c];
+        if (col.width == 8) v = static_cast<const uint64_t*>(col.src)[r];
+        else if (col.width == 4) v = static_cast<const uint32_t*>(col.src)[r];
+        else v = static_cast<const uint8_t*>(col.src)[r];
+        off = col.off;
+        mask |= col.bytes[r] ? 1ull << col.bit : 0;
+      } else {
+        v = mask;
+        off = P.mask_off;
+      }
+      v <<= (off & 7) * 8;
+#pragma unroll
+      for (int i = 0; i < RW; ++i)
+        asm("{.reg .pred p; .reg .b64 t; setp.eq.s32 p, %1, %2; selp.b64 t, %3, 0, p; or.b64 %0, %0, t;}"
+            : "+l"(w[i])
+            : "r"(off >> 3), "r"(i), "l"(v));
+    }
+#pragma unroll
+    for (int i = 0; i < RW; i += 4)
+      asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(out + r * RW + i), "l"(w[i]), "l"(w[i + 1]),
+                   "l"(w[i + 2]), "l"(w[i + 3])
+                   : "memory");
   }
 }
 
@@ -1984,6 +2301,14 @@ struct JoinState {
   DevBuf counts, starts, out_probe, out_build;
   uint64_t nout = 0;
 
+  // Packed build rows for the output gather (0 words: not packed).
+  DevBuf packed;
+  int packed_words = 0, packed_mask = 0;
+  std::vector<int> packed_off;
+  bool pack_rows(uint64_t count);
+  bool rows_ready = false;  // unique keys: `rows` holds the build row of every slot
+  void ensure_rows();
+
   // count/sum sink totals
   DevBuf acc;
   bool acc_init = false;
@@ -1991,7 +2316,7 @@ struct JoinState {
   // as-of join (qeg_asof_create): time columns, tolerance, and the build side
   // sorted by (partition slot, timestamp)
   bool asof = false;
-  bool probe_identity = false;  // output row k of the last probe is probe row k (LEFT as-of)
+  bool probe_identity = false;  // output row k of the last probe is probe row k
   uint32_t ptime = 0, btime = 0;
   int32_t tol_set = 0;
   int64_t tol = 0;
@@ -2001,6 +2326,7 @@ struct JoinState {
   DevBuf krange;  // single integer key: [min enc, max enc, non-NULL count] over the appended batches
   void asof_build();
   void asof_probe(uint64_t n);
+  void identity_output(uint64_t n);
 
   JTable table() const {
     JTable T{};
@@ -2019,7 +2345,7 @@ struct JoinState {
     T.rows = rows.get<uint32_t>();
     T.bitmap = bitmap.get<uint64_t>();
     T.unique = unique;
-    T.bloom = bloom.get<uint64_t>();
+    T.bloom = bloom.get<uint32_t>();
     T.bshift = bloom_shift;
     return T;
   }
@@ -2354,17 +2680,19 @@ void JoinState::build_hash(BuildK& P, uint64_t want_cap) {
     const uint64_t bkeys_n = (cap < full && est_distinct > 0)
                                  ? std::min<uint64_t>(nbuild, static_cast<uint64_t>(2.0 * est_distinct) + 1)
                                  : nbuild;
-    const uint64_t words = next_pow2(std::max<uint64_t>(64, (bkeys_n * kBloomBitsPerKey + 63) / 64));
+    const uint64_t words = next_pow2(std::max<uint64_t>(64, (bkeys_n * kBloomBitsPerKey + 31) / 32));
     int lg = 0;
     while ((1ull << lg) < words) ++lg;
-    bloom.alloc(words * 8, ctx->stream);
-    QEG_CUDA(cudaMemsetAsync(bloom.get(), 0, words * 8, ctx->stream));
+    bloom.alloc(words * 4, ctx->stream);
+    QEG_CUDA(cudaMemsetAsync(bloom.get(), 0, words * 4, ctx->stream));
     bloom_shift = 64 - lg;
-    P.bloom = bloom.get<unsigned long long>();
+    P.bloom = bloom.get<unsigned int>();
   }
   P.T = table();
   if (nbuild) {
-    build_count_kernel<<<grid_for(ctx, nbuild, 256, 8), 256, 0, ctx->stream>>>(P);
+    const unsigned g = grid_for(ctx, nbuild, 256, 8);
+    if (nk == 1) build_insert1_kernel<<<g, 256, 0, ctx->stream>>>(P);
+    else build_count_kernel<<<g, 256, 0, ctx->stream>>>(P);
     ctx->launches++;
     QEG_CUDA(cudaGetLastError());
   }
@@ -2384,7 +2712,7 @@ void partitioned_sink(JoinState& st, const DevCol& key, const DevCol& val, uint6
   K.val = val.data;
   K.n = n;
   K.bits = st.part_bits;
-  K.bloom = st.bloom.get<uint64_t>();
+  K.bloom = st.bloom.get<uint32_t>();
   K.bshift = st.bloom_shift;
   DevBuf hist(static_cast<size_t>(np) * 8, ctx->stream), cursor((static_cast<size_t>(np) + 1) * 8, ctx->stream);
   QEG_CUDA(cudaMemsetAsync(hist.get(), 0, hist.bytes(), ctx->stream));
@@ -2493,6 +2821,70 @@ void JoinState::ensure_csr() {
   csr_built = true;
 }
 
+namespace {
+void (*match_kernel(int nk))(ProbeK) {
+  return nk == 1 ? probe_match_kernel<1> : nk == 2 ? probe_match_kernel<2> : probe_match_kernel<0>;
+}
+}  // namespace
+
+// Unique keys: the build row of every slot, on the first probe that
+// materialises pairs.
+void JoinState::ensure_rows() {
+  if (rows_ready) return;
+  rows.alloc(slots() * 4, ctx->stream);
+  QEG_CUDA(cudaMemsetAsync(rows.get(), 0xff, slots() * 4, ctx->stream));  // kNullRow
+  DevBuf scratch;
+  BuildK P = build_params(scratch);
+  P.rows_out = rows.get<uint32_t>();
+  if (nbuild) {
+    const int nk = static_cast<int>(bkeys.size());
+    void (*kern)(BuildK) = nk == 1 ? build_rows_kernel<1> : nk == 2 ? build_rows_kernel<2> : build_rows_kernel<0>;
+    kern<<<grid_for(ctx, nbuild, 256, 8), 256, 0, ctx->stream>>>(P);
+    ctx->launches++;
+    QEG_CUDA(cudaGetLastError());
+  }
+  rows_ready = true;
+}
+
+// Packs the build columns into rows when an output of `count` rows pays for
+// the pass (it reads and writes every build row once; each output row then
+// saves a random access per column and validity byte) and a row fits 64
+// bytes. Returns whether packed rows are there.
+bool JoinState::pack_rows(uint64_t count) {
+  if (packed_words) return true;
+  const int nc = static_cast<int>(btypes.size());
+  if (nc == 0 || nc > kMaxGatherCols || nbuild == 0 || count < 65536 || count * 2 < nbuild) return false;
+  packed_off.assign(nc, 0);
+  int at = 0;
+  for (int w : {8, 4, 1})
+    for (int c = 0; c < nc; ++c)
+      if (static_cast<int>(type_width(btypes[c])) == w) {
+        packed_off[c] = at;
+        at += w;
+      }
+  packed_mask = (at + 3) / 4 * 4;
+  const int words = packed_mask + 4 <= 32 ? 4 : packed_mask + 4 <= 64 ? 8 : 0;
+  if (words == 0) return false;
+  GatherK G{};
+  G.ncols = nc;
+  G.mask_off = packed_mask;
+  for (int c = 0; c < nc; ++c) {
+    G.c[c].src = bvals[c].get();
+    G.c[c].bytes = bvalid[c].get<uint8_t>();
+    G.c[c].width = static_cast<int>(type_width(btypes[c]));
+    G.c[c].off = packed_off[c];
+    G.c[c].bit = c;
+  }
+  packed.alloc(nbuild * words * 8, ctx->stream);
+  const unsigned g = grid_for(ctx, nbuild, 256, 8);
+  if (words == 4) pack_rows_kernel<4><<<g, 256, 0, ctx->stream>>>(G, nbuild, packed.get<uint64_t>());
+  else pack_rows_kernel<8><<<g, 256, 0, ctx->stream>>>(G, nbuild, packed.get<uint64_t>());
+  ctx->launches++;
+  QEG_CUDA(cudaGetLastError());
+  packed_words = words;
+  return true;
+}
+
 }  // namespace qeg
 
 struct qeg_join {
@@ -2513,6 +2905,18 @@ void validate_probe(const JoinState& st, const qeg_column* cols, int ncols) {
 }
 
 }  // namespace
+
+// Output row k of the probe is probe row k: the gather needs no probe row
+// indices (the per-column kernels of very wide outputs do).
+void JoinState::identity_output(uint64_t n) {
+  probe_identity = true;
+  out_probe.release();
+  if (ptypes.size() + btypes.size() <= static_cast<size_t>(kMaxGatherCols)) return;
+  out_probe.alloc(n * 4, ctx->stream);
+  iota_kernel<<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>(out_probe.get<uint32_t>(), n);
+  ctx->launches++;
+  QEG_CUDA(cudaGetLastError());
+}
 
 void JoinState::asof_probe(uint64_t n) {
   AsofProbeK P{};
@@ -2537,16 +2941,14 @@ void JoinState::asof_probe(uint64_t n) {
   const size_t hsb = static_cast<size_t>(8) << P.hint_bits;  // slot + position per entry
   const unsigned g = grid_for(ctx, n, 256, 8);
   if (P.left) {
-    out_probe.alloc(n * 4, ctx->stream);
     out_build.alloc(n * 4, ctx->stream);
-    P.out_probe = out_probe.get<uint32_t>();
     P.out_build = out_build.get<uint32_t>();
     asof_probe_kernel<<<g, 256, hsb, ctx->stream>>>(P);
     ctx->launches++;
     QEG_CUDA(cudaGetLastError());
+    identity_output(n);
     check_device_error(ctx);
     nout = n;
-    probe_identity = true;
     return;
   }
   amatch.alloc(n * 4, ctx->stream);
@@ -2706,13 +3108,56 @@ qeg_status qeg_join_probe(qeg_join* j, const qeg_column* cols, int ncols, uint64
       *out_rows = st.nout;
       return;
     }
+    const bool left = st.join_type == QEG_LEFT;
+    const uint64_t chunks = (n + kProbeChunk - 1) / kProbeChunk;
+    void (*match)(ProbeK) = match_kernel(static_cast<int>(st.pkeys.size()));
+    const unsigned g = grid_for(ctx, chunks * 32, 256, 8);
+    if (st.unique) {
+      // Every probe row matches at most one build row: one lookup pass, and
+      // for an inner join a compaction over the chunks' match counts.
+      st.ensure_rows();
+      DevBuf found;
+      ProbeK P = probe_params(st, n);
+      st.out_build.alloc(n * 4, ctx->stream);
+      if (left) {
+        P.match = st.out_build.get<uint32_t>();
+      } else {
+        found.alloc(n * 4, ctx->stream);
+        st.counts.alloc(chunks * 4, ctx->stream);
+        st.starts.alloc((chunks + 1) * 8, ctx->stream);
+        P.match = found.get<uint32_t>();
+        P.counts = st.counts.get<uint32_t>();
+      }
+      match<<<g, 256, 0, ctx->stream>>>(P);
+      ctx->launches++;
+      QEG_CUDA(cudaGetLastError());
+      uint64_t total = n;
+      if (left) {
+        st.identity_output(n);
+      } else {
+        total = exclusive_scan(ctx, st.counts.get<uint32_t>(), chunks, st.starts.get<uint64_t>());
+        st.out_probe.alloc(std::max<uint64_t>(total, 1) * 4, ctx->stream);
+        P.starts = st.starts.get<uint64_t>();
+        P.out_probe = st.out_probe.get<uint32_t>();
+        P.out_build = st.out_build.get<uint32_t>();
+        probe_compact_kernel<<<g, 256, 0, ctx->stream>>>(P);
+        ctx->launches++;
+        QEG_CUDA(cudaGetLastError());
+      }
+      check_device_error(ctx);
+      st.nout = total;
+      *out_rows = total;
+      return;
+    }
     st.ensure_csr();
+    require(st.slots() < kNullRow, "join table too large");
+    DevBuf slot(n * 4, ctx->stream);
     st.counts.alloc(n * 4, ctx->stream);
     st.starts.alloc((n + 1) * 8, ctx->stream);
     ProbeK P = probe_params(st, n);
     P.counts = st.counts.get<uint32_t>();
-    const unsigned g = grid_for(ctx, n, 256, 8);
-    probe_count_kernel<<<g, 256, 0, ctx->stream>>>(P);
+    P.match = slot.get<uint32_t>();
+    match<<<g, 256, 0, ctx->stream>>>(P);
     ctx->launches++;
     QEG_CUDA(cudaGetLastError());
     const uint64_t total = exclusive_scan(ctx, st.counts.get<uint32_t>(), n, st.starts.get<uint64_t>());
@@ -2721,7 +3166,7 @@ qeg_status qeg_join_probe(qeg_join* j, const qeg_column* cols, int ncols, uint64
     P.starts = st.starts.get<uint64_t>();
     P.out_probe = st.out_probe.get<uint32_t>();
     P.out_build = st.out_build.get<uint32_t>();
-    probe_emit_kernel<<<g, 256, 0, ctx->stream>>>(P);
+    probe_emit_kernel<<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>(P);
     ctx->launches++;
     QEG_CUDA(cudaGetLastError());
     check_device_error(ctx);
@@ -2765,14 +3210,32 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
       } else {
         g.src = st.bvals[bc].get();
         g.bytes = st.bvalid[bc].get<uint8_t>();
+        if (st.packed_words) {
+          g.off = st.packed_off[bc];
+          g.bit = static_cast<int>(bc);
+        }
       }
+    };
+    st.pack_rows(count);
+    auto launch_gather = [&](GatherK& G, uint64_t at, unsigned grid) {
+      G.idx[0] = st.out_probe.get() ? st.out_probe.get<uint32_t>() + at : nullptr;
+      G.idx[1] = st.out_build.get<uint32_t>() + at;
+      G.first = at;
+      G.packed = st.packed.get<uint64_t>();
+      G.mask_off = st.packed_mask;
+      if (st.packed_words == 4) gather_cols_kernel<4><<<grid, 256, 0, ctx->stream>>>(G);
+      else if (st.packed_words == 8) gather_cols_kernel<8><<<grid, 256, 0, ctx->stream>>>(G);
+      else gather_cols_kernel<0><<<grid, 256, 0, ctx->stream>>>(G);
+      ctx->launches++;
+      QEG_CUDA(cudaGetLastError());
     };
     if (dev_out) {
       // One pass per column into the caller's device buffers, one sync.
       DevBuf flags(ncol * 4, ctx->stream);
       QEG_CUDA(cudaMemsetAsync(flags.get(), 0, ncol * 4, ctx->stream));
       const unsigned gw = grid_for(ctx, (count + 63) / 64 * 32, 256, 8);
-      // Output row k = probe row first + k (LEFT as-of) with a word-aligned
+      // Output row k = probe row first + k (LEFT joins with at most one match
+      // per probe row) with a word-aligned
       // start: probe columns are plain copies, made by the copy engines on a
       // side stream while the gather kernel fills the build columns.
       std::vector<char> copied(ncol, 0);
@@ -2817,17 +3280,11 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
       }
       if (ncol <= static_cast<size_t>(kMaxGatherCols)) {
         GatherK G{};
-        G.idx[0] = st.out_probe.get<uint32_t>() + first;
-        G.idx[1] = st.out_build.get<uint32_t>() + first;
         G.n = count;
         G.flags = flags.get<unsigned int>();
         for (size_t c = 0; c < ncol; ++c)
           if (!copied[c]) gather_col(G.c[G.ncols++], c, outs[c].data, outs[c].validity);
-        if (G.ncols > 0) {
-          gather_cols_kernel<<<gw, 256, 0, ctx->stream>>>(G);
-          ctx->launches++;
-          QEG_CUDA(cudaGetLastError());
-        }
+        if (G.ncols > 0) launch_gather(G, first, gw);
       }
       if (forked) QEG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->side_out, 0));
       for (size_t c = 0; c < ncol && ncol > static_cast<size_t>(kMaxGatherCols); ++c) {
@@ -2858,6 +3315,42 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
         if (outs[c].all_valid) *outs[c].all_valid = f[c] ? 0 : 1;
       return;
     }
+    // Small host outputs: gathered straight into the context's page-locked
+    // buffer and copied from there by the host, without a copy command per
+    // column and its words (see fetch_columns for the line).
+    constexpr size_t kSmallFetch = 256 << 10;
+    size_t small = ncol * 4 + 16;
+    for (size_t c = 0; c < ncol; ++c)
+      small += (count * type_width(c < st.ptypes.size() ? st.ptypes[c] : st.btypes[c - st.ptypes.size()]) + 15) / 16 * 16 +
+               ((count + 63) / 64 * 8 + 15) / 16 * 16;
+    bool host_only = true;
+    for (size_t c = 0; c < ncol; ++c)
+      host_only = host_only && !(outs[c].data && is_device_ptr(outs[c].data)) &&
+                  !(outs[c].validity && is_device_ptr(outs[c].validity));
+    if (host_only && small <= kSmallFetch && ncol <= static_cast<size_t>(kMaxGatherCols)) {
+      uint8_t* pin = static_cast<uint8_t*>(ctx->pinned_in.reserve(small));
+      std::memset(pin, 0, ncol * 4);
+      uint8_t* at = pin + (ncol * 4 + 15) / 16 * 16;
+      const size_t nw = (count + 63) / 64;
+      GatherK G{};
+      G.ncols = static_cast<int>(ncol);
+      G.n = count;
+      G.flags = reinterpret_cast<unsigned int*>(pin);
+      for (size_t c = 0; c < ncol; ++c) {
+        const size_t w = type_width(c < st.ptypes.size() ? st.ptypes[c] : st.btypes[c - st.ptypes.size()]);
+        uint8_t* words = at + (count * w + 15) / 16 * 16;
+        gather_col(G.c[c], c, at, reinterpret_cast<uint64_t*>(words));
+        at = words + (nw * 8 + 15) / 16 * 16;
+      }
+      launch_gather(G, first, grid_for(ctx, nw * 32, 256, 8));
+      QEG_CUDA(cudaStreamSynchronize(ctx->stream));
+      for (size_t c = 0; c < ncol; ++c) {
+        if (outs[c].data) std::memcpy(outs[c].data, G.c[c].out, count * static_cast<size_t>(G.c[c].width));
+        if (outs[c].validity) std::memcpy(outs[c].validity, G.c[c].words, nw * 8);
+        if (outs[c].all_valid) *outs[c].all_valid = G.flags[c] ? 0 : 1;
+      }
+      return;
+    }
     if (ncol <= static_cast<size_t>(kMaxGatherCols)) {
       // Host (or mixed) outputs: chunks of rows gathered in one pass into
       // device staging buffers, each column then copied out; one sync.
@@ -2875,15 +3368,11 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
         const uint64_t n = std::min(chunk, count - off);
         GatherK G{};
         G.ncols = static_cast<int>(ncol);
-        G.idx[0] = st.out_probe.get<uint32_t>() + first + off;
-        G.idx[1] = st.out_build.get<uint32_t>() + first + off;
         G.n = n;
         G.flags = flags.get<unsigned int>();
         for (size_t c = 0; c < ncol; ++c)
           gather_col(G.c[c], c, vals.get<uint8_t>() + vofs[c], words.get<uint64_t>() + c * cw);
-        gather_cols_kernel<<<grid_for(ctx, (n + 63) / 64 * 32, 256, 8), 256, 0, ctx->stream>>>(G);
-        ctx->launches++;
-        QEG_CUDA(cudaGetLastError());
+        launch_gather(G, first + off, grid_for(ctx, (n + 63) / 64 * 32, 256, 8));
         for (size_t c = 0; c < ncol; ++c) {
           const size_t w = static_cast<size_t>(G.c[c].width);
           if (outs[c].data)
@@ -2967,7 +3456,6 @@ qeg_status qeg_join_probe_count_sum(qeg_join* j, const qeg_column* probe_key, co
       S.n = n;
       S.T = st.table();
       S.acc = st.acc.get<unsigned long long>();
-      if (const char* e = getenv("QEG_JOIN_TABLE_KEEP_L2")) S.keep_table = atoi(e) != 0;
       if (st.strategy == QEG_JOIN_PARTITIONED && v.dev.all_valid) {
         // (Payload NULLs would need a partitioned validity column: the direct
         // hashed sink below handles them.)
