@@ -277,9 +277,18 @@ __device__ __forceinline__ bool filter_bits(const PipeK& P, uint64_t b) {
   }
 }
 
-// Largest CTA of the thread-private kernels (the typed trades kernel fits 320
-// threads' states for 32 groups beside its translation table).
+// Largest CTA of the thread-private kernels (but the typed trades kernel's).
 constexpr int kLanesMaxThreads = 384;
+
+// Shared memory of the typed trades kernel's states: an F64 sum per group and
+// thread, three 32-bit words per group and lane. One launch gives each lane of
+// a CTA at most kLanesFastRows rows.
+__host__ __device__ constexpr size_t lanes_fast_state_bytes(int ngroups, int threads) {
+  return static_cast<size_t>(ngroups) * (static_cast<size_t>(threads) * 8 + 32 * 12);
+}
+constexpr uint64_t kLanesFastRows = (1u << 16) - 512;
+constexpr int kLanesFastThreads = 768;
+constexpr int kLanesFastR = 8;  // rows per thread in flight
 
 // Active fields of a field set: field 0 (the row count) and every field
 // whose kind is not 0, in field order ("compact" indexes).
@@ -317,7 +326,8 @@ __host__ __device__ constexpr int spec_compact(uint32_t spec, int i) {
 // global state. NA = the active field count (spec_nactive, or nfields for
 // the generic field set).
 template <uint32_t SPEC, int R, int FASTOP>
-__global__ void __launch_bounds__(kLanesMaxThreads, 1) pipeline_lanes_kernel(const PipeK P, int NA) {
+__global__ void __launch_bounds__(FASTOP >= 0 ? kLanesFastThreads : kLanesMaxThreads, 1)
+    pipeline_lanes_kernel(const PipeK P, int NA) {
   extern __shared__ unsigned long long acc[];
   constexpr int NVR = SPEC == kGenericSpec ? kPipeMaxVals : 2;  // value columns a row carries
   const int T = blockDim.x;
@@ -349,18 +359,49 @@ __global__ void __launch_bounds__(kLanesMaxThreads, 1) pipeline_lanes_kernel(con
     const double* __restrict__ price = static_cast<const double*>(P.val[0].data);
     const int32_t* __restrict__ qty = static_cast<const int32_t*>(P.val[1].data);
     const double lit = P.flit_f;
-    // Shared memory: the row counts as u32 (a thread counts fewer than 2^32
-    // rows), [group][thread]; then the sums, [group][SUM(F64), SUM(int)]
-    // [thread]; then the u16 translation table. 20 bytes per group and
-    // thread instead of 24 leave room for more threads.
-    const size_t cnt_words = (static_cast<size_t>(P.ngroups) * T + 1) / 2;
-    uint32_t* const cnt = reinterpret_cast<uint32_t*>(acc);
-    unsigned long long* const sums = acc + cnt_words;
-    uint16_t* kf16 = reinterpret_cast<uint16_t*>(sums + static_cast<size_t>(P.ngroups) * 2 * T);
-    for (size_t i = threadIdx.x; i < cnt_words + static_cast<size_t>(P.ngroups) * 2 * T; i += T) acc[i] = 0;
+    // Shared memory: the F64 sums, [group][thread]; then, [group][lane] for
+    // the whole CTA, the row counts (u32) and SUM(int) as the sums of the
+    // values' low 16 bits (u32) and of their high halves (i32), none of which
+    // can overflow in kLanesFastRows rows; then the u16 translation table.
+    // Counts and halves are 32-bit shared reductions: native, 2 clocks per
+    // warp, and nothing waits for them, so all warps may share them. The F64
+    // sum is a load, add and store and has to be the thread's own. 8 bytes per
+    // group and thread instead of 20 leave room for 768 threads instead of 320
+    // (200M trades onto 32 sectors: 0.96 ms with 320 threads whose warps
+    // issued one instruction in 11 clocks each).
+    const size_t words = static_cast<size_t>(P.ngroups) * T;
+    const uint32_t lwords = static_cast<uint32_t>(P.ngroups) * 32u;
+    double* const sumf = reinterpret_cast<double*>(acc);
+    uint32_t* const cnt = reinterpret_cast<uint32_t*>(sumf + words);
+    uint32_t* const qlo = cnt + lwords;
+    uint32_t* const qhi = qlo + lwords;
+    uint16_t* kf16 = reinterpret_cast<uint16_t*>(acc) + lanes_fast_state_bytes(P.ngroups, T) / 2;
+    for (size_t i = threadIdx.x; i < words; i += T) sumf[i] = 0.0;
+    for (uint32_t i = threadIdx.x; i < lwords * 3; i += T) cnt[i] = 0;
     for (uint64_t i = threadIdx.x; i < P.key_domain; i += T) kf16[i] = P.kf16[i];
     __syncthreads();
+    // A positive finite literal is compared through the doubles' two 32-bit
+    // halves: a negative value's sign bit makes its signed high half smaller
+    // than any positive literal's. The F64 pipe takes 16 clocks per warp
+    // instruction, as much for a compare as for the add below.
+    const bool lit_pos = lit > 0.0 && lit <= 1.7976931348623157e308;
+    const int32_t lit_hi = __double2hiint(lit);
+    const uint32_t lit_lo = static_cast<uint32_t>(__double2loint(lit));
     auto pass_of = [&](double v) {
+      if (lit_pos) {
+        const int32_t hi = __double2hiint(v);
+        const uint32_t lo = static_cast<uint32_t>(__double2loint(v));
+        const bool eq = hi == lit_hi && lo == lit_lo;
+        if constexpr (FASTOP == kEQ) return eq;
+        if constexpr (FASTOP == kNE) return !eq;
+        const uint32_t mag = static_cast<uint32_t>(hi) & 0x7fffffffu;
+        const bool nan = mag > 0x7ff00000u || (mag == 0x7ff00000u && lo != 0);
+        const bool gt = hi > lit_hi || (hi == lit_hi && lo > lit_lo);
+        if constexpr (FASTOP == kGT) return gt && !nan;
+        else if constexpr (FASTOP == kGE) return (gt || eq) && !nan;
+        else if constexpr (FASTOP == kLE) return !gt && !nan;
+        else return !gt && !eq && !nan;
+      }
       if constexpr (FASTOP == kLT) return v < lit;
       else if constexpr (FASTOP == kLE) return v <= lit;
       else if constexpr (FASTOP == kGT) return v > lit;
@@ -372,17 +413,21 @@ __global__ void __launch_bounds__(kLanesMaxThreads, 1) pipeline_lanes_kernel(con
     // 4-byte keys and their domain need 32-bit arithmetic only.
     const int32_t kmin32 = static_cast<int32_t>(P.key_min);
     const uint32_t dom32 = static_cast<uint32_t>(P.key_domain);
-    uint32_t* const my_cnt = cnt + threadIdx.x;
-    unsigned long long* const my_sum = sums + threadIdx.x;
+    const uint32_t my_cnt = static_cast<uint32_t>(__cvta_generic_to_shared(cnt + lane));
+    const uint32_t q_lo = lwords * 4u, q_hi = lwords * 8u;
+    double* const my_sum = sumf + threadIdx.x;
     auto apply = [&](int32_t k, double v, int32_t q) {
       const uint32_t sl = static_cast<uint32_t>(k) - static_cast<uint32_t>(kmin32);
-      if (!pass_of(v) || k < kmin32 || sl >= dom32) return;
-      const uint32_t g = kf16[sl];
-      if (g == 0xffffu) return;
-      my_cnt[g * T] += 1u;
-      unsigned long long* a = my_sum + 2 * g * T;
-      a[0] = static_cast<unsigned long long>(__double_as_longlong(__longlong_as_double(static_cast<long long>(a[0])) + v));
-      a[T] += static_cast<unsigned long long>(static_cast<long long>(q));
+      bool ok = pass_of(v) & (k >= kmin32) & (sl < dom32);
+      const uint32_t g = kf16[ok ? sl : 0];
+      ok &= g != 0xffffu;
+      if (ok) {
+        const uint32_t at = my_cnt + g * 128u;
+        asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(at) : "memory");
+        asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(at + q_lo), "r"(static_cast<uint32_t>(q) & 0xffffu) : "memory");
+        asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(at + q_hi), "r"(static_cast<uint32_t>(q >> 16)) : "memory");
+        my_sum[g * T] += v;
+      }
     };
     const uint64_t full = P.n / tile * tile;  // rows in full tiles
     for (uint64_t base = blockIdx.x * tile; base < full; base += static_cast<uint64_t>(gridDim.x) * tile) {
@@ -415,8 +460,12 @@ __global__ void __launch_bounds__(kLanesMaxThreads, 1) pipeline_lanes_kernel(con
       const int f = spec_active_field(SPEC, c);
       const uint8_t kind = static_cast<uint8_t>(c == 0 ? F_ROWS : spec_kind(SPEC, f));
       uint64_t x = 0;
-      for (int t = static_cast<int>(lane); t < T; t += 32)
-        x = field_combine(kind, x, c == 0 ? static_cast<uint64_t>(cnt[g * T + t]) : sums[(2 * g + c - 1) * T + t]);
+      const uint32_t i = static_cast<uint32_t>(g) * 32u + lane;
+      if (c == 0) x = cnt[i];
+      else if (c == 2) x = static_cast<uint64_t>(static_cast<int64_t>(static_cast<int32_t>(qhi[i])) * 65536 + qlo[i]);
+      else
+        for (int t = static_cast<int>(lane); t < T; t += 32)
+          x = field_combine(kind, x, static_cast<uint64_t>(__double_as_longlong(sumf[g * T + t])));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) x = field_combine(kind, x, __shfl_xor_sync(0xffffffffu, x, o));
       if (lane == 0 && x)
@@ -924,13 +973,9 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
                              (reinterpret_cast<uintptr_t>(P.val[0].data) % 16) == 0 &&
                              (reinterpret_cast<uintptr_t>(P.val[1].data) % 16) == 0;
         // Threads of the typed kernel: the most (a multiple of 32, at most
-        // kLanesMaxThreads) whose states (20 bytes per group and thread) and
-        // the translation table fit.
-        auto fast_bytes = [&](int t) {
-          const size_t cw = (static_cast<size_t>(P.ngroups) * t + 1) / 2;
-          return (cw + static_cast<size_t>(P.ngroups) * 2 * t) * 8 + ((domain * 2 + 15) / 16) * 16;
-        };
-        int T_fast = kLanesMaxThreads;
+        // kLanesFastThreads) whose states and the translation table fit.
+        auto fast_bytes = [&](int t) { return lanes_fast_state_bytes(P.ngroups, t) + ((domain * 2 + 15) / 16) * 16; };
+        int T_fast = kLanesFastThreads;
         while (T_fast > 64 && fast_bytes(T_fast) > ctx->smem_optin) T_fast -= 32;
         const size_t fast_sb = fast_bytes(T_fast);
         const bool single = std::none_of(kf16.begin(), kf16.end(), [](uint16_t x) { return x == 0xfffeu; });
@@ -940,23 +985,33 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
           lsb_fast = fast_sb;
           T = T_fast;
           switch (P.fop) {
-            case kLT: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, 16, kLT>; break;
-            case kLE: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, 16, kLE>; break;
-            case kGT: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, 16, kGT>; break;
-            case kGE: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, 16, kGE>; break;
-            case kEQ: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, 16, kEQ>; break;
-            case kNE: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, 16, kNE>; break;
+            case kLT: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, kLanesFastR, kLT>; break;
+            case kLE: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, kLanesFastR, kLE>; break;
+            case kGT: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, kLanesFastR, kGT>; break;
+            case kGE: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, kLanesFastR, kGE>; break;
+            case kEQ: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, kLanesFastR, kEQ>; break;
+            case kNE: lk = pipeline_lanes_kernel<kPipeSpecAvgSum, kLanesFastR, kNE>; break;
             default: break;
           }
         }
         const size_t lsb = lsb_fast ? lsb_fast : static_cast<size_t>(P.ngroups) * na * 8 * T;
         const int lper = blocks_per_sm(reinterpret_cast<const void*>(lk), T, lsb);
-        const int rows_per_tile = T * (spec == kGenericSpec ? 8 : 16);
+        const int rows_per_tile = T * (lsb_fast ? kLanesFastR : spec == kGenericSpec ? 8 : 16);
         const uint64_t lwant = (np + rows_per_tile - 1) / rows_per_tile;
         const unsigned lgrid = static_cast<unsigned>(
             std::max<uint64_t>(1, std::min<uint64_t>(lwant, static_cast<uint64_t>(ctx->sms) * std::max(lper, 1))));
-        if (np > 0 && domain > 0 && ngroups > 0) {
-          lk<<<lgrid, T, lsb, ctx->stream>>>(P, na);
+        // (The typed kernel's 32-bit sums hold kLanesFastRows rows per CTA and
+        // lane: more take several launches, whose results add up in the state.)
+        const uint64_t most = lsb_fast ? static_cast<uint64_t>(lgrid) * 32 * kLanesFastRows : np;
+        for (uint64_t first = 0; first < np && domain > 0 && ngroups > 0; first += most) {
+          PipeK L = P;
+          L.n = std::min(most, np - first);
+          if (lsb_fast) {
+            L.key.data = static_cast<const int32_t*>(P.key.data) + first;
+            L.val[0].data = static_cast<const double*>(P.val[0].data) + first;
+            L.val[1].data = static_cast<const int32_t*>(P.val[1].data) + first;
+          }
+          lk<<<lgrid, T, lsb, ctx->stream>>>(L, na);
           ctx->launches++;
           QEG_CUDA(cudaGetLastError());
         }
