@@ -568,6 +568,21 @@ __global__ void __launch_bounds__(FASTOP >= 0 ? kLanesFastThreads : kLanesMaxThr
   }
 }
 
+// Small device arrays of 4-byte words into page-locked host memory, one row of
+// blocks per array.
+constexpr size_t kCollectBytes = 256 << 10;
+struct CollectK {
+  const uint32_t* src[8];
+  uint32_t* dst[8];
+  uint32_t words[8];
+  unsigned n;
+};
+__global__ void __launch_bounds__(256) collect_kernel(const CollectK C) {
+  const uint32_t* src = C.src[blockIdx.y];
+  uint32_t* dst = C.dst[blockIdx.y];
+  for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < C.words[blockIdx.y]; i += gridDim.x * 256u) dst[i] = src[i];
+}
+
 }  // namespace
 
 }  // namespace qeg
@@ -635,19 +650,29 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
       f_pmap = want(probe[d->probe_key].code_map, probe[d->probe_key].code_map_len * 4);
     }
     uint8_t* fetched = static_cast<uint8_t*>(ctx->pinned_in.reserve(std::max<size_t>(fetch_bytes, 16)));
-    bool any_dev = false;
+    // Device arrays: one kernel writes all of them into the page-locked buffer
+    // (a copy command each costs more than its bytes); large ones are copied.
+    CollectK C{};
     for (const Fetch& f : fetches) {
       if (f.bytes == 0) continue;
-      if (f.dev) {
-        QEG_CUDA(cudaMemcpyAsync(fetched + f.off, f.src, f.bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        any_dev = true;
-      } else {
+      if (!f.dev) {
         std::memcpy(fetched + f.off, f.src, f.bytes);
+      } else if (f.bytes <= kCollectBytes && reinterpret_cast<uintptr_t>(f.src) % 4 == 0 && f.bytes % 4 == 0) {
+        C.src[C.n] = static_cast<const uint32_t*>(f.src);
+        C.dst[C.n] = reinterpret_cast<uint32_t*>(fetched + f.off);
+        C.words[C.n++] = static_cast<uint32_t>(f.bytes / 4);
+      } else {
+        QEG_CUDA(cudaMemcpyAsync(fetched + f.off, f.src, f.bytes, cudaMemcpyDeviceToHost, ctx->stream));
       }
     }
-    if (any_dev) QEG_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (C.n) {
+      collect_kernel<<<dim3(16, C.n), 256, 0, ctx->stream>>>(C);
+      ctx->launches++;
+      QEG_CUDA(cudaGetLastError());
+    }
+    QEG_CUDA(cudaStreamSynchronize(ctx->stream));
     auto at = [&](size_t i) -> const uint8_t* { return i == SIZE_MAX ? nullptr : fetched + fetches[i].off; };
-    auto valid_at = [](const uint8_t* words, uint64_t i) {
+    auto valid_at = [](const uint8_t* words, uint64_t i) -> bool {
       if (!words) return true;
       uint64_t w;
       std::memcpy(&w, words + (i >> 6) * 8, 8);
@@ -779,25 +804,59 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
       kmin = vmin;
       domain = static_cast<uint64_t>(vmax - vmin) + 1;
     }
-    // Counting sort of the build rows by join value (values span < 2^24, STR
-    // value ids are dense): glist holds the group ids value by value, and a
-    // probe key's run is [vstart[v], vstart[v] + vcount[v]).
     const uint64_t vrange = bval.empty() ? 0 : static_cast<uint64_t>(vmax - vmin) + 1;
     require(vrange < (1ull << 26), "join key values span too many values for the fused pipeline");
-    std::vector<uint32_t> vstart(vrange + 1, 0), glist(bval.size());
-    for (int64_t v : bval) ++vstart[static_cast<size_t>(v - vmin) + 1];
-    for (uint64_t i = 0; i < vrange; ++i) vstart[i + 1] += vstart[i];
-    {
+    // Group of each join value's build row, while every value has one row.
+    constexpr uint32_t kNoGroup = 0xffffffffu;
+    std::vector<uint32_t> vgroup(vrange, kNoGroup);
+    bool single = true;
+    for (size_t i = 0; i < bval.size() && single; ++i) {
+      uint32_t& g = vgroup[static_cast<size_t>(bval[i] - vmin)];
+      single = g == kNoGroup;
+      g = bgrp[i];
+    }
+    // Translation of the probe keys. kfirst: the group of a key that matches
+    // exactly one build row, kNoGroup for none, else the key's slot with the
+    // top bit set. Every key's groups are glist[kstart[s]...] (kcount[s] of
+    // them): the shared-state kernel reads these alone.
+    const uint64_t nslots = std::max<uint64_t>(domain, 1);
+    std::vector<uint32_t> kfirst(nslots, kNoGroup), kstart, kcount, glist;
+    auto slot_value = [&](uint64_t sl) {
+      return kt == QEG_STR ? static_cast<int64_t>(pmap[sl]) : kmin + static_cast<int64_t>(sl);
+    };
+    if (single) {
+      for (uint64_t sl = 0; sl < domain; ++sl) {
+        const int64_t v = slot_value(sl);
+        if (v >= vmin && v <= vmax) kfirst[sl] = vgroup[static_cast<size_t>(v - vmin)];
+      }
+      glist = kfirst;
+      kstart.resize(nslots);
+      kcount.resize(nslots);
+      for (uint64_t sl = 0; sl < nslots; ++sl) {
+        kstart[sl] = static_cast<uint32_t>(sl);
+        kcount[sl] = kfirst[sl] != kNoGroup ? 1 : 0;
+      }
+    } else {
+      // Counting sort of the build rows by join value (values span < 2^24, STR
+      // value ids are dense): glist holds the group ids value by value, and a
+      // probe key's run is [vstart[v], vstart[v] + vcount[v]).
+      std::vector<uint32_t> vstart(vrange + 1, 0);
+      glist.resize(bval.size());
+      for (int64_t v : bval) ++vstart[static_cast<size_t>(v - vmin) + 1];
+      for (uint64_t i = 0; i < vrange; ++i) vstart[i + 1] += vstart[i];
       std::vector<uint32_t> fill(vstart.begin(), vstart.end() - 1);
       for (size_t i = 0; i < bval.size(); ++i) glist[fill[static_cast<size_t>(bval[i] - vmin)]++] = bgrp[i];
-    }
-    std::vector<uint32_t> kstart(std::max<uint64_t>(domain, 1), 0), kcount(std::max<uint64_t>(domain, 1), 0);
-    for (uint64_t s = 0; s < domain; ++s) {
-      const int64_t v = kt == QEG_STR ? pmap[s] : kmin + static_cast<int64_t>(s);
-      if (v < vmin || v > vmax) continue;
-      const size_t i = static_cast<size_t>(v - vmin);
-      kstart[s] = vstart[i];
-      kcount[s] = vstart[i + 1] - vstart[i];
+      kstart.assign(nslots, 0);
+      kcount.assign(nslots, 0);
+      for (uint64_t sl = 0; sl < domain; ++sl) {
+        const int64_t v = slot_value(sl);
+        if (v < vmin || v > vmax) continue;
+        const size_t i = static_cast<size_t>(v - vmin);
+        kstart[sl] = vstart[i];
+        kcount[sl] = vstart[i + 1] - vstart[i];
+        if (kcount[sl] == 1) kfirst[sl] = glist[kstart[sl]];
+        else if (kcount[sl] > 1) kfirst[sl] = 0x80000000u | static_cast<uint32_t>(sl);
+      }
     }
 
     // ---- aggregate fields over probe columns (the AggState encodings) ------
@@ -895,17 +954,11 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
     P.key_domain = domain;
     for (size_t c = 0; c < vcols.size(); ++c) P.val[c] = staged[vcols[c]].dev;
     P.n = np;
-    // One-load translation for keys that match exactly one build row.
-    std::vector<uint32_t> kfirst(kstart.size(), 0xffffffffu);
-    for (uint64_t sl = 0; sl < domain; ++sl) {
-      if (kcount[sl] == 1) kfirst[sl] = glist[kstart[sl]];
-      else if (kcount[sl] > 1) kfirst[sl] = 0x80000000u | static_cast<uint32_t>(sl);
-    }
+    // The same as u16 for the typed kernel.
     std::vector<uint16_t> kf16;
-    if (ngroups <= 65533) {
+    if (ngroups <= 65533 && single) {
       kf16.resize(kfirst.size());
-      for (size_t i = 0; i < kfirst.size(); ++i)
-        kf16[i] = kfirst[i] == 0xffffffffu ? 0xffffu : (kfirst[i] & 0x80000000u) ? 0xfffeu : static_cast<uint16_t>(kfirst[i]);
+      for (size_t i = 0; i < kfirst.size(); ++i) kf16[i] = static_cast<uint16_t>(kfirst[i]);  // (kNoGroup: 0xffff)
     }
     // The translation tables go to the device in one copy from the context's
     // page-locked buffer into one device buffer: kstart, kcount, kfirst,
@@ -978,7 +1031,6 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
         int T_fast = kLanesFastThreads;
         while (T_fast > 64 && fast_bytes(T_fast) > ctx->smem_optin) T_fast -= 32;
         const size_t fast_sb = fast_bytes(T_fast);
-        const bool single = std::none_of(kf16.begin(), kf16.end(), [](uint16_t x) { return x == 0xfffeu; });
         if (spec == kPipeSpecAvgSum && key4 && P.key.all_valid && fsame && P.val[1].type == kI32 &&
             P.val[1].all_valid && aligned && P.kf16 && single && domain < (1ull << 31) &&
             fast_sb <= ctx->smem_optin) {
@@ -1040,10 +1092,8 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
         QEG_CUDA(cudaGetLastError());
       }
     }
-    std::vector<unsigned long long> st(static_cast<size_t>(P.ngroups) * P.nfields);
-    QEG_CUDA(cudaMemcpyAsync(st.data(), dstate.get(), st.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    QEG_CUDA(cudaStreamSynchronize(ctx->stream));
-    check_device_error(ctx);
+    std::vector<uint64_t> st(static_cast<size_t>(P.ngroups) * P.nfields);
+    read_words_and_error(ctx, dstate.get(), st.size(), st.data());
 
     // ---- finalise (ops/agg_internal.h:169-229) into the caller's columns ---
     uint64_t out = 0;
@@ -1051,7 +1101,7 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
     std::vector<std::vector<uint8_t>> vals(ncol);
     std::vector<std::vector<uint8_t>> ok(ncol);
     for (int g = 0; g < ngroups; ++g) {
-      const unsigned long long* f = &st[static_cast<size_t>(g) * P.nfields];
+      const uint64_t* f = &st[static_cast<size_t>(g) * P.nfields];
       if (f[0] == 0) continue;  // no joined row landed in this group
       auto put = [&](int c, uint64_t w, bool valid) {
         const size_t wd = type_width(rtypes[c]);
