@@ -2,8 +2,7 @@
 
 For every (group-count, skew) bucket of the batch planner it generates a
 seeded synthetic batch of queries of that bucket, runs the batch under every
-candidate (CTA-private table slots x rows per work item x warp peer
-aggregation on/off), times the graph replays with CUDA events and keeps the
+candidate (CTA-private table slots x rows per work item), times the graph replays with CUDA events and keeps the
 fastest; then it picks the block size on a mixed batch. The result is the
 tuning table qeg_batch_create takes, written as JSON beside libqeg.so
 (batch_tuning.json):
@@ -29,8 +28,8 @@ import qeg  # noqa: E402
 
 BUCKETS = [2.0, 6.0, 10.0, 14.0, 17.0, 20.0]  # upper bounds on log2(groups)
 SLOTS = [0, 256, 1024, 2048, 4096]
-ITEMS = [1 << 13, 1 << 14, 1 << 16]
-PEER = [0, 1]
+ITEMS = [1 << 13, 1 << 14, 1 << 16, 1 << 18]
+PEER = [0]  # (1 only asks for a private table, as slots > 0 does)
 BLOCKS = [256, 512, 1024]
 AGGS = [(qeg.COUNT_STAR, 0), (qeg.SUM, 1), (qeg.AVG, 1), (qeg.MIN, 1), (qeg.MAX, 1)]
 

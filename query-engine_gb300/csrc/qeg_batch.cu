@@ -23,6 +23,7 @@
 
 #include "qeg_agg.h"
 #include "qeg_mlp.h"
+#include "qeg_privagg.cuh"
 #include "qeg_warpagg.cuh"
 
 namespace qeg {
@@ -42,8 +43,6 @@ struct BatchQ {
   uint64_t cap;        // hash slots (+2 side rows follow)
   uint64_t out_off;    // first output row
   int32_t smem;        // 1: CTA-private shared-memory table first
-  int32_t smem_slots;  // power of two <= kBatchMaxSlots
-  int32_t peer;        // 1: lanes of a warp combine rows of one group first
   int32_t pad;
 };
 
@@ -59,55 +58,98 @@ struct BatchK {
   int W;  // words per row: key + fields
   int nfields;
   uint8_t fkind[kMaxFields];
-  int val_first, val_nf;  // value-column fields (cfirst/cnf of column 0)
+  uint8_t fcol[kMaxFields];  // (the one value column)
   uint32_t* overflow;     // per query
 };
 
+// Hash of a batch key word, and a key's row in its query's table: found or
+// claimed, or nullptr (the table is too full; the query is re-run). Past the
+// home slot's look every probe is one compare-and-swap (see global_rows1 in
+// qeg_agg.cu).
+__device__ __forceinline__ uint64_t batch_hash(uint64_t k) {
+  uint64_t x = k * 0x9E3779B97F4A7C15ull;
+  x ^= x >> 32;
+  return x * 0xD1342543DE82EF95ull;
+}
+template <int U>
+__device__ __forceinline__ void batch_global_rows(const BatchK& P, const BatchQ& Q, bool (&want)[U],
+                                                  const uint64_t (&k)[U], const uint64_t (&h)[U], uint64_t* (&r)[U]) {
+  uint64_t* T = P.arena + Q.table_off * P.W;
+  uint64_t s[U];
+  unsigned long long cur[U];
+  bool any = false;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    r[u] = nullptr;
+    s[u] = __umul64hi(h[u], Q.cap);
+    cur[u] = want[u] ? *reinterpret_cast<volatile unsigned long long*>(T + s[u] * P.W) : 0;
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (!want[u]) continue;
+    if (cur[u] == k[u]) {
+      r[u] = T + s[u] * P.W;
+      want[u] = false;
+    } else {
+      if (cur[u] != 0 && ++s[u] == Q.cap) s[u] = 0;
+      any = true;
+    }
+  }
+  for (int t = 0; any && t < 128; ++t) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (want[u])
+        cur[u] = atomicCAS(reinterpret_cast<unsigned long long*>(T + s[u] * P.W), 0ull,
+                           static_cast<unsigned long long>(k[u]));
+    any = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (!want[u]) continue;
+      if (cur[u] == 0 || cur[u] == k[u]) {
+        r[u] = T + s[u] * P.W;
+        want[u] = false;
+      } else {
+        if (++s[u] == Q.cap) s[u] = 0;
+        any = true;
+      }
+    }
+  }
+}
+
+// The one-key form for any key: the NULL key and key word 0 have rows of
+// their own after the slots.
 __device__ __forceinline__ uint64_t* batch_global_row(const BatchK& P, const BatchQ& Q, bool kv, uint64_t k) {
   uint64_t* T = P.arena + Q.table_off * P.W;
   if (!kv) return T + (Q.cap + 1) * P.W;
   if (k == 0) return T + Q.cap * P.W;
-  // Linear probing: the home slot alone, then four slots per step whose key
-  // words are loaded together (see global_row1 in qeg_agg.cu).
-  uint64_t s = __umul64hi(hash_fold(kHashSeed, k), Q.cap);
-  for (int t = 0; t < 128;) {
-    const int width = t == 0 ? 1 : 4;
-    uint64_t idx[4];
-    unsigned long long cur[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (j < width) {
-        uint64_t x = s + j;
-        if (x >= Q.cap) x -= Q.cap;
-        idx[j] = x;
-        cur[j] = *reinterpret_cast<volatile unsigned long long*>(T + x * P.W);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (j < width) {
-        uint64_t* r = T + idx[j] * P.W;
-        if (cur[j] == k) return r;
-        if (cur[j] == 0) {
-          const unsigned long long old =
-              atomicCAS(reinterpret_cast<unsigned long long*>(r), 0ull, static_cast<unsigned long long>(k));
-          if (old == 0 || old == k) return r;
-        }
-      }
-    }
-    t += width;
-    s += width;
-    if (s >= Q.cap) s -= Q.cap;
-  }
-  return nullptr;
+  bool want[1] = {true};
+  const uint64_t key[1] = {k}, h[1] = {batch_hash(k)};
+  uint64_t* r[1];
+  batch_global_rows<1>(P, Q, want, key, h, r);
+  return r[0];
 }
 
+// Rows per thread in flight.
+constexpr int kBatchU = 2;
+
+// Persistent CTAs take work items (a row range of one query) in turn. Rows are
+// added lane by lane to the CTA's private table (qeg_privagg.cuh), or to the
+// query's global table when their key has no place there; the private table
+// is merged into the global one and cleared at the end of each item. (Combining
+// the rows of a warp first took 480 warp instructions per 32 rows.)
 // SPEC: the value fields' set (qeg_warpagg.cuh), or kGenericSpec.
 template <uint32_t SPEC>
-__global__ void __launch_bounds__(1024) batch_agg_kernel(const BatchK P) {
-  extern __shared__ uint64_t sm[];
-  const int SW = P.W | 1;  // odd row stride in shared memory: fewer bank conflicts
+__global__ void __launch_bounds__(1024) batch_agg_kernel(const __grid_constant__ BatchK P,
+                                                         const __grid_constant__ PrivK A) {
+  extern __shared__ __align__(16) uint64_t sm[];
   __shared__ uint32_t s_item;
+  __shared__ unsigned s_nrep;
+  __shared__ uint16_t s_rslot[kPrivReps];
+  uint64_t* keys = sm;
+  const PrivT T = priv_init(sm, A);
+  uint8_t* rep = reinterpret_cast<uint8_t*>(sm) + A.rep_off;
+  const unsigned lane = threadIdx.x & 31u;
+  if (threadIdx.x == 0) s_nrep = 0;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(P.next, 1u);
     __syncthreads();
@@ -115,108 +157,83 @@ __global__ void __launch_bounds__(1024) batch_agg_kernel(const BatchK P) {
     if (item >= P.nitems) break;
     const uint32_t q = P.item_q[item];
     const BatchQ Q = P.qs[q];
-    const int S = Q.smem ? Q.smem_slots : 0;
-    if (S) {
-      for (int i = threadIdx.x; i < (S + 2) * SW; i += blockDim.x) sm[i] = 0;
-      __syncthreads();
-    }
+    const int S = Q.smem ? A.slots : 0;
     const uint64_t start = P.item_start[item];
     const uint32_t len = P.item_len[item];
     bool ovf = false;
-    const unsigned lane = threadIdx.x & 31u;
-    // Warps walk the item 32 rows at a time. With Q.peer, lanes of one group
-    // combine their rows first (warp peer aggregation) and the group's leader
-    // applies them; otherwise every lane applies its own row.
-    for (uint32_t wb = threadIdx.x & ~31u; wb < len; wb += blockDim.x) {
-      const uint32_t i = wb + lane;
-      const bool live = i < len;
-      const uint64_t p = start + i;
-      const bool kv = live && col_valid(P.key, p);
-      const uint64_t k = kv ? key_word(P.key, p) : 0;
-      const bool v = live && col_valid(P.val, p);
-      const uint64_t b = !v ? 0
-                         : (P.val.type == kF64 ? static_cast<uint64_t>(__double_as_longlong(f64_value(P.val, p)))
-                                               : static_cast<uint64_t>(int_value(P.val, p)));
-      unsigned peers = 1u << lane;
-      if (Q.peer) {
-        const unsigned livemask = __ballot_sync(0xffffffffu, live);
-        const unsigned same = match_word64(k, lane, P.key.type == kI32 || P.key.type == kSTR || P.key.type == kBOOL);
-        const unsigned vmask = __ballot_sync(0xffffffffu, kv);
-        if (live) peers = same & livemask & (kv ? vmask : ~vmask);
-      }
-      const bool leader = live && __ffs(peers) - 1 == static_cast<int>(lane);
-      uint64_t* f = nullptr;
-      int space = kRowGlobal;
-      if (leader) {
-        int srow = -1;
-        if (S) {
-          if (!kv) {
-            srow = S + 1;
-          } else if (k == 0) {
-            srow = S;
-          } else {
-            uint64_t s = hash_fold(kHashSeed, k) & (S - 1);
-            for (int t = 0; t < 8; ++t) {
-              unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&sm[s * SW]);
-              if (cur == 0)
-                cur = atomicCAS(reinterpret_cast<unsigned long long*>(&sm[s * SW]), 0ull,
-                                static_cast<unsigned long long>(k));
-              if (cur == 0 || cur == k) {
-                srow = static_cast<int>(s);
-                break;
-              }
-              s = (s + 1) & (S - 1);
-            }
-          }
+    uint32_t step = 0;
+    for (uint32_t b0 = 0; b0 < len; b0 += blockDim.x * kBatchU, ++step) {
+      bool live[kBatchU], kv[kBatchU], cold[kBatchU], vv[kBatchU][kMaxVals];
+      uint64_t k[kBatchU], h[kBatchU], vb[kBatchU][kMaxVals];
+      int slot[kBatchU];
+#pragma unroll
+      for (int u = 0; u < kBatchU; ++u) {
+        const uint32_t i = b0 + u * blockDim.x + threadIdx.x;
+        const uint64_t p = start + i;
+        live[u] = i < len;
+        kv[u] = live[u] && col_valid(P.key, p);
+        k[u] = kv[u] ? key_word(P.key, p) : 0;
+#pragma unroll
+        for (int c = 0; c < kMaxVals; ++c) {
+          vv[u][c] = false;
+          vb[u][c] = 0;
         }
-        if (srow >= 0) {
-          f = &sm[srow * SW + 1];
-          space = kRowShared;
-        } else {
-          uint64_t* r = batch_global_row(P, Q, kv, k);
-          if (r) f = r + 1;
-          else ovf = true;  // the query is recomputed exactly after the run
+        vv[u][0] = live[u] && col_valid(P.val, p);
+        if (vv[u][0])
+          vb[u][0] = P.val.type == kF64 ? static_cast<uint64_t>(__double_as_longlong(f64_value(P.val, p)))
+                                        : static_cast<uint64_t>(int_value(P.val, p));
+      }
+#pragma unroll
+      for (int u = 0; u < kBatchU; ++u) {
+        h[u] = batch_hash(k[u]);
+        slot[u] = -1;
+        if (S && live[u]) slot[u] = !kv[u] ? S + 1 : (k[u] == 0 ? S : priv_slot(keys, S, k[u], h[u]));
+      }
+      if (S && (step < 4 || (step & 7) == 0)) priv_promote(slot[0], rep, s_rslot, &s_nrep, lane);
+#pragma unroll
+      for (int u = 0; u < kBatchU; ++u) {
+        if (slot[u] >= 0) {
+          const int id = rep[slot[u]];
+          priv_apply<SPEC, 1>(T, A, id ? S + 2 + (id - 1) * 32 + static_cast<int>(lane) : slot[u], P.fkind, P.fcol,
+                              P.nfields, vv[u], vb[u]);
         }
       }
-      const PeerPlan pp = plan_peers(peers, lane);
-      const bool apply = leader && f != nullptr;
-      if constexpr (SPEC != kGenericSpec) {
-        bool vv[8] = {v};
-        uint64_t vb[8] = {b};
-        spec_apply<SPEC, 1>(f, apply, space, peers, pp, vv, vb);
-      } else {
-        if (apply) field_red_at(space, f, F_ROWS, static_cast<uint64_t>(__popc(peers)));
-        for (int j = 0; j < P.val_nf; ++j) {
-          const uint8_t kind = P.fkind[P.val_first + j];
-          const uint64_t x = peer_reduce(field_contrib(kind, v, b), kind, pp);
-          if (apply) field_red_at(space, f + P.val_first + j, kind, x);
-        }
+      uint64_t* r[kBatchU];
+#pragma unroll
+      for (int u = 0; u < kBatchU; ++u) cold[u] = live[u] && slot[u] < 0 && kv[u] && k[u] != 0;
+      batch_global_rows<kBatchU>(P, Q, cold, k, h, r);
+#pragma unroll
+      for (int u = 0; u < kBatchU; ++u) {
+        if (!live[u] || slot[u] >= 0) continue;
+        if (!kv[u] || k[u] == 0) r[u] = batch_global_row(P, Q, kv[u], k[u]);
+        if (r[u]) global_apply<SPEC, 1>(r[u] + 1, P.fkind, P.fcol, P.nfields, vv[u], vb[u]);
+        else ovf = true;  // the query is recomputed exactly after the run
       }
     }
     if (ovf) atomicOr(P.overflow + q, 1u);
     if (S) {
-      __syncthreads();
-      for (int sr = threadIdx.x; sr < S + 2; sr += blockDim.x) {
-        const uint64_t* src = &sm[sr * SW];
-        if (src[1] == 0) continue;
-        uint64_t* dst;
-        if (sr == S + 1) dst = batch_global_row(P, Q, false, 0);
-        else if (sr == S) dst = batch_global_row(P, Q, true, 0);
-        else dst = batch_global_row(P, Q, true, src[0]);
-        if (!dst) {
-          atomicOr(P.overflow + q, 1u);
-          continue;
-        }
+      priv_fence();
+      priv_fold(T, A, s_rslot, s_nrep, P.fkind, P.nfields);
+      priv_fence();
+      // (CTAs of one query start at different slots.)
+      const int rot = static_cast<int>((blockIdx.x * 97u) % static_cast<unsigned>(S + 2));
+      for (int i = threadIdx.x; i < S + 2; i += blockDim.x) {
+        int sr = i + rot;
+        if (sr >= S + 2) sr -= S + 2;
+        rep[sr] = 0;
+        if (priv_load(T, A, 0, F_ROWS, sr) == 0) continue;
+        const uint64_t key = sr < S ? keys[sr] : 0;
+        uint64_t* dst = batch_global_row(P, Q, sr != S + 1, key);
+        if (sr < S) keys[sr] = 0;
+        if (!dst) atomicOr(P.overflow + q, 1u);
+#pragma unroll 1
         for (int f = 0; f < P.nfields; ++f) {
-          const uint64_t x = src[1 + f];
-          if (!x) continue;
-          unsigned long long* d = reinterpret_cast<unsigned long long*>(dst + 1 + f);
-          const uint8_t kind = P.fkind[f];
-          if (kind == F_SUMF) atomicAdd(reinterpret_cast<double*>(d), __longlong_as_double(static_cast<long long>(x)));
-          else if (kind >= F_MINI) atomicMax(d, static_cast<unsigned long long>(x));
-          else atomicAdd(d, static_cast<unsigned long long>(x));
+          if ((A.skip >> f) & 1u) continue;
+          if (dst) field_red<kRowGlobal>(dst + 1 + f, P.fkind[f], priv_load(T, A, f, P.fkind[f], sr));
+          priv_clear(T, A, f, P.fkind[f], sr);
         }
       }
+      if (threadIdx.x == 0) s_nrep = 0;
     }
     __syncthreads();
   }
@@ -335,11 +352,15 @@ struct Round {
   std::vector<BatchQ> qs;
   uint32_t nitems = 0, nfin = 0;
   int32_t max_slots = 0;  // largest CTA-private table of the round (sizes the shared memory)
+  unsigned grid = 1;      // CTAs of the persistent kernel
+  DevBuf sums;            // F64 sums of their private tables
   DevBuf dqs, ditem_q, ditem_start, ditem_len, dfin_q, dfin_start, dfin_len, dnext, arena, overflow, counts;
   std::vector<DevBuf> out_vals, out_valid;
 };
 
-constexpr uint32_t kFinRows = 1u << 16;  // table rows per finalize block
+// Table rows per finalize block: enough blocks to fill the GPU for a few
+// queries too (64K rows: 119 blocks for 64 queries, 370 us).
+constexpr uint32_t kFinRows = 1u << 13;
 
 struct BatchState {
   qeg_ctx* ctx = nullptr;
@@ -382,8 +403,11 @@ struct BatchState {
     for (uint32_t l = 0; l < n; ++l) {
       const uint32_t q = qids[l];
       const uint64_t cap = caps[l];
-      R.qs[l] = BatchQ{table_rows, cap, table_rows, slots[q] > 0 ? 1 : 0, std::max(slots[q], 64), peer[q], 0};
-      R.max_slots = std::max(R.max_slots, slots[q]);
+      // (Peer aggregation asked for without a private table: the private table
+      // is what keeps the hot rows of a warp from queueing up at one address.)
+      const bool priv = slots[q] > 0 || peer[q];
+      R.qs[l] = BatchQ{table_rows, cap, table_rows, priv ? 1 : 0, 0};
+      R.max_slots = std::max(R.max_slots, priv ? std::max(slots[q], 256) : 0);
       table_rows += cap + 2;
       const uint64_t rows = rows_of(q);
       for (uint64_t s0 = 0; s0 < rows; s0 += chunk[q]) {
@@ -427,6 +451,12 @@ struct BatchState {
     R.overflow.alloc(std::max<uint32_t>(n, 1) * 4, ctx->stream);
     QEG_CUDA(cudaMemsetAsync(R.overflow.get(), 0, R.overflow.bytes(), ctx->stream));
     R.counts.alloc(std::max<uint32_t>(n, 1) * 8, ctx->stream);
+    const PrivK A = priv_table(R.max_slots);
+    const int per_sm = blocks_per_sm(reinterpret_cast<const void*>(agg_kernel_for()), block, A.bytes);
+    require(per_sm > 0, "batch kernel does not fit on an SM with this configuration");
+    R.grid = static_cast<unsigned>(
+        std::max(1, std::min<int>(ctx->sms * per_sm, static_cast<int>(std::max<uint32_t>(R.nitems, 1)))));
+    R.sums.alloc(std::max<size_t>(static_cast<size_t>(A.sum_bytes) * R.grid, 16), ctx->stream);
     R.out_vals.resize(plan.rtypes.size());
     R.out_valid.resize(plan.rtypes.size());
     for (size_t c = 0; c < plan.rtypes.size(); ++c) {
@@ -449,8 +479,6 @@ struct BatchState {
     P.W = plan.row_words;
     P.nfields = plan.nfields;
     for (int f = 0; f < plan.nfields; ++f) P.fkind[f] = plan.fkind[f];
-    P.val_first = plan.cfirst.empty() ? 0 : plan.cfirst[0];
-    P.val_nf = plan.cnf.empty() ? 0 : plan.cnf[0];
     P.overflow = R.overflow.get<uint32_t>();
     return P;
   }
@@ -482,7 +510,7 @@ struct BatchState {
 
   // The batch kernel for this plan's field set: COUNT/SUM/AVG/MIN/MAX over
   // one value column (with or without its NULL count) has its own kernel.
-  void (*agg_kernel_for() const)(BatchK) {
+  void (*agg_kernel_for() const)(BatchK, PrivK) {
     const int n = plan.nfields - 1;
     if (n > 7) return batch_agg_kernel<kGenericSpec>;
     uint32_t spec = static_cast<uint32_t>(n);
@@ -496,18 +524,19 @@ struct BatchState {
     return batch_agg_kernel<kGenericSpec>;
   }
 
-  size_t smem_bytes(int32_t max_slots) const { return static_cast<size_t>(max_slots + 2) * (plan.row_words | 1) * 8; }
+  // The CTA-private table of a round whose largest has `max_slots` slots (a
+  // power of two; every query of the round uses that many).
+  PrivK priv_table(int32_t max_slots) const {
+    const uint32_t skip = val.dev.all_valid && !plan.val_cols.empty() ? plan.null_field(0) : 0;
+    return priv_layout(plan.fkind.data(), plan.nfields, std::max(max_slots, 64), skip, kPrivReps);
+  }
 
   void enqueue(Round& R) {
     QEG_CUDA(cudaMemsetAsync(R.dnext.get(), 0, 4, ctx->stream));
     QEG_CUDA(cudaMemsetAsync(R.counts.get(), 0, R.counts.bytes(), ctx->stream));
-    const size_t sb = smem_bytes(R.max_slots);
-    int per_sm = 1;
-    void (*kern)(BatchK) = agg_kernel_for();
-    QEG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, sb));
-    const unsigned grid = static_cast<unsigned>(
-        std::max(1, std::min<int>(ctx->sms * std::max(per_sm, 1), static_cast<int>(std::max<uint32_t>(R.nitems, 1)))));
-    kern<<<grid, block, sb, ctx->stream>>>(kparams(R));
+    PrivK A = priv_table(R.max_slots);
+    A.sums = R.sums.get<uint8_t>();
+    agg_kernel_for()<<<R.grid, block, A.bytes, ctx->stream>>>(kparams(R), A);
     if (R.nfin) batch_finalize_kernel<<<R.nfin, 512, 0, ctx->stream>>>(finparams(R));
   }
 
@@ -643,9 +672,12 @@ qeg_status qeg_batch_create(qeg_ctx* ctx, uint32_t nqueries, const uint64_t* row
       all[q] = q;
       caps[q] = std::max<uint64_t>(64, static_cast<uint64_t>(kEstimateHeadroom * g / kTargetLoad) + 16);
     }
-    const size_t sb = S.smem_bytes(kBatchMaxSlots);
-    require(sb <= ctx->smem_optin, "batch rows are too wide for the shared-memory tables");
-    raise_dynamic_smem(reinterpret_cast<const void*>(S.agg_kernel_for()), sb);
+    // Private tables as large as a third of an SM's shared memory allows at
+    // most (three CTAs of 512 threads), at least 256 slots.
+    int32_t most = kBatchMaxSlots;
+    while (most > 256 && S.priv_table(most).bytes > ctx->smem_optin / 3) most /= 2;
+    require(S.priv_table(most).bytes <= ctx->smem_optin, "batch rows are too wide for the shared-memory tables");
+    for (int32_t& sl : S.slots) sl = std::min(sl, most);
     S.rounds.resize(1);
     S.setup_round(S.rounds[0], all, caps);
     QEG_CUDA(cudaStreamSynchronize(ctx->stream));
