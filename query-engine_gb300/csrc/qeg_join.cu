@@ -361,45 +361,6 @@ __global__ void popc_kernel(const unsigned long long* __restrict__ w, uint64_t n
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
 
-// Range of the non-null values of one integer key column.
-__global__ void minmax_kernel(DevCol c, uint64_t n, unsigned long long* out /* [0]=min enc, [1]=max enc, [2]=count */) {
-  unsigned long long mn = ~0ull, mx = 0, cnt = 0;
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
-    if (!col_valid(c, r)) continue;
-    const unsigned long long e = enc_i64(int_value(c, r));
-    mn = e < mn ? e : mn;
-    mx = e > mx ? e : mx;
-    ++cnt;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    mn = min(mn, __shfl_down_sync(0xffffffffu, mn, o));
-    mx = max(mx, __shfl_down_sync(0xffffffffu, mx, o));
-    cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-  }
-  // One set of global atomics per CTA (per-warp atomics on three words
-  // serialise at the L2).
-  __shared__ unsigned long long smn[32], smx[32], scn[32];
-  const unsigned warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    smn[warp] = mn;
-    smx[warp] = mx;
-    scn[warp] = cnt;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (unsigned w = 1; w < nwarps; ++w) {
-      mn = min(mn, smn[w]);
-      mx = max(mx, smx[w]);
-      cnt += scn[w];
-    }
-    if (cnt) {
-      atomicMin(out + 0, mn);
-      atomicMax(out + 1, mx);
-      atomicAdd(out + 2, cnt);
-    }
-  }
-}
-
 // Slot of a probe key, or -1 on a miss (NULL keys are filtered by the caller).
 __device__ __forceinline__ int64_t probe_slot(const JTable& T, const DevCol* kc, uint64_t p, const uint64_t* w,
                                               uint64_t h, uint32_t* err) {
@@ -1710,23 +1671,24 @@ __global__ void iota_kernel(uint32_t* __restrict__ out, uint64_t n) {
 }
 
 // ---- as-of join (tsx/asof.cpp) ---------------------------------------------
-// Build: every build row becomes an item (partition slot, timestamp - tmin,
-// row); rows with a NULL key or a NULL timestamp get the sentinel slot
-// `nslots` and sort after every partition (they never match,
-// tsx/asof.cpp:211-216). After a stable sort by (slot, timestamp) each
-// partition is one timestamp-ascending run whose equal timestamps keep the
-// build order, like the reference's sorted build lists (tsx/asof.cpp:158-219).
-struct AsofItemsK {
+// Build: every build row has a partition slot; rows with a NULL key or a NULL
+// timestamp get the sentinel slot `nslots` (they never match,
+// tsx/asof.cpp:211-216). A build side that is not in time order, or whose
+// probes do not suit the merge below, is sorted: items (slot, timestamp -
+// tmin, row), after whose stable sort each partition is one
+// timestamp-ascending run whose equal timestamps keep the build order, like
+// the reference's sorted build lists (tsx/asof.cpp:158-219).
+struct AsofScanK {
   DevCol key[kMaxKeys];
   int nkeys;
-  DevCol ts;
+  DevCol ts;              // (its validity is vbytes)
+  const uint8_t* vbytes;
   uint64_t n;
   JTable T;
   uint32_t nslots;
-  int64_t tmin;
-  uint64_t* lo;
-  uint32_t* hi;
-  uint32_t* val;
+  uint32_t* slot;
+  unsigned long long* out;  // {min enc, max enc, rows with a time, some row's time is below the previous row's,
+                            //  longest same-slot chain of a step, summed over kAsofSampleSteps sample steps}
   uint32_t* err;
 };
 
@@ -1745,30 +1707,338 @@ __device__ __forceinline__ int64_t asof_slot(const DevCol* key, int nkeys, const
   return load_key(key, nkeys, p, w, h) ? probe_slot(T, key, p, w, h, err) : -1;
 }
 
-__global__ void asof_items_kernel(const AsofItemsK P) {
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < P.n; r += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t slot = P.nslots;
-    uint64_t rel = 0;
-    if (col_valid(P.ts, r)) {
+constexpr int kAsofStep = 128;        // build rows per step of the merge
+constexpr int kAsofSampleSteps = 64;  // steps sampled for their longest same-slot chain
+
+// Where the merge is taken: tables of more slots leave fewer than three CTAs
+// to an SM; a warp walks its longest chain (the sampled mean stays below this
+// share of a step); and every probe batch reads the build side once more, which
+// a batch of fewer rows than that does not pay for.
+constexpr uint32_t kAsofMergeMaxSlots = 16384;
+constexpr uint64_t kAsofMaxChain = 48;
+constexpr uint64_t kAsofMinSlice = 2048;  // rows of both sides per slice
+
+// One pass over the build side: slots, time range, time order. The first
+// blocks also count, each for one sample step of the merge, the rows of the
+// slot that the step holds most often.
+__global__ void __launch_bounds__(256) asof_scan_kernel(const AsofScanK P) {
+  __shared__ uint32_t step[kAsofStep];
+  __shared__ unsigned int longest;
+  if (blockIdx.x < kAsofSampleSteps && P.n >= kAsofStep) {
+    if (threadIdx.x == 0) longest = 0;
+    if (threadIdx.x < kAsofStep) {
+      const uint64_t r = (P.n - kAsofStep) * blockIdx.x / kAsofSampleSteps + threadIdx.x;
       const int64_t s = asof_slot(P.key, P.nkeys, P.T, r, P.err);
-      if (s >= 0) {
-        slot = static_cast<uint32_t>(s);
-        rel = static_cast<uint64_t>(int_value(P.ts, r)) - static_cast<uint64_t>(P.tmin);
-      }
+      step[threadIdx.x] = s >= 0 ? static_cast<uint32_t>(s) : P.nslots;
     }
-    P.lo[r] = rel;
-    P.hi[r] = slot;
-    P.val[r] = static_cast<uint32_t>(r);
+    __syncthreads();
+    if (threadIdx.x < kAsofStep && step[threadIdx.x] < P.nslots) {
+      unsigned int same = 0;
+      for (int k = 0; k < kAsofStep; ++k) same += step[k] == step[threadIdx.x];
+      atomicMax(&longest, same);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(P.out + 4, static_cast<unsigned long long>(longest));
+  }
+  unsigned long long mn = ~0ull, mx = 0, cnt = 0;
+  bool bad = false;
+  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < P.n; r += (uint64_t)gridDim.x * blockDim.x) {
+    const int64_t t = int_value(P.ts, r);
+    if (r + 1 < P.n) bad |= t > int_value(P.ts, r + 1);
+    uint32_t slot = P.nslots;
+    if (P.vbytes[r]) {
+      const unsigned long long e = enc_i64(t);
+      mn = e < mn ? e : mn;
+      mx = e > mx ? e : mx;
+      ++cnt;
+      const int64_t s = asof_slot(P.key, P.nkeys, P.T, r, P.err);
+      if (s >= 0) slot = static_cast<uint32_t>(s);
+    }
+    P.slot[r] = slot;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    mn = min(mn, __shfl_down_sync(0xffffffffu, mn, o));
+    mx = max(mx, __shfl_down_sync(0xffffffffu, mx, o));
+    cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+  }
+  // One set of global atomics per CTA (per-warp atomics on three words
+  // serialise at the L2).
+  __shared__ unsigned long long smn[8], smx[8], scn[8];
+  if ((threadIdx.x & 31) == 0) {
+    smn[threadIdx.x >> 5] = mn;
+    smx[threadIdx.x >> 5] = mx;
+    scn[threadIdx.x >> 5] = cnt;
+  }
+  const int any_bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) {
+      mn = min(mn, smn[w]);
+      mx = max(mx, smx[w]);
+      cnt += scn[w];
+    }
+    if (cnt) {
+      atomicMin(P.out + 0, mn);
+      atomicMax(P.out + 1, mx);
+      atomicAdd(P.out + 2, cnt);
+    }
+    if (any_bad) P.out[3] = 1;
   }
 }
 
-// Sets *unsorted when some row's time is below the previous row's (times
-// without NULLs): a build side in time order only needs sorting by slot.
-__global__ void time_order_kernel(DevCol ts, uint64_t n, unsigned int* unsorted) {
-  bool bad = false;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i + 1 < n; i += (uint64_t)gridDim.x * blockDim.x)
-    bad |= int_value(ts, i) > int_value(ts, i + 1);
-  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(unsorted, 1u);
+// Sort items of the build rows, from their slots.
+__global__ void asof_items_kernel(const uint32_t* __restrict__ slot, DevCol ts, int64_t tmin, uint32_t nslots,
+                                  uint64_t n, uint64_t* __restrict__ lo, uint32_t* __restrict__ hi,
+                                  uint32_t* __restrict__ val) {
+  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t s = slot[r];
+    lo[r] = s < nslots ? static_cast<uint64_t>(int_value(ts, r)) - static_cast<uint64_t>(tmin) : 0;
+    hi[r] = s;
+    val[r] = static_cast<uint32_t>(r);
+  }
+}
+
+// Merge of two sides in time order. Sorting the build side by slot moves
+// every row several times and each probe row then searches its run in L2 (5M
+// quotes, 20M trades, 10k symbols: 500 us until the build side is sorted, 410
+// us for the searches; the merge takes 67 us at the build for the slots, and
+// 23 + 31 + 293 us per probe). When both sides are in time order already, the last build row of
+// every slot at a time is all a probe row needs, and one 4-byte entry per slot
+// fits shared memory. The merged sequence is cut into slices of equal length,
+// one CTA each:
+//   asof_heads_kernel   finds the slices' ends (a build row precedes the probe
+//                       rows of its own time) and takes, per slice and slot,
+//                       the last build row;
+//   asof_carry_kernel   turns these into the last build row before the slice;
+//   asof_merge_kernel   walks its slice in steps of kAsofStep build rows. Rows
+//                       of a step go into their slots' chains (one exchange
+//                       each, in any order); a probe row below the next
+//                       step's first time walks its slot's chain for the
+//                       latest row that is not after it, and below the step
+//                       the entry is final. Threads keep their probe row until
+//                       a step covers it, so a block of probe rows is read
+//                       once.
+// Probe rows in some other order are noticed (every neighbouring pair is
+// compared, a sample of them before the slices are walked): the caller then
+// drops the result and searches the sorted runs instead.
+struct AsofMergeK {
+  DevCol key[kMaxKeys];
+  int nkeys;
+  DevCol ts;   // probe times, no NULLs
+  uint64_t n;
+  JTable T;
+  DevCol bts;  // build times, ascending, no NULLs
+  const uint32_t* bslot;
+  uint32_t nbuild, nslots;
+  uint2* split;     // per slice end: build rows, probe rows before it
+  uint32_t* heads;  // [slice][slot]: last build row + 1, 0: none
+  uint32_t* unsorted;  // [0]: found before, [1]: found by the walk
+  int left, tol_set;
+  uint64_t tol;
+  uint32_t* match;
+  uint32_t* counts;
+  uint32_t* out_build;
+  uint32_t* err;
+};
+
+// Build rows among the first d rows of the merged sequence, found by one warp
+// in steps of 32 candidates.
+__device__ __forceinline__ uint32_t asof_split_at(const AsofMergeK& P, uint64_t d) {
+  const unsigned lane = threadIdx.x & 31u;
+  uint64_t lo = d > P.n ? d - P.n : 0, hi = d < P.nbuild ? d : P.nbuild;
+  while (lo < hi) {
+    const uint64_t stride = (hi - lo + 31) / 32, m = lo + lane * stride;
+    const bool before = m < hi && int_value(P.bts, m) <= int_value(P.ts, d - 1 - m);
+    const unsigned no = ~__ballot_sync(0xffffffffu, before);
+    const unsigned ones = no ? __ffs(no) - 1 : 32;
+    if (ones == 0) break;
+    const uint64_t end = lo + ones * stride;
+    lo += (ones - 1) * stride + 1;
+    hi = end < hi ? end : hi;
+  }
+  return static_cast<uint32_t>(lo);
+}
+
+__global__ void __launch_bounds__(256) asof_heads_kernel(const AsofMergeK P) {
+  extern __shared__ __align__(16) uint32_t amem[];
+  __shared__ uint32_t ends[2];
+  const uint64_t total = P.n + P.nbuild;
+  const unsigned warp = threadIdx.x >> 5;
+  if (warp < 2) {
+    const uint64_t c = blockIdx.x + warp;
+    const uint64_t d = total * c / gridDim.x;
+    const uint32_t q = asof_split_at(P, d);
+    if ((threadIdx.x & 31) == 0) {
+      ends[warp] = q;
+      if (warp == 0 || c == gridDim.x) P.split[c] = make_uint2(q, static_cast<uint32_t>(d - q));
+    }
+  }
+  for (uint32_t s = threadIdx.x; s < P.nslots; s += blockDim.x) amem[s] = 0;
+  // 256 neighbouring pairs of this block's share of the probe rows.
+  const uint64_t pr = P.n * blockIdx.x / gridDim.x + threadIdx.x;
+  if (pr + 1 < P.n && int_value(P.ts, pr) > int_value(P.ts, pr + 1)) P.unsorted[0] = 1;
+  __syncthreads();
+  for (uint64_t r = ends[0] + static_cast<uint64_t>(threadIdx.x); r < ends[1]; r += blockDim.x) {
+    const uint32_t s = P.bslot[r];
+    if (s < P.nslots) atomicMax(&amem[s], static_cast<uint32_t>(r) + 1u);
+  }
+  __syncthreads();
+  uint32_t* out = P.heads + static_cast<uint64_t>(blockIdx.x) * P.nslots;
+  for (uint32_t s = threadIdx.x; s < P.nslots; s += blockDim.x) out[s] = amem[s];
+}
+
+// Per slot the exclusive running maximum over the slices: a block takes 32
+// slots, each of its 8 warps an eighth of the slices.
+__global__ void __launch_bounds__(256) asof_carry_kernel(uint32_t* __restrict__ heads, uint32_t nslots,
+                                                         uint32_t slices) {
+  __shared__ uint32_t part[8][32];
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint64_t s = blockIdx.x * 32ull + lane;
+  const uint32_t c0 = slices * warp / 8, c1 = slices * (warp + 1) / 8;
+  uint32_t mx = 0;
+  if (s < nslots)
+#pragma unroll 8
+    for (uint32_t c = c0; c < c1; ++c) mx = max(mx, heads[c * static_cast<uint64_t>(nslots) + s]);
+  part[warp][lane] = mx;
+  __syncthreads();
+  if (s >= nslots) return;
+  uint32_t run = 0;
+  for (unsigned w = 0; w < warp; ++w) run = max(run, part[w][lane]);
+#pragma unroll 8
+  for (uint32_t c = c0; c < c1; ++c) {
+    uint32_t* at = heads + c * static_cast<uint64_t>(nslots) + s;
+    const uint32_t v = *at;
+    *at = run;
+    run = max(run, v);
+  }
+}
+
+// PLAIN: 8-byte times on both sides and one 4-byte key column without NULLs
+// and code map in a dense table: rows are fetched a block ahead of their use.
+template <bool PLAIN>
+__global__ void __launch_bounds__(256) asof_merge_kernel(const __grid_constant__ AsofMergeK P) {
+  extern __shared__ __align__(16) uint32_t amem[];
+  __shared__ long long next_time;
+  long long* qts = reinterpret_cast<long long*>(amem);
+  uint32_t* qprev = amem + 2 * kAsofStep;
+  uint32_t* table = qprev + kAsofStep;
+  if (P.unsorted[0]) return;  // (written by the launch before only)
+  const uint32_t tid = threadIdx.x;
+  const uint2 from = P.split[blockIdx.x], to = P.split[blockIdx.x + 1];
+  if (from.x > to.x || from.y > to.y) {  // only when the probe side is not in time order
+    if (tid == 0) P.unsorted[1] = 1;
+    return;
+  }
+  if (from.y == to.y) return;
+  {
+    const uint32_t* in = P.heads + static_cast<uint64_t>(blockIdx.x) * P.nslots;
+    for (uint32_t s = tid; s < P.nslots; s += blockDim.x) table[s] = in[s];
+  }
+  const int* pkey = static_cast<const int*>(P.key[0].data);
+  const long long* pts = static_cast<const long long*>(P.ts.data);
+  const long long* bts = static_cast<const long long*>(P.bts.data);
+  auto probe_time = [&](uint64_t p) -> long long { return PLAIN ? __ldg(pts + p) : int_value(P.ts, p); };
+  auto build_time = [&](uint64_t r) -> long long { return PLAIN ? __ldg(bts + r) : int_value(P.bts, r); };
+
+  // The next build rows (thread k: row k of the next step; thread 0 also the
+  // time after that step) and the next probe rows.
+  uint64_t base = from.x;  // the step in the chains: build rows [base, base + nq)
+  uint32_t nq = 0;
+  long long bt = 0, after = 0;
+  uint32_t bs = P.nslots, cur = P.nslots;
+  auto fetch_build = [&](uint64_t first) {
+    if (tid < kAsofStep && first + tid < to.x) {
+      bt = build_time(first + tid);
+      bs = __ldg(P.bslot + first + tid);
+    }
+    if (tid == 0 && first + kAsofStep < to.x) after = build_time(first + kAsofStep);
+  };
+  fetch_build(base);
+  long long limit = base < to.x ? build_time(base) : 0;  // probe rows below it are covered
+  bool last = base >= to.x;                                // every row is
+  uint64_t blk = from.y;
+  long long nt = 0, nbefore = 0;
+  int nkey = 0;
+  auto fetch_probe = [&](uint64_t first) {
+    const uint64_t p = first + tid;
+    if (p >= to.y) return;
+    nt = probe_time(p);
+    if (PLAIN) nkey = __ldg(pkey + p);
+    if ((tid & 31) == 0) nbefore = p > 0 ? probe_time(p - 1) : nt;
+  };
+  fetch_probe(blk);
+  bool pending = false, bad = false;
+  long long t = 0;
+  uint32_t slot = P.nslots;
+  auto take_probe = [&]() {
+    const uint64_t p = blk + tid;
+    pending = p < to.y;
+    t = nt;
+    long long before = __shfl_up_sync(0xffffffffu, t, 1);
+    if ((tid & 31) == 0) before = nbefore;
+    if (pending) {
+      bad |= before > t;
+      if (PLAIN) {
+        const int64_t s = static_cast<int64_t>(nkey) - P.T.dmin;
+        slot = s >= 0 && s < static_cast<int64_t>(P.nslots) ? static_cast<uint32_t>(s) : P.nslots;
+      } else {
+        const int64_t s = asof_slot(P.key, P.nkeys, P.T, p, P.err);
+        slot = s >= 0 ? static_cast<uint32_t>(s) : P.nslots;
+      }
+    }
+    fetch_probe(blk + blockDim.x);
+  };
+  take_probe();
+  __syncthreads();
+  for (;;) {
+    if (pending && (last || t < limit)) {
+      uint32_t m = kNullRow;
+      if (slot < P.nslots) {
+        uint32_t v = table[slot], best = 0;
+        while (v > base) {
+          const uint32_t k = v - 1 - static_cast<uint32_t>(base);
+          if (qts[k] <= t) best = max(best, v);
+          v = qprev[k];
+        }
+        if (best == 0) best = v;
+        if (best && P.tol_set) {
+          const long long tb = best > base ? qts[best - 1 - static_cast<uint32_t>(base)] : build_time(best - 1);
+          if (static_cast<uint64_t>(t) - static_cast<uint64_t>(tb) > P.tol) best = 0;
+        }
+        if (best) m = best - 1;
+      }
+      const uint64_t p = blk + tid;
+      if (P.left) {
+        P.out_build[p] = m;
+      } else {
+        P.match[p] = m;
+        P.counts[p] = m != kNullRow ? 1u : 0u;
+      }
+      pending = false;
+    }
+    if (!__syncthreads_or(pending)) {
+      blk += blockDim.x;
+      if (blk >= to.y) break;
+      take_probe();
+      continue;
+    }
+    // Rows are left over, so the slice has build rows left: the finished
+    // step's entries become their slots' last rows, the next step enters.
+    if (tid < nq && cur < P.nslots) atomicMax(&table[cur], static_cast<uint32_t>(base) + tid + 1u);
+    __syncthreads();
+    base += nq;
+    nq = static_cast<uint32_t>(to.x - base < kAsofStep ? to.x - base : kAsofStep);
+    if (tid < nq) {
+      cur = bs;
+      qts[tid] = bt;
+      if (cur < P.nslots) qprev[tid] = atomicExch(&table[cur], static_cast<uint32_t>(base) + tid + 1u);
+    }
+    if (tid == 0) next_time = after;
+    fetch_build(base + nq);
+    __syncthreads();
+    limit = next_time;
+    last = base + nq >= to.x;
+  }
+  if (__syncthreads_or(bad) && tid == 0) P.unsorted[1] = 1;
 }
 
 // Partition runs of the sorted items: run [beg[s], end[s]) of every slot that
@@ -2322,9 +2592,23 @@ struct JoinState {
   int64_t tol = 0;
   int64_t tmin = 0;
   uint32_t aslots = 0;
-  DevBuf ats, arow, aruns, asamp, tbits, amatch;
+  DevBuf ats, arow, aruns, asamp, amatch;
+  DevBuf bslot;                // partition slot of every build row
+  int alo_bits = 0;            // bits of the build side's relative times (0: in time order)
+  bool amerge = false;         // the build side suits the merge
+  bool asorted = false;        // the sorted runs are there
+  bool aprobe_unsorted = false;  // a probe batch was not in time order
   DevBuf krange;  // single integer key: [min enc, max enc, non-NULL count] over the appended batches
+  DevCol build_time() const {
+    DevCol c{};
+    c.type = btypes[btime];
+    c.data = bvals[btime].get();
+    c.all_valid = 1;
+    return c;
+  }
   void asof_build();
+  void asof_sort();
+  bool asof_merge(uint64_t n);
   void asof_probe(uint64_t n);
   void identity_output(uint64_t n);
 
@@ -2561,79 +2845,74 @@ void JoinState::finish_build() {
   if (asof) asof_build();
 }
 
-// As-of build: items per build row, a stable radix sort by (slot, timestamp),
-// partition runs from the per-slot counts.
+// As-of build: the slot of every build row, the time range and whether the
+// rows are in time order already.
 void JoinState::asof_build() {
   const int nk = static_cast<int>(bkeys.size());
   const uint64_t ns = nk == 0 ? 1 : slots();
   require(ns < 0xffffffffull, "as-of join: too many partitions");
   aslots = static_cast<uint32_t>(ns);
-  tbits.alloc(((nbuild + 63) / 64 + 1) * 8, ctx->stream);
-  if (nbuild) {
-    bytes_to_bits_kernel<<<grid_for(ctx, (nbuild / 64 + 1) * 32, 256, 8), 256, 0, ctx->stream>>>(
-        bvalid[btime].get<uint8_t>(), nbuild, tbits.get<uint64_t>());
-    ctx->launches++;
+  if (nbuild == 0) {
+    asof_sort();
+    return;
   }
-  DevCol ts{};
-  ts.type = btypes[btime];
-  ts.data = bvals[btime].get();
-  ts.validity = tbits.get<uint64_t>();
-  // Timestamp range of the build side (relative timestamps need its low end).
-  DevBuf mm(24, ctx->stream);
-  unsigned long long init[3] = {~0ull, 0ull, 0ull};
-  QEG_CUDA(cudaMemcpyAsync(mm.get(), init, 24, cudaMemcpyHostToDevice, ctx->stream));
-  if (nbuild) {
-    minmax_kernel<<<grid_for(ctx, nbuild, 256, 8), 256, 0, ctx->stream>>>(ts, nbuild, mm.get<unsigned long long>());
-    ctx->launches++;
-  }
-  unsigned long long r[3];
-  QEG_CUDA(cudaMemcpyAsync(r, mm.get(), 24, cudaMemcpyDeviceToHost, ctx->stream));
-  QEG_CUDA(cudaStreamSynchronize(ctx->stream));
+  bslot.alloc(nbuild * 4, ctx->stream);
+  DevBuf out(40, ctx->stream);
+  QEG_CUDA(cudaMemsetAsync(out.get(), 0xff, 8, ctx->stream));
+  QEG_CUDA(cudaMemsetAsync(out.get<uint8_t>() + 8, 0, 32, ctx->stream));
+  AsofScanK P{};
+  P.nkeys = nk;
+  for (int j = 0; j < nk; ++j) P.key[j] = store_key(j);
+  P.ts = build_time();
+  P.vbytes = bvalid[btime].get<uint8_t>();
+  P.n = nbuild;
+  if (nk) P.T = table();
+  P.nslots = aslots;
+  P.slot = bslot.get<uint32_t>();
+  P.out = out.get<unsigned long long>();
+  P.err = static_cast<uint32_t*>(ctx->dev_err.get());
+  asof_scan_kernel<<<grid_for(ctx, nbuild, 256, 8), 256, 0, ctx->stream>>>(P);
+  ctx->launches++;
+  QEG_CUDA(cudaGetLastError());
+  uint64_t r[5];
+  read_words_and_error(ctx, out.get(), 5, r);
   tmin = r[2] ? dec_i64(r[0]) : 0;
   const uint64_t range = r[2] ? r[1] - r[0] : 0;
-  int lo_bits = 0, hi_bits = 0;
-  while (lo_bits < 64 && (range >> lo_bits) != 0) ++lo_bits;
-  while (hi_bits < 32 && (static_cast<uint64_t>(aslots) >> hi_bits) != 0) ++hi_bits;
+  while (alo_bits < 64 && (range >> alo_bits) != 0) ++alo_bits;
+  // A build side in time order (no NULL times) only needs its stable sort by
+  // slot, if any: time order within every slot is kept.
+  const bool ordered = r[2] == nbuild && r[3] == 0;
+  if (ordered) alo_bits = 0;
+  const uint64_t steps = std::min<uint64_t>(kAsofSampleSteps, grid_for(ctx, nbuild, 256, 8));
+  amerge = ordered && nbuild >= kAsofStep && aslots <= kAsofMergeMaxSlots && r[4] <= kAsofMaxChain * steps;
+  if (!amerge) asof_sort();
+}
 
+// The build side sorted by (slot, time): items per build row, a stable radix
+// sort, partition runs. At once when the merge cannot serve this build side,
+// otherwise on the first probe that the merge does not take.
+void JoinState::asof_sort() {
+  if (asorted) return;
+  asorted = true;
+  int hi_bits = 0;
+  while (hi_bits < 32 && (static_cast<uint64_t>(aslots) >> hi_bits) != 0) ++hi_bits;
   const uint64_t n = nbuild;
-  // A build side already in time order (no NULL times) only needs its stable
-  // sort by slot: time order within every slot is kept.
-  if (n > 1 && r[2] == n) {
-    DevBuf flag(4, ctx->stream);
-    QEG_CUDA(cudaMemsetAsync(flag.get(), 0, 4, ctx->stream));
-    time_order_kernel<<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>(ts, n, flag.get<unsigned int>());
-    ctx->launches++;
-    uint32_t unsorted = 1;
-    QEG_CUDA(cudaMemcpyAsync(&unsorted, flag.get(), 4, cudaMemcpyDeviceToHost, ctx->stream));
-    QEG_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (!unsorted) lo_bits = 0;
-  }
   DevBuf a_lo(std::max<uint64_t>(n, 1) * 8, ctx->stream), b_lo(std::max<uint64_t>(n, 1) * 8, ctx->stream);
   DevBuf a_hi(std::max<uint64_t>(n, 1) * 4, ctx->stream), b_hi(std::max<uint64_t>(n, 1) * 4, ctx->stream);
   DevBuf a_val(std::max<uint64_t>(n, 1) * 4, ctx->stream), b_val(std::max<uint64_t>(n, 1) * 4, ctx->stream);
   if (n) {
-    AsofItemsK P{};
-    P.nkeys = nk;
-    for (int j = 0; j < nk; ++j) P.key[j] = store_key(j);
-    P.ts = ts;
-    P.n = n;
-    if (nk) P.T = table();
-    P.nslots = aslots;
-    P.tmin = tmin;
-    P.lo = a_lo.get<uint64_t>();
-    P.hi = a_hi.get<uint32_t>();
-    P.val = a_val.get<uint32_t>();
-    P.err = static_cast<uint32_t*>(ctx->dev_err.get());
-    asof_items_kernel<<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>(P);
+    asof_items_kernel<<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>(
+        bslot.get<uint32_t>(), build_time(), tmin, aslots, n, a_lo.get<uint64_t>(), a_hi.get<uint32_t>(),
+        a_val.get<uint32_t>());
     ctx->launches++;
     QEG_CUDA(cudaGetLastError());
   }
   SortItems A{a_lo.get<uint64_t>(), a_hi.get<uint32_t>(), a_val.get<uint32_t>()};
   SortItems B{b_lo.get<uint64_t>(), b_hi.get<uint32_t>(), b_val.get<uint32_t>()};
-  const SortItems R = radix_sort_items(ctx, A, B, n, lo_bits, hi_bits);
-  aruns.alloc(ns * 8, ctx->stream);
+  const SortItems R = radix_sort_items(ctx, A, B, n, alo_bits, hi_bits);
+  aruns.alloc(static_cast<uint64_t>(aslots) * 8, ctx->stream);
   asamp.alloc((n / kAsofSample + 1) * 8, ctx->stream);
-  QEG_CUDA(cudaMemsetAsync(aruns.get(), 0, ns * 8, ctx->stream));
+  QEG_CUDA(cudaMemsetAsync(aruns.get(), 0, static_cast<uint64_t>(aslots) * 8, ctx->stream));
   if (n) {
     asof_runs_kernel<<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>(
         R.hi, R.lo, n, aslots, aruns.get<uint2>(), asamp.get<uint64_t>());
@@ -2918,47 +3197,98 @@ void JoinState::identity_output(uint64_t n) {
   QEG_CUDA(cudaGetLastError());
 }
 
-void JoinState::asof_probe(uint64_t n) {
-  AsofProbeK P{};
+// Takes a probe batch by the merge: false when its shape does not suit, or
+// when it turns out not to be in time order.
+bool JoinState::asof_merge(uint64_t n) {
+  if (!amerge || aprobe_unsorted || !probe_staged[ptime].dev.all_valid || n < nbuild) return false;
+  AsofMergeK P{};
   P.nkeys = static_cast<int>(pkeys.size());
   for (int j = 0; j < P.nkeys; ++j) P.key[j] = probe_staged[pkeys[j]].dev;
   P.ts = probe_staged[ptime].dev;
   P.n = n;
   if (P.nkeys) P.T = table();
-  P.tmin = tmin;
-  P.ats = ats.get<uint64_t>();
-  P.arow = arow.get<uint32_t>();
-  P.aruns = aruns.get<uint2>();
-  P.asamp = asamp.get<uint64_t>();
+  P.bts = build_time();
+  P.bslot = bslot.get<uint32_t>();
+  P.nbuild = static_cast<uint32_t>(nbuild);
+  P.nslots = aslots;
   P.left = join_type == QEG_LEFT;
   P.tol_set = tol_set;
   P.tol = static_cast<uint64_t>(tol);
+  P.match = amatch.get<uint32_t>();
+  P.counts = counts.get<uint32_t>();
+  P.out_build = P.left ? out_build.get<uint32_t>() : nullptr;
   P.err = static_cast<uint32_t*>(ctx->dev_err.get());
-  {
+  const auto wide = [](int32_t type) { return type == QEG_I64 || type == QEG_TS; };
+  const DevCol& k = P.key[0];
+  const bool plain = wide(P.ts.type) && wide(P.bts.type) && P.nkeys == 1 && strategy == QEG_JOIN_DENSE &&
+                     k.all_valid && k.code_map == nullptr && (k.type == QEG_I32 || k.type == QEG_STR);
+  const auto merge = plain ? asof_merge_kernel<true> : asof_merge_kernel<false>;
+  const size_t heads_smem = static_cast<size_t>(aslots) * 4, smem = heads_smem + kAsofStep * 12;
+  raise_dynamic_smem(reinterpret_cast<const void*>(asof_heads_kernel), heads_smem);
+  raise_dynamic_smem(reinterpret_cast<const void*>(merge), smem);
+  const int per_sm = std::max(1, blocks_per_sm(reinterpret_cast<const void*>(merge), 256, smem));
+  const unsigned slices = static_cast<unsigned>(std::max<uint64_t>(
+      1, std::min<uint64_t>((n + nbuild) / kAsofMinSlice, static_cast<uint64_t>(ctx->sms) * per_sm)));
+  DevBuf split((slices + 1) * 8, ctx->stream), heads(static_cast<uint64_t>(slices) * aslots * 4, ctx->stream),
+      flags(8, ctx->stream);
+  P.split = split.get<uint2>();
+  P.heads = heads.get<uint32_t>();
+  P.unsorted = flags.get<uint32_t>();
+  QEG_CUDA(cudaMemsetAsync(flags.get(), 0, 8, ctx->stream));
+  asof_heads_kernel<<<slices, 256, heads_smem, ctx->stream>>>(P);
+  asof_carry_kernel<<<(aslots + 31) / 32, 256, 0, ctx->stream>>>(P.heads, aslots, slices);
+  merge<<<slices, 256, smem, ctx->stream>>>(P);
+  ctx->launches += 3;
+  QEG_CUDA(cudaGetLastError());
+  uint64_t unsorted = 0;
+  read_words_and_error(ctx, flags.get(), 1, &unsorted);
+  aprobe_unsorted = unsorted != 0;
+  return !aprobe_unsorted;
+}
+
+void JoinState::asof_probe(uint64_t n) {
+  const bool left = join_type == QEG_LEFT;
+  if (left) {
+    out_build.alloc(n * 4, ctx->stream);
+  } else {
+    amatch.alloc(n * 4, ctx->stream);
+    counts.alloc(n * 4, ctx->stream);
+    starts.alloc((n + 1) * 8, ctx->stream);
+  }
+  AsofProbeK P{};
+  P.n = n;
+  P.match = amatch.get<uint32_t>();
+  P.counts = counts.get<uint32_t>();
+  const unsigned g = grid_for(ctx, n, 256, 8);
+  if (!asof_merge(n)) {
+    asof_sort();
+    P.nkeys = static_cast<int>(pkeys.size());
+    for (int j = 0; j < P.nkeys; ++j) P.key[j] = probe_staged[pkeys[j]].dev;
+    P.ts = probe_staged[ptime].dev;
+    if (P.nkeys) P.T = table();
+    P.tmin = tmin;
+    P.ats = ats.get<uint64_t>();
+    P.arow = arow.get<uint32_t>();
+    P.aruns = aruns.get<uint2>();
+    P.asamp = asamp.get<uint64_t>();
+    P.left = left;
+    P.tol_set = tol_set;
+    P.tol = static_cast<uint64_t>(tol);
+    P.out_build = left ? out_build.get<uint32_t>() : nullptr;
+    P.err = static_cast<uint32_t*>(ctx->dev_err.get());
     const char* e = std::getenv("QEG_ASOF_HINT_BITS");
     P.hint_bits = e ? std::max(6, std::min(12, std::atoi(e))) : kAsofHintBits;
-  }
-  const size_t hsb = static_cast<size_t>(8) << P.hint_bits;  // slot + position per entry
-  const unsigned g = grid_for(ctx, n, 256, 8);
-  if (P.left) {
-    out_build.alloc(n * 4, ctx->stream);
-    P.out_build = out_build.get<uint32_t>();
+    const size_t hsb = static_cast<size_t>(8) << P.hint_bits;  // slot + position per entry
     asof_probe_kernel<<<g, 256, hsb, ctx->stream>>>(P);
     ctx->launches++;
     QEG_CUDA(cudaGetLastError());
+    if (left) check_device_error(ctx);
+  }
+  if (left) {
     identity_output(n);
-    check_device_error(ctx);
     nout = n;
     return;
   }
-  amatch.alloc(n * 4, ctx->stream);
-  counts.alloc(n * 4, ctx->stream);
-  starts.alloc((n + 1) * 8, ctx->stream);
-  P.match = amatch.get<uint32_t>();
-  P.counts = counts.get<uint32_t>();
-  asof_probe_kernel<<<g, 256, hsb, ctx->stream>>>(P);
-  ctx->launches++;
-  QEG_CUDA(cudaGetLastError());
   const uint64_t total = exclusive_scan(ctx, counts.get<uint32_t>(), n, starts.get<uint64_t>());
   out_probe.alloc(std::max<uint64_t>(total, 1) * 4, ctx->stream);
   out_build.alloc(std::max<uint64_t>(total, 1) * 4, ctx->stream);
