@@ -97,6 +97,8 @@ struct SketchResult {
   double total_rows = 0;
   double null_frac = 0;
   double top_share[16] = {};  // share of sampled rows in the top 2^i candidates
+  bool have_net = false;      // the sketch's launch ran the estimator network
+  float net[2] = {};          // its outputs for `features`
 };
 
 // Builds the sketch of one key column (qeg_sketch.cu).

@@ -52,7 +52,11 @@ double learned_groups(const SketchResult& s, float out0, double deadband) {
 
 bool learned_estimate(qeg_ctx* ctx, const SketchResult& s, double* groups, double* hot_share) {
   if (!ctx->mlp || !ctx->mlp->loaded) return false;
-  const std::vector<float> y = predict_host(ctx, s.features, 1);
+  float y[kOut] = {s.net[0], s.net[1]};
+  if (!s.have_net) {
+    const std::vector<float> p = predict_host(ctx, s.features, 1);
+    std::copy(p.begin(), p.end(), y);
+  }
   double g = learned_groups(s, y[0], ctx->mlp->deadband);
   // Never below what the sample itself proves, never above the non-null rows.
   const double nonnull = s.total_rows * (1.0 - s.null_frac);

@@ -4,11 +4,13 @@
 // table and picks its strategy (the reference sizes by growth only,
 // ops/hashtable.h:83-94; results never depend on the estimate, because an
 // overflowing table is grown and the affected rows replayed).
+#include <cuda_bf16.h>
+
 #include <algorithm>
 #include <cmath>
-#include <functional>
 
 #include "qeg_agg.h"
+#include "qeg_mlp.h"
 
 namespace qeg {
 
@@ -22,6 +24,16 @@ constexpr int kCandLocal = 1024;
 constexpr int kCandGlobal = 8192;
 constexpr int kSampleBlock = 256;
 
+// What the host needs of a sketch: whole numbers, from which it computes the
+// features, and the network's outputs for them.
+struct SketchOut {
+  uint32_t hist[66];             // registers by value (the last: padding)
+  unsigned long long top[12];    // sum of the 2^i largest candidate estimates
+  unsigned long long f2;         // sum of squares of the first count-min row
+  unsigned long long rows, nulls;
+  float net[2];
+};
+
 struct SketchK {
   DevCol key;
   const uint32_t* sel;
@@ -33,6 +45,10 @@ struct SketchK {
   unsigned long long* cand_key;  // kCandGlobal
   unsigned long long* cand_cnt;  // kCandGlobal
   unsigned long long* stats;     // [0] sampled rows, [1] sampled nulls
+  unsigned int* done;            // CTAs that have merged their part
+  SketchOut* out;
+  const __nv_bfloat16* net;      // estimator weights, or nullptr
+  float log_rows, log_total, sampled;  // features 75..77 (known before the sample is read)
   uint32_t* err;
 };
 
@@ -43,6 +59,176 @@ __device__ __forceinline__ uint64_t sketch_hash(uint64_t w) { return mix64(w ^ 0
 // latency of the loads and shared-memory atomics (256 threads: 67 us for 1M
 // sampled rows).
 constexpr int kSketchThreads = 1024;
+
+// The merged sketch's host part, by the last CTA: register histogram,
+// candidates ranked by their count-min estimates, features, network. On the
+// host this took up to 0.3 ms (225 KB copied, 8192 candidates sorted, and the
+// network as a round trip of its own); here it adds 10 to 25 us to the launch.
+__device__ void sketch_finish(const SketchK& P, uint32_t* sh) {
+  uint32_t* ranked = sh;                                     // kCandGlobal
+  __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(sh + kCandGlobal);  // kParams
+  uint32_t* cms = sh + kHllM;                                // kCmsDepth * kCmsWidth
+  static_assert(kCandGlobal * 4 + kParams * 2 <= kHllM * 4, "candidates and weights take the registers' place");
+  __shared__ uint32_t hist[66], nranked;
+  __shared__ unsigned long long top[12], f2;
+  __shared__ float f[kIn], h1[kHid], h2[kHid];
+  const unsigned tid = threadIdx.x, lane = tid & 31u;
+  if (tid < 66) hist[tid] = 0;
+  if (tid < 12) top[tid] = 0;
+  if (tid == 0) {
+    nranked = 0;
+    f2 = 0;
+  }
+  if (P.net)
+    for (unsigned i = tid; i < kParams; i += blockDim.x) w[i] = P.net[i];
+  for (unsigned i = tid; i < kCmsDepth * kCmsWidth; i += blockDim.x) cms[i] = __ldcg(P.cms + i);
+  __syncthreads();
+  for (unsigned i = tid; i < kHllM; i += blockDim.x) {  // (kHllM is a multiple of the block)
+    const uint32_t r = min(__ldcg(P.hll + i), 64u);
+    const unsigned same = __match_any_sync(0xffffffffu, r);
+    if (static_cast<unsigned>(__ffs(same)) == lane + 1) atomicAdd(&hist[r], static_cast<unsigned>(__popc(same)));
+  }
+  unsigned long long sq = 0;
+  for (unsigned c = tid; c < kCmsWidth; c += blockDim.x) sq += static_cast<unsigned long long>(cms[c]) * cms[c];
+  for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
+  if (lane == 0) atomicAdd(&f2, sq);
+  for (unsigned i = tid; i < kCandGlobal; i += blockDim.x) {
+    const unsigned long long kk = __ldcg(P.cand_key + i);
+    if (!kk) continue;
+    const uint64_t h = sketch_hash(kk - 1);
+    uint32_t best = UINT32_MAX;
+#pragma unroll
+    for (int d = 0; d < kCmsDepth; ++d) {
+      const uint32_t c = static_cast<uint32_t>(mix64(h + 0x9E3779B97F4A7C15ull * (d + 1)) >> 40) & (kCmsWidth - 1);
+      best = min(best, cms[d * kCmsWidth + c]);
+    }
+    ranked[atomicAdd(&nranked, 1u)] = best;
+  }
+  __syncthreads();
+  // Descending bitonic sort, padded with zeros to a power of two. A thread
+  // holds 8 neighbours, a warp 256: steps within them are exchanges of
+  // registers and lanes, the wider ones go through shared memory (step by step
+  // there, 8192 candidates took 45 us).
+  const unsigned n = nranked;
+  unsigned size = 256;
+  while (size < n) size *= 2;
+  for (unsigned i = n + tid; i < size; i += blockDim.x) ranked[i] = 0;
+  __syncthreads();
+  for (unsigned k = 2; k <= size; k <<= 1) {
+    for (unsigned j = k >> 1; j >= 256; j >>= 1) {
+      for (unsigned q = tid; q < size / 2; q += blockDim.x) {
+        const unsigned i = 2 * q - (q & (j - 1)), x = i + j;
+        const uint32_t a = ranked[i], b = ranked[x];
+        if ((i & k) == 0 ? a < b : a > b) {
+          ranked[i] = b;
+          ranked[x] = a;
+        }
+      }
+      __syncthreads();
+    }
+    if (tid * 8 < size) {  // whole warps: size is a multiple of 256
+      uint32_t v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = ranked[tid * 8 + e];
+      for (unsigned j = min(k >> 1, 128u); j >= 8; j >>= 1) {
+        const bool larger = ((tid * 8 & k) == 0) == ((tid * 8 & j) == 0);  // this end takes the larger one
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const uint32_t o = __shfl_xor_sync(0xffffffffu, v[e], j / 8);
+          v[e] = larger ? max(v[e], o) : min(v[e], o);
+        }
+      }
+#pragma unroll
+      for (unsigned j = 4; j >= 1; j >>= 1) {
+        if (j >= k) continue;
+#pragma unroll
+        for (unsigned e = 0; e < 8; ++e) {
+          if (e & j) continue;
+          const uint32_t lo = min(v[e], v[e | j]), hi = max(v[e], v[e | j]);
+          const bool down = ((tid * 8 + e) & k) == 0;
+          v[e] = down ? hi : lo;
+          v[e | j] = down ? lo : hi;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ranked[tid * 8 + e] = v[e];
+    }
+    __syncthreads();
+  }
+  // The estimate at position j counts toward every prefix longer than j:
+  // bucket bitlength(j) and above (the same for 32 aligned positions from 32 on).
+  for (unsigned j = tid; j < 2048 && j - lane < size; j += blockDim.x) {
+    const int b = j == 0 ? 0 : 32 - __clz(j);
+    unsigned long long v = ranked[j];
+    if (j < 32) {
+      atomicAdd(&top[b], v);
+    } else {
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) atomicAdd(&top[b], v);
+    }
+  }
+  __syncthreads();
+  if (tid == 0)
+    for (int i = 1; i < 12; ++i) top[i] += top[i - 1];
+  __syncthreads();
+  const unsigned long long rows = __ldcg(P.stats), nulls = __ldcg(P.stats + 1);
+  if (P.net) {
+    // Features as the host computes them (sketch_features).
+    const double nonnull = static_cast<double>(rows) - static_cast<double>(nulls);
+    if (tid < kIn) {
+      float v = 0;
+      if (tid < 64) {
+        v = static_cast<float>(hist[tid]) / kHllM;
+        if (tid == 63) v += static_cast<float>(hist[64]) / kHllM;
+      } else if (tid < 74) {
+        v = nonnull > 0 ? static_cast<float>(fmin(1.0, static_cast<double>(top[tid - 64]) / nonnull)) : 0.f;
+      } else if (tid == 74) {
+        v = nonnull > 0 ? static_cast<float>(static_cast<double>(f2) / (nonnull * nonnull)) : 0.f;
+      } else if (tid == 75) {
+        v = P.log_rows;
+      } else if (tid == 76) {
+        v = P.log_total;
+      } else if (tid == 77) {
+        v = P.sampled;
+      } else if (tid == 78) {
+        v = rows ? static_cast<float>(static_cast<double>(nulls) / static_cast<double>(rows)) : 0.f;
+      } else if (nonnull > 0) {
+        double sum = 0;
+        for (int r = 0; r <= 64; ++r) sum += hist[r] * ldexp(1.0, -r);
+        const double m = kHllM;
+        double e = (0.7213 / (1.0 + 1.079 / m)) * m * m / sum;
+        if (e <= 2.5 * m && hist[0] > 0) e = m * log(m / hist[0]);
+        v = static_cast<float>(fmin(1.0, e / nonnull));
+      }
+      f[tid] = v;
+    }
+    __syncthreads();
+    if (tid < kHid) {
+      float acc = __bfloat162float(w[kOffB1 + tid]);
+      for (int i = 0; i < kIn; ++i) acc = fmaf(f[i], __bfloat162float(w[kOffW1 + tid * kIn + i]), acc);
+      h1[tid] = fmaxf(acc, 0.f);
+    }
+    __syncthreads();
+    if (tid < kHid) {
+      float acc = __bfloat162float(w[kOffB2 + tid]);
+      for (int i = 0; i < kHid; ++i) acc = fmaf(h1[i], __bfloat162float(w[kOffW2 + tid * kHid + i]), acc);
+      h2[tid] = fmaxf(acc, 0.f);
+    }
+    __syncthreads();
+    if (tid < kOut) {
+      float acc = __bfloat162float(w[kOffB3 + tid]);
+      for (int i = 0; i < kHid; ++i) acc = fmaf(h2[i], __bfloat162float(w[kOffW3 + tid * kHid + i]), acc);
+      P.out->net[tid] = acc;
+    }
+  }
+  if (tid < 66) P.out->hist[tid] = hist[tid];
+  if (tid < 12) P.out->top[tid] = top[tid];
+  if (tid == 0) {
+    P.out->f2 = f2;
+    P.out->rows = rows;
+    P.out->nulls = nulls;
+  }
+}
 
 __global__ void __launch_bounds__(kSketchThreads) sketch_kernel(const SketchK P) {
   extern __shared__ uint32_t sh[];
@@ -101,13 +287,26 @@ __global__ void __launch_bounds__(kSketchThreads) sketch_kernel(const SketchK P)
       s = (s + 1) & (kCandLocal - 1);
     }
   }
-  atomicAdd(&s_rows, rows);
-  atomicAdd(&s_nulls, nulls);
+  for (int o = 16; o > 0; o >>= 1) {
+    rows += __shfl_down_sync(0xffffffffu, rows, o);
+    nulls += __shfl_down_sync(0xffffffffu, nulls, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&s_rows, rows);
+    atomicAdd(&s_nulls, nulls);
+  }
   __syncthreads();
-  for (int i = threadIdx.x; i < kHllM; i += blockDim.x)
+  // Every CTA starts at its own place: all of them adding to the same words in
+  // the same order would queue up at the L2.
+  const unsigned turn = blockIdx.x * 1664u;
+  for (int k = threadIdx.x; k < kHllM; k += blockDim.x) {
+    const unsigned i = (k + turn) & (kHllM - 1);
     if (hll[i]) atomicMax(&P.hll[i], hll[i]);
-  for (int i = threadIdx.x; i < kCmsDepth * kCmsWidth; i += blockDim.x)
+  }
+  for (int k = threadIdx.x; k < kCmsDepth * kCmsWidth; k += blockDim.x) {
+    const unsigned i = (k + turn) & (kCmsDepth * kCmsWidth - 1);
     if (cms[i]) atomicAdd(&P.cms[i], cms[i]);
+  }
   for (int i = threadIdx.x; i < kCandLocal; i += blockDim.x) {
     if (cc[i] < 2) continue;
     const unsigned long long kk = ck[i];
@@ -125,6 +324,14 @@ __global__ void __launch_bounds__(kSketchThreads) sketch_kernel(const SketchK P)
     atomicAdd(&P.stats[0], s_rows);
     atomicAdd(&P.stats[1], s_nulls);
   }
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(P.done, 1u) + 1 == gridDim.x;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  sketch_finish(P, sh);
 }
 
 // Exact counts of the sampled keys (the heavy-hitter candidates of a GROUP BY
@@ -198,7 +405,7 @@ __global__ void heavy_compact_kernel(const HeavyK P) {
 }
 
 // HyperLogLog estimate from the number of registers of each value.
-double hll_estimate(const uint32_t (&regs)[65]) {
+double hll_estimate(const uint32_t (&regs)[66]) {
   const double m = kHllM;
   double sum = 0;
   for (int r = 0; r <= 64; ++r) sum += regs[r] * std::ldexp(1.0, -r);
@@ -230,82 +437,73 @@ void sketch_key_column(qeg_ctx* ctx, const DevCol& key, const uint32_t* sel, uin
   out.total_rows = static_cast<double>(nrows);
   uint64_t stride, nblocks;
   sample_blocks(nrows, sample_target, stride, nblocks);
-  const size_t words = kHllM + kCmsDepth * kCmsWidth;
-  DevBuf buf(words * 4 + kCandGlobal * 16 + 16, ctx->stream);
-  QEG_CUDA(cudaMemsetAsync(buf.get(), 0, buf.bytes(), ctx->stream));
-  SketchK P{};
-  P.key = key;
-  P.sel = sel;
-  P.nrows = nrows;
-  P.len = len;
-  P.stride = stride;
-  P.nblocks = nblocks;
-  P.hll = buf.get<uint32_t>();
-  P.cms = P.hll + kHllM;
-  P.cand_key = reinterpret_cast<unsigned long long*>(P.cms + kCmsDepth * kCmsWidth);
-  P.cand_cnt = P.cand_key + kCandGlobal;
-  P.stats = P.cand_cnt + kCandGlobal;
-  P.err = static_cast<uint32_t*>(ctx->dev_err.get());
-  const size_t sb = words * 4 + kCandLocal * 12;
-  raise_dynamic_smem(reinterpret_cast<const void*>(sketch_kernel), sb);
-  constexpr uint64_t kPer = kSketchThreads / kSampleBlock;
-  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((nblocks + kPer - 1) / kPer, ctx->sms));
+  // Rows of the sample blocks: all but the last are whole.
+  uint64_t sampled = 0;
   if (nblocks > 0) {
+    const uint64_t whole = nrows >= kSampleBlock ? std::min(nblocks, (nrows - kSampleBlock) / stride + 1) : 0;
+    sampled = whole * kSampleBlock + (whole < nblocks ? nrows - whole * stride : 0);
+  }
+  SketchOut o{};
+  o.hist[0] = kHllM;  // (no rows: an empty sketch)
+  out.have_net = false;
+  const double log_rows = std::log2(1.0 + static_cast<double>(sampled)) / 32.0;
+  const double log_total = std::log2(1.0 + out.total_rows) / 32.0;
+  const double share = out.total_rows > 0 ? static_cast<double>(sampled) / out.total_rows : 1.0;
+  if (nblocks > 0) {
+    const size_t words = kHllM + kCmsDepth * kCmsWidth;
+    static_assert(sizeof(SketchOut) % 8 == 0, "copied in words");
+    const size_t head = words * 4 + kCandGlobal * 16 + 24;
+    DevBuf buf(head + sizeof(SketchOut), ctx->stream);
+    QEG_CUDA(cudaMemsetAsync(buf.get(), 0, head, ctx->stream));
+    SketchK P{};
+    P.key = key;
+    P.sel = sel;
+    P.nrows = nrows;
+    P.len = len;
+    P.stride = stride;
+    P.nblocks = nblocks;
+    P.hll = buf.get<uint32_t>();
+    P.cms = P.hll + kHllM;
+    P.cand_key = reinterpret_cast<unsigned long long*>(P.cms + kCmsDepth * kCmsWidth);
+    P.cand_cnt = P.cand_key + kCandGlobal;
+    P.stats = P.cand_cnt + kCandGlobal;
+    P.done = reinterpret_cast<unsigned int*>(P.stats + 2);
+    P.out = reinterpret_cast<SketchOut*>(P.stats + 3);
+    P.net = ctx->mlp && ctx->mlp->loaded ? ctx->mlp->wbf.get<__nv_bfloat16>() : nullptr;
+    P.log_rows = static_cast<float>(log_rows);
+    P.log_total = static_cast<float>(log_total);
+    P.sampled = static_cast<float>(share);
+    P.err = static_cast<uint32_t*>(ctx->dev_err.get());
+    const size_t sb = words * 4 + kCandLocal * 12;
+    raise_dynamic_smem(reinterpret_cast<const void*>(sketch_kernel), sb);
+    constexpr uint64_t kPer = kSketchThreads / kSampleBlock;
+    const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((nblocks + kPer - 1) / kPer, ctx->sms));
     sketch_kernel<<<grid, kSketchThreads, sb, ctx->stream>>>(P);
     ctx->launches++;
     QEG_CUDA(cudaGetLastError());
+    read_words_and_error(ctx, P.out, sizeof(SketchOut) / 8, reinterpret_cast<uint64_t*>(&o));
+    out.have_net = P.net != nullptr;
+    out.net[0] = o.net[0];
+    out.net[1] = o.net[1];
   }
-  // Registers, sketch, candidates and totals lie back to back: one copy into
-  // page-locked memory, with the error word.
-  std::vector<uint64_t> host((words * 4 + kCandGlobal * 16 + 16) / 8);
-  read_words_and_error(ctx, buf.get(), host.size(), host.data());
-  const uint32_t* regs = reinterpret_cast<const uint32_t*>(host.data());
-  const uint64_t* cand = host.data() + words / 2;
 
-  uint32_t hll[65] = {};  // registers by value
-  for (int i = 0; i < kHllM; ++i) ++hll[std::min<uint32_t>(regs[i], 64)];
-  out.sample_rows = static_cast<double>(cand[2 * kCandGlobal]);
-  const double nulls = static_cast<double>(cand[2 * kCandGlobal + 1]);
+  out.sample_rows = static_cast<double>(o.rows);
+  const double nulls = static_cast<double>(o.nulls);
   out.null_frac = out.sample_rows > 0 ? nulls / out.sample_rows : 0;
   const double nonnull = out.sample_rows - nulls;
-  out.hll_estimate = nonnull > 0 ? hll_estimate(hll) : 0;
-
-  // Candidates ranked by their count-min estimate.
-  auto cms_est = [&](uint64_t w) {
-    const uint64_t h = mix64(w ^ 0x243F6A8885A308D3ull);
-    uint32_t best = UINT32_MAX;
-    for (int d = 0; d < kCmsDepth; ++d) {
-      const uint32_t c = static_cast<uint32_t>(mix64(h + 0x9E3779B97F4A7C15ull * (d + 1)) >> 40) & (kCmsWidth - 1);
-      best = std::min(best, regs[kHllM + d * kCmsWidth + c]);
-    }
-    return best;
-  };
-  std::vector<uint32_t> ranked;
-  for (int i = 0; i < kCandGlobal; ++i)
-    if (cand[i]) ranked.push_back(cms_est(cand[i] - 1));
-  std::sort(ranked.begin(), ranked.end(), std::greater<uint32_t>());
+  out.hll_estimate = nonnull > 0 ? hll_estimate(o.hist) : 0;
 
   // Features: 64 normalised HLL register-value bins, then 16 frequency features.
   float* f = out.features;
   for (int i = 0; i < kSketchFeatures; ++i) f[i] = 0;
-  for (uint32_t r = 0; r <= 64; ++r) f[std::min<uint32_t>(r, 63)] += static_cast<float>(hll[r]) / kHllM;
-  double cum = 0;
-  size_t k = 0;
-  for (int i = 0; i < 12; ++i) {
-    const size_t upto = size_t(1) << i;
-    while (k < ranked.size() && k < upto) cum += ranked[k++];
-    out.top_share[i] = nonnull > 0 ? std::min(1.0, cum / nonnull) : 0;
-  }
+  for (uint32_t r = 0; r <= 64; ++r) f[std::min<uint32_t>(r, 63)] += static_cast<float>(o.hist[r]) / kHllM;
+  for (int i = 0; i < 12; ++i)
+    out.top_share[i] = nonnull > 0 ? std::min(1.0, static_cast<double>(o.top[i]) / nonnull) : 0;
   for (int i = 0; i < 10; ++i) f[64 + i] = static_cast<float>(out.top_share[i]);
-  double f2 = 0;
-  for (int c = 0; c < kCmsWidth; ++c) {
-    const double v = regs[kHllM + c];
-    f2 += v * v;
-  }
-  f[74] = nonnull > 0 ? static_cast<float>(f2 / (nonnull * nonnull)) : 0.f;
-  f[75] = static_cast<float>(std::log2(1.0 + out.sample_rows) / 32.0);
-  f[76] = static_cast<float>(std::log2(1.0 + out.total_rows) / 32.0);
-  f[77] = out.total_rows > 0 ? static_cast<float>(out.sample_rows / out.total_rows) : 1.f;
+  f[74] = nonnull > 0 ? static_cast<float>(static_cast<double>(o.f2) / (nonnull * nonnull)) : 0.f;
+  f[75] = static_cast<float>(log_rows);
+  f[76] = static_cast<float>(log_total);
+  f[77] = static_cast<float>(share);
   f[78] = static_cast<float>(out.null_frac);
   f[79] = nonnull > 0 ? static_cast<float>(std::min(1.0, out.hll_estimate / nonnull)) : 0.f;
 }
