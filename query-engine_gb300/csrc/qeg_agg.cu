@@ -1663,35 +1663,67 @@ DevCol AggState::key_col(const std::vector<StagedCol>& staged, size_t j) const {
 }
 
 namespace {
-// Smallest and largest value of an integer column (valid rows), as
-// order-preserving encodings: out[0] = min, out[1] = max.
-__global__ void int_range_kernel(DevCol c, uint64_t n, unsigned long long* out) {
-  unsigned long long mn = ~0ull, mx = 0;
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
-    if (!col_valid(c, r)) continue;
-    const unsigned long long e = enc_i64(int_value(c, r));
-    mn = e < mn ? e : mn;
-    mx = e > mx ? e : mx;
+// Smallest and largest value of an integer column without NULLs, as
+// order-preserving encodings: out[0] = min, out[1] = max. Reads 32 bytes per
+// access from the first aligned one on (one value per thread and step took 180
+// us for 50M 8-byte times).
+template <class T>
+__global__ void __launch_bounds__(256) int_range_kernel(const T* __restrict__ v, uint64_t n, uint64_t head,
+                                                        unsigned long long* out) {
+  using V = Vec32<T>;
+  const uint64_t at = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+  const uint64_t step = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  const uint64_t nv = (n - head) / V::kN;
+  T lo = v[0], hi = v[0];
+  for (uint64_t i = at; i < nv; i += 2 * step) {
+    V a, b;
+    const bool two = i + step < nv;
+    a.load(v + head + i * V::kN);
+    if (two) b.load(v + head + (i + step) * V::kN);
+#pragma unroll
+    for (int e = 0; e < V::kN; ++e) {
+      const T x = a.at(e), y = two ? b.at(e) : x;
+      lo = min(lo, min(x, y));
+      hi = max(hi, max(x, y));
+    }
   }
+  for (uint64_t i = at; i < head + (n - head) % V::kN; i += step) {  // before and behind the aligned part
+    const T x = v[i < head ? i : i + nv * V::kN];
+    lo = min(lo, x);
+    hi = max(hi, x);
+  }
+  int64_t mn = lo, mx = hi;
   for (int o = 16; o > 0; o >>= 1) {
     mn = min(mn, __shfl_down_sync(0xffffffffu, mn, o));
     mx = max(mx, __shfl_down_sync(0xffffffffu, mx, o));
   }
-  __shared__ unsigned long long smn[32], smx[32];
-  const unsigned warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  __shared__ int64_t smn[8], smx[8];
   if ((threadIdx.x & 31) == 0) {
-    smn[warp] = mn;
-    smx[warp] = mx;
+    smn[threadIdx.x >> 5] = mn;
+    smx[threadIdx.x >> 5] = mx;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (unsigned w = 1; w < nwarps; ++w) {
+    for (int w = 1; w < 8; ++w) {
       mn = min(mn, smn[w]);
       mx = max(mx, smx[w]);
     }
-    atomicMin(out + 0, mn);
-    atomicMax(out + 1, mx);
+    atomicMin(out + 0, static_cast<unsigned long long>(enc_i64(mn)));
+    atomicMax(out + 1, static_cast<unsigned long long>(enc_i64(mx)));
   }
+}
+
+template <class T>
+void launch_range(qeg_ctx* ctx, const void* data, uint64_t n, unsigned long long* out) {
+  const uint64_t off = reinterpret_cast<uintptr_t>(data) % 32;
+  const uint64_t head = std::min<uint64_t>(n, off ? (32 - off) / sizeof(T) : 0);
+  int_range_kernel<T><<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>(static_cast<const T*>(data), n, head, out);
+  ctx->launches++;
+}
+
+void column_range(qeg_ctx* ctx, const DevCol& c, uint64_t n, unsigned long long* out) {
+  if (c.type == kI32) launch_range<int32_t>(ctx, c.data, n, out);
+  else launch_range<int64_t>(ctx, c.data, n, out);
 }
 
 // Packed rows -> composite rows: every occupied single-key row (and the key-0
@@ -1759,12 +1791,8 @@ bool AggState::can_pack(const std::vector<StagedCol>& staged, uint64_t len) {
   DevBuf mm(32, ctx->stream);
   const unsigned long long init[4] = {~0ull, 0ull, ~0ull, 0ull};
   QEG_CUDA(cudaMemcpyAsync(mm.get(), init, 32, cudaMemcpyHostToDevice, ctx->stream));
-  int_range_kernel<<<grid_for(ctx, len, 256, 4), 256, 0, ctx->stream>>>(t, len, mm.get<unsigned long long>());
-  ctx->launches++;
-  if (wide_key) {
-    int_range_kernel<<<grid_for(ctx, len, 256, 4), 256, 0, ctx->stream>>>(a, len, mm.get<unsigned long long>() + 2);
-    ctx->launches++;
-  }
+  column_range(ctx, t, len, mm.get<unsigned long long>());
+  if (wide_key) column_range(ctx, a, len, mm.get<unsigned long long>() + 2);
   QEG_CUDA(cudaGetLastError());
   unsigned long long r[4];
   QEG_CUDA(cudaMemcpyAsync(r, mm.get(), 32, cudaMemcpyDeviceToHost, ctx->stream));

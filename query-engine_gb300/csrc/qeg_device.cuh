@@ -155,6 +155,26 @@ __host__ __device__ __forceinline__ uint64_t enc_i64(int64_t v) {
 __host__ __device__ __forceinline__ int64_t dec_i64(uint64_t u) {
   return static_cast<int64_t>(u ^ 0x8000000000000000ull);
 }
+
+// 32 bytes of a column of T (1, 4 or 8 bytes each) in one access; `p` is
+// 32-byte aligned.
+template <class T>
+struct Vec32 {
+  static constexpr int kN = 32 / sizeof(T);
+  uint64_t w[4];
+  __device__ __forceinline__ T at(int i) const {
+    return static_cast<T>(w[i / (kN / 4)] >> (i % (kN / 4) * sizeof(T) * 8));
+  }
+  __device__ __forceinline__ void load(const T* p) {
+    asm volatile("ld.global.L1::no_allocate.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
+                 : "l"(p));
+  }
+  __device__ __forceinline__ void store(T* p) const {
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(w[0]), "l"(w[1]), "l"(w[2]), "l"(w[3])
+                 : "memory");
+  }
+};
 __host__ __device__ __forceinline__ uint64_t enc_f64_bits(uint64_t b) {
   if ((b & 0x7fffffffffffffffull) > 0x7ff0000000000000ull) b = kCanonNaN;
   return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
