@@ -1715,8 +1715,7 @@ __global__ void iota_kernel(uint32_t* __restrict__ out, uint64_t n) {
 struct AsofScanK {
   DevCol key[kMaxKeys];
   int nkeys;
-  DevCol ts;              // (its validity is vbytes)
-  const uint8_t* vbytes;  // nullptr: no NULLs
+  DevCol ts;
   uint64_t n;
   JTable T;
   uint32_t nslots;
@@ -1780,7 +1779,7 @@ __global__ void __launch_bounds__(256) asof_scan_kernel(const AsofScanK P) {
     const int64_t t = int_value(P.ts, r);
     if (r + 1 < P.n) bad |= t > int_value(P.ts, r + 1);
     uint32_t slot = P.nslots;
-    if (!P.vbytes || P.vbytes[r]) {
+    if (col_valid(P.ts, r)) {
       const unsigned long long e = enc_i64(t);
       mn = e < mn ? e : mn;
       mx = e > mx ? e : mx;
@@ -2246,7 +2245,7 @@ __global__ void asof_emit_kernel(const AsofProbeK P, const uint64_t* __restrict_
 // idx[k] is kNullRow. Source validity is either a bitmap (probe columns) or a
 // byte per row (build store).
 __global__ void gather_kernel(const void* __restrict__ src, const uint64_t* __restrict__ src_bits,
-                              const uint8_t* __restrict__ src_bytes, const int32_t* __restrict__ code_map, int width,
+                              const int32_t* __restrict__ code_map, int width,
                               const uint32_t* __restrict__ idx, uint64_t n, void* __restrict__ out,
                               uint8_t* __restrict__ valid) {
   for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
@@ -2260,7 +2259,6 @@ __global__ void gather_kernel(const void* __restrict__ src, const uint64_t* __re
     }
     uint8_t ok = 1;
     if (src_bits) ok = (src_bits[r >> 6] >> (r & 63)) & 1ull;
-    else if (src_bytes) ok = src_bytes[r];
     valid[k] = ok;
     if (width == 8) static_cast<uint64_t*>(out)[k] = static_cast<const uint64_t*>(src)[r];
     else if (code_map) static_cast<int32_t*>(out)[k] = ok ? code_map[static_cast<const int32_t*>(src)[r]] : 0;
@@ -2273,7 +2271,7 @@ __global__ void gather_kernel(const void* __restrict__ src, const uint64_t* __re
 // validity packed on the fly (a warp covers 64 rows and makes one word from
 // two ballots; padding bits set), so an output row is written once.
 __global__ void gather_out_kernel(const void* __restrict__ src, const uint64_t* __restrict__ src_bits,
-                                  const uint8_t* __restrict__ src_bytes, const int32_t* __restrict__ code_map,
+                                  const int32_t* __restrict__ code_map,
                                   int width, const uint32_t* __restrict__ idx, uint64_t n, void* __restrict__ out,
                                   uint64_t* __restrict__ out_words, unsigned int* __restrict__ any_null) {
   const unsigned lane = threadIdx.x & 31u;
@@ -2290,7 +2288,6 @@ __global__ void gather_out_kernel(const void* __restrict__ src, const uint64_t* 
         ok = r != kNullRow;
         if (ok) {
           if (src_bits) ok = (src_bits[r >> 6] >> (r & 63)) & 1ull;
-          else if (src_bytes) ok = src_bytes[r];
         }
         if (width == 8) {
           static_cast<uint64_t*>(out)[k] = r == kNullRow ? 0 : static_cast<const uint64_t*>(src)[r];
@@ -2326,8 +2323,7 @@ constexpr int kMaxGatherCols = 32;
 
 struct GatherCol {
   const void* src;
-  const uint64_t* bits;
-  const uint8_t* bytes;
+  const uint64_t* bits;  // nullptr: no NULLs
   const int32_t* code_map;
   void* out;
   uint64_t* words;
@@ -2353,7 +2349,6 @@ __device__ __forceinline__ bool gather_one(const GatherCol& c, uint32_t r, uint6
   bool ok = r != kNullRow;
   if (ok) {
     if (c.bits) ok = (c.bits[r >> 6] >> (r & 63)) & 1ull;
-    else if (c.bytes) ok = c.bytes[r];
   }
   if (c.width == 8) {
     static_cast<uint64_t*>(c.out)[k] = r == kNullRow ? 0 : static_cast<const uint64_t*>(c.src)[r];
@@ -2473,7 +2468,7 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(const __grid_constant__ 
         else if (col.width == 4) v = static_cast<const uint32_t*>(col.src)[r];
         else v = static_cast<const uint8_t*>(col.src)[r];
         off = col.off;
-        mask |= !col.bytes || col.bytes[r] ? 1ull << col.bit : 0;
+        mask |= !col.bits || ((col.bits[r >> 6] >> (r & 63)) & 1ull) ? 1ull << col.bit : 0;
       } else {
         v = mask;
         off = P.mask_off;
@@ -2510,121 +2505,124 @@ __global__ void words_finish_kernel(uint64_t* __restrict__ words, uint64_t nw, u
   if (__any_sync(0xffffffffu, null_seen) && (threadIdx.x & 31) == 0) atomicOr(flag, 1u);
 }
 
-// Appends a batch column into the build store: values are copied, validity is
-// expanded to a byte per row; STR codes are translated to value ids.
-// RANGE (the single integer key of a build): the same pass also folds the
-// key's smallest and largest value and its non-NULL count into range[0..2]
-// (order-preserving encodings; one set of atomics per CTA), so the dense /
-// hash decision needs no separate pass over the key.
-template <bool RANGE>
-__global__ void store_append_kernel(DevCol c, uint64_t n, int width, void* __restrict__ dst,
-                                    uint8_t* __restrict__ dvalid, unsigned long long* __restrict__ range) {
-  unsigned long long mn = ~0ull, mx = 0, cnt = 0;
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
-    const bool ok = col_valid(c, r);
-    if (dvalid) dvalid[r] = ok ? 1 : 0;
-    if (c.type == kSTR) {
-      static_cast<int32_t*>(dst)[r] = ok ? static_cast<int32_t>(int_value(c, r)) : 0;
-    } else if (width == 8) {
-      static_cast<uint64_t*>(dst)[r] = __ldg(static_cast<const unsigned long long*>(c.data) + r);
-    } else if (width == 4) {
-      static_cast<uint32_t*>(dst)[r] = __ldg(static_cast<const unsigned int*>(c.data) + r);
-    } else {
-      static_cast<uint8_t*>(dst)[r] = __ldg(static_cast<const uint8_t*>(c.data) + r);
-    }
-    if (RANGE && ok) {
-      const unsigned long long e = enc_i64(int_value(c, r));
-      mn = e < mn ? e : mn;
-      mx = e > mx ? e : mx;
-      ++cnt;
-    }
-  }
-  if (!RANGE) return;
-  for (int o = 16; o > 0; o >>= 1) {
-    mn = min(mn, __shfl_down_sync(0xffffffffu, mn, o));
-    mx = max(mx, __shfl_down_sync(0xffffffffu, mx, o));
-    cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-  }
-  __shared__ unsigned long long smn[32], smx[32], scn[32];
-  const unsigned warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    smn[warp] = mn;
-    smx[warp] = mx;
-    scn[warp] = cnt;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (unsigned w = 1; w < nwarps; ++w) {
-      mn = min(mn, smn[w]);
-      mx = max(mx, smx[w]);
-      cnt += scn[w];
-    }
-    if (cnt) {
-      atomicMin(range + 0, mn);
-      atomicMax(range + 1, mx);
-      atomicAdd(range + 2, cnt);
-    }
+// Validity words of a batch (src; nullptr: no NULLs) behind the `base` rows
+// that dst holds already.
+__global__ void append_words_kernel(const uint64_t* __restrict__ src, uint64_t n, uint64_t* __restrict__ dst,
+                                    uint64_t base) {
+  const uint64_t first = base / 64, words = (base + n - 1) / 64 - first + 1, nsrc = (n + 63) / 64;
+  const unsigned sh = base % 64;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < words; i += (uint64_t)gridDim.x * blockDim.x) {
+    // Word i takes the upper bits of source word i - 1 and the lower ones of word i.
+    uint64_t v = (i < nsrc ? (src ? src[i] : ~0ull) : 0ull) << sh;
+    if (sh) v |= i > 0 ? (src ? src[i - 1] : ~0ull) >> (64 - sh) : dst[first] & ((1ull << sh) - 1);
+    dst[first + i] = v;
   }
 }
 
-// A batch column without NULLs whose values are stored as they are: copied 32
-// bytes at a time where both ends allow (one value per thread and step, with
-// its validity byte: 62 us for the four columns of 5M quotes),
-// the range as above.
-template <class T, bool RANGE>
-__global__ void __launch_bounds__(256) append_plain_kernel(const T* __restrict__ src, T* __restrict__ dst, uint64_t n,
-                                                           int vec, unsigned long long* __restrict__ range) {
-  using V = Vec32<T>;
-  const uint64_t at = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-  const uint64_t step = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  const uint64_t nv = vec ? n / V::kN : 0;
-  int64_t lo = INT64_MAX, hi = INT64_MIN;
-  for (uint64_t i = at; i < nv; i += 2 * step) {
-    V a, b;
-    const bool two = i + step < nv;
-    a.load(src + i * V::kN);
-    if (two) b.load(src + (i + step) * V::kN);
-    a.store(dst + i * V::kN);
-    if (two) b.store(dst + (i + step) * V::kN);
-    if (RANGE) {
-#pragma unroll
-      for (int e = 0; e < V::kN; ++e) {
-        const int64_t x = a.at(e), y = two ? b.at(e) : x;
-        lo = min(lo, min(x, y));
-        hi = max(hi, max(x, y));
-      }
-    }
-  }
-  for (uint64_t i = nv * V::kN + at; i < n; i += step) {
-    const T x = src[i];
-    dst[i] = x;
-    if (RANGE) {
-      lo = min(lo, static_cast<int64_t>(x));
-      hi = max(hi, static_cast<int64_t>(x));
-    }
-  }
-  if (!RANGE) return;
+// Range of a build key (the single integer key of a join): every append folds
+// the key's smallest and largest value and its non-NULL count into range[0..2]
+// (order-preserving encodings; one set of atomics per CTA), so the dense /
+// hash decision needs no separate pass over the key.
+__device__ __forceinline__ void fold_range(int64_t lo, int64_t hi, unsigned int cnt, unsigned long long* range) {
   for (int o = 16; o > 0; o >>= 1) {
     lo = min(lo, __shfl_down_sync(0xffffffffu, lo, o));
     hi = max(hi, __shfl_down_sync(0xffffffffu, hi, o));
+    cnt += __shfl_down_sync(0xffffffffu, cnt, o);
   }
   __shared__ int64_t slo[8], shi[8];
+  __shared__ unsigned int scnt[8];
   if ((threadIdx.x & 31) == 0) {
     slo[threadIdx.x >> 5] = lo;
     shi[threadIdx.x >> 5] = hi;
+    scnt[threadIdx.x >> 5] = cnt;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < 8; ++w) {
       lo = min(lo, slo[w]);
       hi = max(hi, shi[w]);
+      cnt += scnt[w];
     }
-    if (lo <= hi) {
+    if (cnt) {
       atomicMin(range + 0, static_cast<unsigned long long>(enc_i64(lo)));
       atomicMax(range + 1, static_cast<unsigned long long>(enc_i64(hi)));
+      atomicAdd(range + 2, static_cast<unsigned long long>(cnt));
     }
-    if (blockIdx.x == 0) atomicAdd(range + 2, static_cast<unsigned long long>(n));
   }
+}
+
+// STR columns with a code map or NULLs: codes are stored as value ids, NULLs as 0.
+__global__ void __launch_bounds__(256) append_codes_kernel(DevCol c, uint64_t n, int32_t* __restrict__ dst,
+                                                           unsigned long long* __restrict__ range) {
+  int64_t lo = INT64_MAX, hi = INT64_MIN;
+  unsigned int cnt = 0;
+  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
+    const bool ok = col_valid(c, r);
+    const int64_t x = ok ? int_value(c, r) : 0;
+    dst[r] = static_cast<int32_t>(x);
+    if (ok) {
+      lo = min(lo, x);
+      hi = max(hi, x);
+      ++cnt;
+    }
+  }
+  if (range) fold_range(lo, hi, cnt, range);
+}
+
+// Other columns: values copied as they are, 32 bytes at a time where both ends
+// allow (one value and one validity byte per thread and step took 62 us for
+// four columns of 5M quotes and 66 us for 16M keys). `bits`: the key's
+// validity for the range (nullptr: no NULLs); the rows of a vector lie in one
+// word.
+template <class T, bool RANGE>
+__global__ void __launch_bounds__(256) append_plain_kernel(const T* __restrict__ src, T* __restrict__ dst, uint64_t n,
+                                                           int vec, const uint64_t* __restrict__ bits,
+                                                           unsigned long long* __restrict__ range) {
+  using V = Vec32<T>;
+  const uint64_t at = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+  const uint64_t step = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  const uint64_t nv = vec ? n / V::kN : 0;
+  int64_t lo = INT64_MAX, hi = INT64_MIN;
+  unsigned int cnt = 0;
+  auto rows_ok = [&](uint64_t row) { return bits ? static_cast<uint32_t>(__ldg(bits + row / 64) >> (row % 64)) : ~0u; };
+  auto fold = [&](const V& v, uint32_t ok) {
+#pragma unroll
+    for (int e = 0; e < V::kN; ++e) {
+      const int64_t x = v.at(e);
+      if ((ok >> e) & 1u) {
+        lo = min(lo, x);
+        hi = max(hi, x);
+        ++cnt;
+      }
+    }
+  };
+  for (uint64_t i = at; i < nv; i += 2 * step) {
+    V a, b;
+    const bool two = i + step < nv;
+    uint32_t oka = 0, okb = 0;
+    a.load(src + i * V::kN);
+    if (RANGE) oka = rows_ok(i * V::kN);
+    if (two) {
+      b.load(src + (i + step) * V::kN);
+      if (RANGE) okb = rows_ok((i + step) * V::kN);
+    }
+    a.store(dst + i * V::kN);
+    if (two) b.store(dst + (i + step) * V::kN);
+    if (RANGE) {
+      fold(a, oka);
+      if (two) fold(b, okb);
+    }
+  }
+  for (uint64_t i = nv * V::kN + at; i < n; i += step) {
+    const T x = src[i];
+    dst[i] = x;
+    if (RANGE && (rows_ok(i) & 1u)) {
+      lo = min(lo, static_cast<int64_t>(x));
+      hi = max(hi, static_cast<int64_t>(x));
+      ++cnt;
+    }
+  }
+  if (RANGE) fold_range(lo, hi, cnt, range);
 }
 
 uint64_t next_pow2(uint64_t v) {
@@ -2646,8 +2644,8 @@ struct JoinState {
   double est_distinct = 0;  // distinct build keys the hash table was sized from (0: row count)
   int32_t rebuilds = 0;     // estimate-sized tables that overflowed and were rebuilt
 
-  // build store: values, and a validity byte per row for the columns that got a
-  // batch with a validity bitmap (no buffer: no NULLs)
+  // build store: values, and validity words for the columns that got a batch
+  // with a validity bitmap (no buffer: no NULLs)
   std::vector<DevBuf> bvals, bvalid;
   uint64_t nbuild = 0, bcap = 0;
   bool built = false;
@@ -2701,7 +2699,8 @@ struct JoinState {
     DevCol c{};
     c.type = btypes[btime];
     c.data = bvals[btime].get();
-    c.all_valid = 1;
+    c.validity = bvalid[btime].get<uint64_t>();
+    c.all_valid = c.validity == nullptr;
     return c;
   }
   void asof_build();
@@ -2751,8 +2750,9 @@ struct JoinState {
                                    ctx->stream));
         bvals[c] = std::move(v);
         if (bvalid[c].get()) {
-          DevBuf ok(ncap, ctx->stream);
-          QEG_CUDA(cudaMemcpyAsync(ok.get(), bvalid[c].get(), nbuild, cudaMemcpyDeviceToDevice, ctx->stream));
+          DevBuf ok((ncap + 63) / 64 * 8, ctx->stream);
+          QEG_CUDA(cudaMemcpyAsync(ok.get(), bvalid[c].get(), (nbuild + 63) / 64 * 8, cudaMemcpyDeviceToDevice,
+                                   ctx->stream));
           bvalid[c] = std::move(ok);
         }
       }
@@ -2771,30 +2771,33 @@ struct JoinState {
       host_input = host_input || s.data.get() || s.validity.get() || s.code_map.get();
       const int w = static_cast<int>(type_width(btypes[c]));
       if (!s.dev.all_valid && !bvalid[c].get()) {  // the rows so far are valid
-        bvalid[c].alloc(bcap, ctx->stream);
-        if (nbuild) QEG_CUDA(cudaMemsetAsync(bvalid[c].get(), 1, nbuild, ctx->stream));
+        bvalid[c].alloc((bcap + 63) / 64 * 8, ctx->stream);
+        if (nbuild) QEG_CUDA(cudaMemsetAsync(bvalid[c].get(), 0xff, (nbuild + 63) / 64 * 8, ctx->stream));
+      }
+      const uint64_t* bits = s.dev.all_valid ? nullptr : s.dev.validity;
+      if (bvalid[c].get()) {
+        append_words_kernel<<<grid_for(ctx, n / 64 + 2, 256, 8), 256, 0, ctx->stream>>>(bits, n,
+                                                                                       bvalid[c].get<uint64_t>(), nbuild);
+        ctx->launches++;
+        QEG_CUDA(cudaGetLastError());
       }
       uint8_t* dst = bvals[c].get<uint8_t>() + nbuild * w;
-      uint8_t* ok = bvalid[c].get() ? bvalid[c].get<uint8_t>() + nbuild : nullptr;
       unsigned long long* range = c == range_col ? krange.get<unsigned long long>() : nullptr;
       const unsigned g = grid_for(ctx, n, 256, 8);
-      if (s.dev.all_valid && s.dev.code_map == nullptr) {
-        if (ok) QEG_CUDA(cudaMemsetAsync(ok, 1, n, ctx->stream));
+      if (btypes[c] == QEG_STR && (bits || s.dev.code_map)) {
+        append_codes_kernel<<<g, 256, 0, ctx->stream>>>(s.dev, n, reinterpret_cast<int32_t*>(dst), range);
+      } else {
         const int vec = (reinterpret_cast<uintptr_t>(s.dev.data) | reinterpret_cast<uintptr_t>(dst)) % 32 == 0;
         auto copy = [&](auto zero) {
           using T = decltype(zero);
           const T* src = static_cast<const T*>(s.dev.data);
           T* to = reinterpret_cast<T*>(dst);
-          if (range) append_plain_kernel<T, true><<<g, 256, 0, ctx->stream>>>(src, to, n, vec, range);
-          else append_plain_kernel<T, false><<<g, 256, 0, ctx->stream>>>(src, to, n, vec, nullptr);
+          if (range) append_plain_kernel<T, true><<<g, 256, 0, ctx->stream>>>(src, to, n, vec, bits, range);
+          else append_plain_kernel<T, false><<<g, 256, 0, ctx->stream>>>(src, to, n, vec, nullptr, nullptr);
         };
         if (w == 8) copy(int64_t{});
         else if (w == 4) copy(int32_t{});
         else copy(uint8_t{});
-      } else if (range) {
-        store_append_kernel<true><<<g, 256, 0, ctx->stream>>>(s.dev, n, w, dst, ok, range);
-      } else {
-        store_append_kernel<false><<<g, 256, 0, ctx->stream>>>(s.dev, n, w, dst, ok, nullptr);
       }
       ctx->launches++;
       QEG_CUDA(cudaGetLastError());
@@ -2806,16 +2809,13 @@ struct JoinState {
     nbuild += n;
   }
 
-  // Key columns of the build store as kernel columns (validity as a byte array
-  // is exposed through a bitmap-free path: keys are re-read with col_valid, so
-  // the store keeps a packed bitmap per key column).
-  std::vector<DevBuf> key_bits;
+  // Key columns of the build store as kernel columns.
   DevCol store_key(int j) {
     DevCol c{};
     c.type = btypes[bkeys[j]] == QEG_STR ? QEG_I32 : btypes[bkeys[j]];  // STR stored as value ids
     c.data = bvals[bkeys[j]].get();
-    c.validity = key_bits[j].get<uint64_t>();
-    c.all_valid = key_bits[j].get() == nullptr;
+    c.validity = bvalid[bkeys[j]].get<uint64_t>();
+    c.all_valid = c.validity == nullptr;
     c.code_map = nullptr;
     return c;
   }
@@ -2836,24 +2836,6 @@ struct JoinState {
   bool counts_ready = false;  // cnt holds every slot's build row count
 };
 
-namespace {
-
-// Validity bytes -> 64-bit LSB-first words: a warp turns 64 bytes into one
-// word with two ballots.
-__global__ void bytes_to_bits_kernel(const uint8_t* __restrict__ b, uint64_t n, uint64_t* __restrict__ w) {
-  const uint64_t nw = (n + 63) / 64;
-  const unsigned lane = threadIdx.x & 31u;
-  const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
-  for (uint64_t i = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; i < nw; i += nwarps) {
-    const uint64_t r = i * 64 + lane;
-    const unsigned lo = __ballot_sync(0xffffffffu, r < n && b[r]);
-    const unsigned hi = __ballot_sync(0xffffffffu, r + 32 < n && b[r + 32]);
-    if (lane == 0) w[i] = static_cast<uint64_t>(lo) | (static_cast<uint64_t>(hi) << 32);
-  }
-}
-
-}  // namespace
-
 void JoinState::finish_build() {
   require(!built, "build_finish() called twice");
   built = true;
@@ -2861,16 +2843,6 @@ void JoinState::finish_build() {
   if (asof && nk == 0) {  // one global partition: no table
     asof_build();
     return;
-  }
-  key_bits.clear();
-  for (int j = 0; j < nk; ++j) {
-    key_bits.emplace_back();
-    if (bvalid[bkeys[j]].get()) {
-      key_bits[j].alloc(((nbuild + 63) / 64 + 1) * 8, ctx->stream);
-      bytes_to_bits_kernel<<<grid_for(ctx, (nbuild / 64 + 1) * 32, 256, 8), 256, 0, ctx->stream>>>(
-          bvalid[bkeys[j]].get<uint8_t>(), nbuild, key_bits[j].get<uint64_t>());
-      ctx->launches++;
-    }
   }
   BuildK P{};
   P.nkeys = nk;
@@ -2984,7 +2956,6 @@ void JoinState::asof_build() {
   P.nkeys = nk;
   for (int j = 0; j < nk; ++j) P.key[j] = store_key(j);
   P.ts = build_time();
-  P.vbytes = bvalid[btime].get<uint8_t>();
   P.n = nbuild;
   if (nk) P.T = table();
   P.nslots = aslots;
@@ -3269,7 +3240,7 @@ bool JoinState::pack_rows(uint64_t count) {
   G.mask_off = packed_mask;
   for (int c = 0; c < nc; ++c) {
     G.c[c].src = bvals[c].get();
-    G.c[c].bytes = bvalid[c].get<uint8_t>();
+    G.c[c].bits = bvalid[c].get<uint64_t>();
     G.c[c].width = static_cast<int>(type_width(btypes[c]));
     G.c[c].off = packed_off[c];
     G.c[c].bit = c;
@@ -3659,7 +3630,7 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
         g.code_map = st.ptypes[c] == QEG_STR ? sc.dev.code_map : nullptr;
       } else {
         g.src = st.bvals[bc].get();
-        g.bytes = st.bvalid[bc].get<uint8_t>();
+        g.bits = st.bvalid[bc].get<uint64_t>();
         if (st.packed_words) {
           g.off = st.packed_off[bc];
           g.bit = static_cast<int>(bc);
@@ -3743,7 +3714,6 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
         const int w = static_cast<int>(type_width(pc ? st.ptypes[c] : st.btypes[bc]));
         const void* src = pc ? st.probe_staged[c].dev.data : st.bvals[bc].get();
         const uint64_t* bits = nullptr;
-        const uint8_t* bytes = nullptr;
         const int32_t* cm = nullptr;
         const uint32_t* idx = (pc ? st.out_probe.get<uint32_t>() : st.out_build.get<uint32_t>()) + first;
         if (pc) {
@@ -3751,9 +3721,9 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
           bits = sc.dev.all_valid ? nullptr : sc.dev.validity;
           cm = st.ptypes[c] == QEG_STR ? sc.dev.code_map : nullptr;
         } else {
-          bytes = st.bvalid[bc].get<uint8_t>();
+          bits = st.bvalid[bc].get<uint64_t>();
         }
-        gather_out_kernel<<<gw, 256, 0, ctx->stream>>>(src, bits, bytes, cm, w, idx, count, outs[c].data,
+        gather_out_kernel<<<gw, 256, 0, ctx->stream>>>(src, bits, cm, w, idx, count, outs[c].data,
                                                       outs[c].validity, flags.get<unsigned int>() + c);
         ctx->launches++;
         QEG_CUDA(cudaGetLastError());
@@ -3846,7 +3816,7 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
     for (size_t c = 0; c < st.ptypes.size(); ++c) {
       const StagedCol& s = st.probe_staged[c];
       const int w = static_cast<int>(type_width(st.ptypes[c]));
-      gather_kernel<<<g, 256, 0, ctx->stream>>>(s.dev.data, s.dev.all_valid ? nullptr : s.dev.validity, nullptr,
+      gather_kernel<<<g, 256, 0, ctx->stream>>>(s.dev.data, s.dev.all_valid ? nullptr : s.dev.validity,
                                                st.ptypes[c] == QEG_STR ? s.dev.code_map : nullptr, w,
                                                st.out_probe.get<uint32_t>() + first, count, vals.get(),
                                                valid.get<uint8_t>());
@@ -3856,7 +3826,7 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
     }
     for (size_t c = 0; c < st.btypes.size(); ++c) {
       const int w = static_cast<int>(type_width(st.btypes[c]));
-      gather_kernel<<<g, 256, 0, ctx->stream>>>(st.bvals[c].get(), nullptr, st.bvalid[c].get<uint8_t>(), nullptr, w,
+      gather_kernel<<<g, 256, 0, ctx->stream>>>(st.bvals[c].get(), st.bvalid[c].get<uint64_t>(), nullptr, w,
                                                st.out_build.get<uint32_t>() + first, count, vals.get(),
                                                valid.get<uint8_t>());
       ctx->launches++;
