@@ -88,18 +88,27 @@ __device__ __forceinline__ int priv_slot(uint64_t* keys, int slots, uint64_t k, 
   return -1;
 }
 
-// The two slots of a key in a read-only table of heavy hitters, and the one
-// that holds key word k (nonzero), or -1: two independent loads, no search.
-__host__ __device__ __forceinline__ uint32_t hot_slot1(uint64_t h, int slots) {
-  return static_cast<uint32_t>(h >> 32) & static_cast<uint32_t>(slots - 1);
+// Read-only table of heavy hitters: a key lies in one of two pairs of slots
+// (first slot of each), loaded 16 bytes at a time, without a search. The slot
+// that holds key word k (nonzero), or -1. (Single slots would fill to 0.45 at
+// most, pairs to 0.85: 3480 keys in 4096 slots, 7.77 -> 7.71 ms for 256M Zipf
+// rows.)
+__host__ __device__ __forceinline__ uint32_t hot_pair1(uint64_t h, int slots) {
+  return static_cast<uint32_t>(h >> 32) & static_cast<uint32_t>(slots - 2);
 }
-__host__ __device__ __forceinline__ uint32_t hot_slot2(uint64_t h, int slots) {
-  return static_cast<uint32_t>(h >> 46) & static_cast<uint32_t>(slots - 1);
+__host__ __device__ __forceinline__ uint32_t hot_pair2(uint64_t h, int slots) {
+  return static_cast<uint32_t>(h >> 46) & static_cast<uint32_t>(slots - 2);
 }
 __device__ __forceinline__ int hot_slot(const uint64_t* keys, int slots, uint64_t k, uint64_t h) {
-  const uint32_t s1 = hot_slot1(h, slots), s2 = hot_slot2(h, slots);
-  const uint64_t a = keys[s1], b = keys[s2];
-  return a == k ? static_cast<int>(s1) : (b == k ? static_cast<int>(s2) : -1);
+  const int p = static_cast<int>(hot_pair1(h, slots)), q = static_cast<int>(hot_pair2(h, slots));
+  const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(keys + p);
+  const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(keys + q);
+  int s = -1;
+  if (b.y == k) s = q + 1;
+  if (b.x == k) s = q;
+  if (a.y == k) s = p + 1;
+  if (a.x == k) s = p;
+  return s;
 }
 
 // Merges one contribution x into field f (of kind `kind`) of private row `row`.
