@@ -1398,9 +1398,16 @@ __global__ void __launch_bounds__(1024) finalize_kernel(const AggK P, const FinK
   // Output positions: one atomic per CTA and pass (the warps' counts are
   // prefixed in shared memory), not one per warp -- a sparse table of tens of
   // millions of slots would otherwise serialise on the counter.
-  __shared__ unsigned long long wpos[32];
+  __shared__ unsigned int wpos[32];
+  __shared__ unsigned int s_rows;
+  __shared__ unsigned long long s_first;
   // kFinPer slots per thread and pass: fewer passes, so fewer barriers.
   constexpr int kFinPer = 4;
+  // The occupied slots of a pass, side by side, so that the rows are finalised
+  // by full warps: slot by slot, the half-empty warps of a half-full table took
+  // twice the instructions, FP64 divisions above all (minute bars of 50M
+  // trades, 3.9M groups: 3.20 ms the call, 3.11 now).
+  __shared__ uint16_t list[1024 * kFinPer];
   const uint64_t span = static_cast<uint64_t>(blockDim.x) * kFinPer;
   for (uint64_t base = blockIdx.x * span; base < total; base += gridDim.x * span) {
     bool occk[kFinPer];
@@ -1430,27 +1437,34 @@ __global__ void __launch_bounds__(1024) finalize_kernel(const AggK P, const FinK
     }
     if (lane == 0) wpos[warp] = cnt;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned long long run = 0;
-      for (int w = 0; w < nwarps; ++w) {
-        const unsigned long long c = wpos[w];
-        wpos[w] = run;
-        run += c;
+    if (warp == 0) {
+      const unsigned c = lane < nwarps ? wpos[lane] : 0;
+      unsigned incl = c;
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
       }
-      const unsigned long long b = run ? atomicAdd(F.out_count, run) : 0;
-      for (int w = 0; w < nwarps; ++w) wpos[w] += b;
+      wpos[lane] = incl - c;
+      if (lane == 31) {
+        s_rows = incl;
+        s_first = incl ? atomicAdd(F.out_count, static_cast<unsigned long long>(incl)) : 0;
+      }
     }
     __syncthreads();
-    unsigned long long wbase = wpos[warp];
-    __syncthreads();  // wpos is rewritten by the next pass
+    unsigned at = wpos[warp];
+#pragma unroll
     for (int k = 0; k < kFinPer; ++k) {
-      const unsigned m = mk[k];
-      const unsigned long long kbase = wbase;
-      wbase += __popc(m);
-      if (!occk[k]) continue;
-      const uint64_t s = base + static_cast<uint64_t>(k) * blockDim.x + threadIdx.x;
+      if (occk[k])
+        list[at + __popc(mk[k] & ((1u << lane) - 1u))] = static_cast<uint16_t>(k * blockDim.x + threadIdx.x);
+      at += __popc(mk[k]);
+    }
+    const unsigned nrows = s_rows;
+    const unsigned long long first = s_first;
+    __syncthreads();  // (wpos, s_rows and s_first are rewritten after the next pass's first barrier)
+    for (unsigned i = threadIdx.x; i < nrows; i += blockDim.x) {
+      const uint64_t s = base + list[i];
       const uint64_t* r = P.table + s * W;
-      const uint64_t o = kbase + __popc(m & ((1u << lane) - 1u));
+      const uint64_t o = first + i;
       if (o >= F.out_cap) {
         atomicOr(P.err, kDevSpillOverflow);
         continue;
