@@ -125,7 +125,7 @@ typedef struct qeg_agg_config {
   int32_t rows_per_thread;   /* 0 = tuned                                   */
   int32_t smem_slots;        /* 0 = tuned                                   */
   int32_t hot_keys;          /* > 0: preload that many sketch heavy hitters into the
-                                  CTA tables (the hottest 32 in warp-private rows);
+                                  CTA tables (the hottest 16 with a row per lane);
                                   0 or -1: first-come CTA tables (the default) */
 } qeg_agg_config;
 

@@ -2,7 +2,7 @@
 // (ops/join.h:69-123, ops/join.cpp).
 //
 // Build (ops/join.cpp:133-197): every build batch is appended to a device
-// BuildStore (column values + one validity byte per row, the GPU form of
+// BuildStore (column values + validity words, the GPU form of
 // ops/join_internal.h:38-93). build_finish() then builds a CSR multiplicity
 // map over the rows whose key tuple holds no NULL (NULL keys never match,
 // NullPolicy::kNeverMatch, ops/hashtable.h:36-43):
@@ -17,10 +17,11 @@
 // "unique" flag (HASH) so a probe that only needs the match count reads one
 // bit / one key word per row.
 //
-// Probe: per probe batch, a count kernel sizes each probe row's output (LEFT:
-// at least one row), a scan turns the counts into offsets, an emit kernel
-// writes (probe row, build row | NULL) pairs (build_pairs_for_probe,
-// ops/join.cpp:199-247), and fetch() gathers the output columns, probe columns
+// Probe: per probe batch, one lookup kernel finds every probe row's match
+// (unique keys: its build row; LEFT output row k is then probe row k, an INNER
+// one is compacted) or sizes its output, a scan turns the counts into offsets
+// and an emit kernel writes (probe row, build row | NULL) pairs
+// (build_pairs_for_probe, ops/join.cpp:199-247), and fetch() gathers the output columns, probe columns
 // then build columns (ops/join_internal.h:136-179). The COUNT(*)/SUM(payload)
 // sink is fused into one probe kernel.
 #include <algorithm>
