@@ -14,9 +14,11 @@
 // rows - nulls), integer / F64 sums, and MIN/MAX as order-preserving unsigned
 // encodings updated with atomicMax (qeg_device.cuh).
 //
-// Kernel: each CTA keeps a private shared-memory table (first-come insertion,
-// or preloaded with heavy hitters) and falls back to the global table, whose
-// key words are claimed with one CAS. Rows whose key cannot be placed within
+// Kernels: for single keys each CTA keeps a private shared-memory table
+// (first-come insertion, or preloaded with heavy hitters) that lanes update row
+// by row (qeg_privagg.cuh), and falls back to the global table, whose
+// key words are claimed with one CAS; inputs whose global table would not stay
+// in L2 are partitioned by key hash first. Rows whose key cannot be placed within
 // the probe limit are spilled (row index) and re-run after the host grows the
 // table (rehash) -- the GPU form of HashTable::grow (ops/hashtable.cpp:75-91).
 #include <algorithm>
@@ -296,9 +298,9 @@ __device__ __forceinline__ void warp_apply(uint64_t* f, bool leader, int space, 
 // warp and published every 64; once the count passes P.full_at, lookups of new
 // keys give up after a short probe and spill instead of walking probe_limit
 // slots of a full table.
-__device__ __forceinline__ void track_full(const AggK& P, unsigned lane, uint32_t iter, bool inserted_now,
+__device__ __forceinline__ void track_full(const AggK& P, unsigned lane, uint32_t iter, unsigned inserted_now,
                                            unsigned& pending, bool& full) {
-  pending += __popc(__ballot_sync(0xffffffffu, inserted_now));
+  pending += __reduce_add_sync(0xffffffffu, inserted_now);
   if (pending >= 64 || (iter & 15) == 15) {
     if (lane == 0) {
       if (pending) {
@@ -583,7 +585,7 @@ __global__ void __launch_bounds__(1024) agg_private_kernel(const __grid_constant
     __syncthreads();
   }
 
-  unsigned long long inserted = 0;
+  unsigned long long inserted = 0, tracked = 0;
   unsigned pending = 0;  // table-full signal state (track_full)
   bool full = P.full_flag && ld_relaxed_u32(P.full_flag) != 0;
   unsigned missed = 0;             // this warp's rows of the window that missed the private table
@@ -649,7 +651,6 @@ __global__ void __launch_bounds__(1024) agg_private_kernel(const __grid_constant
                              P.nfields, vv[u], vb[u]);
       }
     }
-    const unsigned long long ins0 = inserted;
     bool cold[kPrivU];
     uint64_t* r[kPrivU];
 #pragma unroll
@@ -662,12 +663,20 @@ __global__ void __launch_bounds__(1024) agg_private_kernel(const __grid_constant
         else spill_row(P, p[u]);
       }
     }
-    if (P.full_flag) track_full(P, lane, step, inserted != ins0, pending, full);
+    if (P.full_flag) {
+      // (With the rows that a flush inserted: without them a table that is
+      // too small was never found full, and every row searched it to the
+      // probe limit.)
+      track_full(P, lane, step, static_cast<unsigned>(inserted - tracked), pending, full);
+      tracked = inserted;
+    }
     if (insert && (step & (kPrivWindow - 1)) == kPrivWindow - 1) {
       // The window's misses, summed over the CTA (three sums in turn: the one
       // cleared here is next used after another barrier).
       unsigned* sum = &s_miss[(step / kPrivWindow) % 3];
-      if (lane == 0 && missed) atomicAdd(sum, missed);
+      // Not once the global table is full: a flush would search it in vain for
+      // most groups, and its refill would spill.
+      if (lane == 0 && missed && !full) atomicAdd(sum, missed);
       missed = 0;
       __syncthreads();
       const unsigned m = *sum;
