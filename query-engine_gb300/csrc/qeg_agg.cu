@@ -1837,8 +1837,14 @@ bool AggState::can_pack(const std::vector<StagedCol>& staged, uint64_t len) {
 }
 
 // Converts the packed single-key table into composite rows (same capacity),
-// after which the window runs as an ordinary composite-key GROUP BY.
+// after which the window or GROUP BY runs as an ordinary composite-key one.
+// The tail rows of a partitioned batch are single-key rows too: they join the
+// table first.
 void AggState::unpack() {
+  merge_tails();
+  tails.release();
+  tails_cap = 0;
+  pool.release();
   DevBuf old;
   old.swap(table);
   const uint64_t old_cap = cap;

@@ -1,0 +1,54 @@
+"""GROUP BY over sequences of batches whose route changes on the way, against
+the oracle: packed pairs of 4-byte keys that were partitioned and then meet a
+NULL key."""
+import numpy as np
+import pytest
+
+import oracle as O
+import qeg
+from util import assert_same, gpu_rows, to_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def whole(batches):
+    """The batches as one table."""
+    cols = []
+    for i, c in enumerate(batches[0]):
+        ok = None
+        if any(b[i].valid is not None for b in batches):
+            ok = np.concatenate([np.ones(b[i].n, bool) if b[i].valid is None else b[i].valid for b in batches])
+        cols.append(O.TCol(c.type, np.concatenate([b[i].values for b in batches]), ok))
+    return cols
+
+
+def check(agg, batches, keys, aggs):
+    agg.finish()
+    gt, grows = gpu_rows(agg.fetch(), agg.result_types)
+    ot, orows = O.groupby(whole(batches), keys, aggs, 1 << 23)
+    assert_same(gt, grows, ot, orows)
+
+
+@pytest.mark.parametrize("null_key", [0, 1])
+def test_packed_pair_partitioned_then_null_keys(ctx, null_key):
+    # The first batch's groups lie in the tail rows when the packing ends.
+    rng = np.random.default_rng(11 + null_key)
+
+    def batch(n, nulls):
+        a = rng.integers(-4, 4, n).astype(np.int32)
+        b = np.where(rng.random(n) < 0.5, rng.integers(0, 30, n), rng.integers(0, 150_000, n)).astype(np.int32)
+        ok = rng.random(n) > 0.1 if nulls else None
+        return [O.TCol(O.I32, a, ok if null_key == 0 else None), O.TCol(O.I32, b, ok if null_key == 1 else None),
+                O.TCol(O.F64, rng.normal(0, 5, n)), O.TCol(O.I32, rng.integers(1, 100, n).astype(np.int32))]
+
+    aggs = [(O.SUM, 3), (O.AVG, 2)]
+    batches = [batch(4_400_003, False), batch(30_001, True), batch(20_000, False)]
+    agg = qeg.Aggregate(ctx, [c.type for c in batches[0]], [0, 1], aggs)
+    try:
+        agg.consume([to_gpu(c) for c in batches[0]])
+        assert agg.stats()["strategy"] == qeg.AGG_PARTITIONED, agg.stats()
+        for b in batches[1:]:
+            agg.consume([to_gpu(c) for c in b])
+        check(agg, batches, [0, 1], aggs)
+    finally:
+        agg.close()
