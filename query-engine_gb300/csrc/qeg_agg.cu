@@ -2159,6 +2159,7 @@ void AggState::consume(const qeg_column* cols, int ncols, const uint32_t* sel, u
   }
   rows_seen += nrows;
   if (nrows == 0) return;
+  fit_private(staged);
 
   if (strategy == QEG_AGG_PARTITIONED) {
     consume_partitioned(staged, nrows, len, dsel);
@@ -2318,11 +2319,7 @@ void AggState::first_consume(const std::vector<StagedCol>& staged, uint64_t nrow
     smem_slots = std::min(std::max(smem_slots, 64), slots);
     smem_insert = go_part ? 0 : 1;
     if (preload) {
-      const int want_hot = cfg.hot_keys > 0 ? cfg.hot_keys : smem_slots;
-      const std::vector<uint64_t> hot = hot_table(std::min(want_hot, smem_slots * 17 / 20), smem_slots, &nhot);
-      hot_keys_dev.alloc(hot.size() * 8, ctx->stream);
-      QEG_CUDA(cudaMemcpyAsync(hot_keys_dev.get(), hot.data(), hot.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
-      QEG_CUDA(cudaStreamSynchronize(ctx->stream));
+      preload_hot();
       smem_insert = 0;
     }
   } else if (strategy == QEG_AGG_SMEM && mode == 2) {
@@ -2340,6 +2337,30 @@ void AggState::first_consume(const std::vector<StagedCol>& staged, uint64_t nrow
   part_cap = static_cast<uint64_t>(ctx->sms) * (mode == 1 ? 2 : 32) * (smem_slots + 2) + 64;
   spill_parts.alloc(part_cap * row_words * 8, ctx->stream);
   if (go_part && smem_slots > 0) setup_partitioned(nrows);
+}
+
+// Uploads the heavy hitters' table for smem_slots slots.
+void AggState::preload_hot() {
+  const int want = cfg.hot_keys > 0 ? cfg.hot_keys : smem_slots;
+  const std::vector<uint64_t> hot = hot_table(std::min(want, smem_slots * 17 / 20), smem_slots, &nhot);
+  hot_keys_dev.alloc(hot.size() * 8, ctx->stream);
+  QEG_CUDA(cudaMemcpyAsync(hot_keys_dev.get(), hot.data(), hot.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
+  QEG_CUDA(cudaStreamSynchronize(ctx->stream));
+}
+
+// The private tables that keep their size from batch to batch (partitioned
+// passes, preloaded heavy hitters) were laid out for the first batch's fields:
+// a batch whose values have NULLs needs their counts too, and may not fit with
+// as many slots. It gets fewer, and a heavy hitters' table of that size.
+void AggState::fit_private(const std::vector<StagedCol>& staged) {
+  if (mode != 1 || (strategy != QEG_AGG_PARTITIONED && nhot == 0)) return;
+  uint32_t skip = 0;
+  for (size_t c = 0; c < val_cols.size(); ++c)
+    if (staged[val_cols[c]].dev.all_valid) skip |= null_field(static_cast<int>(c));
+  const int most = priv_max_slots(skip);
+  if (smem_slots <= most) return;
+  smem_slots = most;
+  if (nhot > 0) preload_hot();
 }
 
 bool AggState::part_eligible(const std::vector<StagedCol>& staged) const {

@@ -1,6 +1,6 @@
 """GROUP BY over sequences of batches whose route changes on the way, against
 the oracle: packed pairs of 4-byte keys that were partitioned and then meet a
-NULL key."""
+NULL key, partitioned and preloaded private tables whose values gain NULLs."""
 import numpy as np
 import pytest
 
@@ -50,5 +50,31 @@ def test_packed_pair_partitioned_then_null_keys(ctx, null_key):
         for b in batches[1:]:
             agg.consume([to_gpu(c) for c in b])
         check(agg, batches, [0, 1], aggs)
+    finally:
+        agg.close()
+
+
+@pytest.mark.parametrize("strategy", [qeg.AGG_PARTITIONED, qeg.AGG_SMEM])
+@pytest.mark.parametrize("ncols,t", [(2, O.F64), (3, O.I64)])
+def test_values_gain_nulls(ctx, strategy, ncols, t):
+    # As many private slots as fit without NULL counts: with them the same
+    # number does not. The heavy hitters are preloaded.
+    rng = np.random.default_rng(ncols)
+
+    def batch(n, nulls):
+        key = (30_000 ** rng.random(n)).astype(np.int64) - 1
+        vals = [rng.normal(0, 9, n) if t == O.F64 else rng.integers(-99, 99, n) for _ in range(ncols)]
+        return [O.TCol(O.I64, key * 0x51ED270B7)] + [O.TCol(t, v, rng.random(n) > 0.2 if nulls else None) for v in vals]
+
+    batches = [batch(300_000, False), batch(200_003, True), batch(100_001, False)]
+    aggs = [(f, c) for c in range(1, ncols + 1) for f in (O.SUM, O.MIN, O.MAX)]
+    agg = qeg.Aggregate(ctx, [c.type for c in batches[0]], [0], aggs,
+                        qeg.agg_config(strategy=strategy, hot_keys=4096, smem_slots=4096, expected_groups=30_000))
+    try:
+        for b in batches:
+            agg.consume([to_gpu(c) for c in b])
+            st = agg.stats()
+            assert st["strategy"] == strategy and st["hot_keys"] > 500, st
+        check(agg, batches, [0], aggs)
     finally:
         agg.close()
