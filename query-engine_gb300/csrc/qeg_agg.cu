@@ -1836,8 +1836,11 @@ bool AggState::can_pack(const std::vector<StagedCol>& staged, uint64_t len) {
   return qmin >= INT32_MIN && qmax <= INT32_MAX;
 }
 
-// Converts the packed single-key table into composite rows (same capacity),
-// after which the window or GROUP BY runs as an ordinary composite-key one.
+// Converts the packed single-key table into composite rows, after which the
+// window or GROUP BY runs as an ordinary composite-key one. A single-key table
+// fills to 0.85 before it grows, where runs of taken slots pass the probe limit
+// even in small tables: the composite one is at most half full, and its rows
+// are placed however far the search takes (as a grown table's are).
 // The tail rows of a partitioned batch are single-key rows too: they join the
 // table first.
 void AggState::unpack() {
@@ -1855,11 +1858,12 @@ void AggState::unpack() {
   strategy = QEG_AGG_GLOBAL;
   smem_slots = 0;
   nhot = 0;
-  alloc_table(old_cap);
+  alloc_table(std::max(old_cap, next_pow2(2 * (inserted + 1))));
   part_cap = static_cast<uint64_t>(ctx->sms) * 32 * 2 + 64;
   spill_parts.alloc(part_cap * row_words * 8, ctx->stream);
   QEG_CUDA(cudaMemsetAsync(counters.get<uint8_t>() + 16, 0, 8, ctx->stream));
   AggK P = kparams_base();
+  P.probe_limit = static_cast<int>(std::min<uint64_t>(cap, 1u << 30));
   const unsigned g = grid_for(ctx, old_cap + 2, 256, 8);
   unpack_kernel<<<g, 256, 0, ctx->stream>>>(P, old.get<uint64_t>(), old_cap, old_w, bucket_width, types[keys[0]],
                                             types[keys[1]]);

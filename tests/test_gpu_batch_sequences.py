@@ -1,6 +1,7 @@
 """GROUP BY over sequences of batches whose route changes on the way, against
 the oracle: packed pairs of 4-byte keys that were partitioned and then meet a
-NULL key, partitioned and preloaded private tables whose values gain NULLs."""
+NULL key, partitioned and preloaded private tables whose values gain NULLs,
+packed tables that are nearly full."""
 import numpy as np
 import pytest
 
@@ -76,5 +77,29 @@ def test_values_gain_nulls(ctx, strategy, ncols, t):
             st = agg.stats()
             assert st["strategy"] == strategy and st["hot_keys"] > 500, st
         check(agg, batches, [0], aggs)
+    finally:
+        agg.close()
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_nearly_full_packed_table_meets_null_keys(ctx, seed):
+    rng = np.random.default_rng(seed)
+    cap = 1024 << (seed % 4)
+    first = cap * 6 // 10 - 64  # (the table has first / 0.6 + 64 slots)
+    keys = rng.permutation(1 << 24)[:cap * 82 // 100]  # 0.82 of its slots taken
+
+    def batch(k, nulls):
+        n = len(k)
+        return [O.TCol(O.I32, (k >> 12).astype(np.int32)), O.TCol(O.I32, (k & 4095).astype(np.int32),
+                rng.random(n) > 0.5 if nulls else None), O.TCol(O.I64, rng.integers(0, 9, n))]
+
+    batches = [batch(keys[:first], False)] + [batch(p, False) for p in np.array_split(keys[first:], 8)]
+    batches.append(batch(keys[:100], True))
+    aggs = [(O.COUNT_STAR, 0), (O.SUM, 2)]
+    agg = qeg.Aggregate(ctx, [c.type for c in batches[0]], [0, 1], aggs)
+    try:
+        for b in batches:
+            agg.consume([to_gpu(c) for c in b])
+        check(agg, batches, [0, 1], aggs)
     finally:
         agg.close()
