@@ -2216,11 +2216,12 @@ void AggState::settle(const std::vector<StagedCol>& staged, uint64_t len) {
 
 void AggState::first_consume(const std::vector<StagedCol>& staged, uint64_t nrows, uint64_t len,
                              const uint32_t* dsel) {
-  // A window with one I32 partition key starts packed when the batch allows.
-  if (packable && can_pack(staged, len)) {
-    packed = true;
-    mode = 1;
-    row_words = 1 + nfields;
+  // Two packable keys start packed when the batch allows. (Decided anew when an
+  // earlier first batch was refused before there was a table.)
+  if (packable) {
+    packed = can_pack(staged, len);
+    mode = packed ? 1 : 2;
+    row_words = (packed ? 1 : 2 + static_cast<int>(keys.size())) + nfields;
   }
   // Sizing. QEG_SIZE_FIXED: the configured (or default) first capacity, grown on
   // overflow. QEG_SIZE_LEARNED: the estimator's group count (see qeg_estimate),

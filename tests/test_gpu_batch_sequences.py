@@ -1,7 +1,7 @@
 """GROUP BY over sequences of batches whose route changes on the way, against
 the oracle: packed pairs of 4-byte keys that were partitioned and then meet a
 NULL key, partitioned and preloaded private tables whose values gain NULLs,
-packed tables that are nearly full."""
+packed tables that are nearly full, and a first batch that was refused."""
 import numpy as np
 import pytest
 
@@ -101,5 +101,26 @@ def test_nearly_full_packed_table_meets_null_keys(ctx, seed):
         for b in batches:
             agg.consume([to_gpu(c) for c in b])
         check(agg, batches, [0, 1], aggs)
+    finally:
+        agg.close()
+
+
+def test_null_keys_after_a_refused_first_batch(ctx):
+    # The first batch starts packed and is refused for its selection, before
+    # there is a table; the next one has NULL keys.
+    rng = np.random.default_rng(5)
+
+    def batch(n, nulls):
+        return [O.TCol(O.I32, rng.integers(0, 5, n).astype(np.int32)),
+                O.TCol(O.I32, rng.integers(0, 5, n).astype(np.int32), rng.random(n) > 0.5 if nulls else None)]
+
+    n = 4_300_000
+    agg = qeg.Aggregate(ctx, [O.I32, O.I32], [0, 1], [(O.COUNT_STAR, 0)])
+    try:
+        with pytest.raises(qeg.QegError):
+            agg.consume([to_gpu(c) for c in batch(n, False)], np.full(n, n, np.uint32))
+        b = batch(10_000, True)
+        agg.consume([to_gpu(c) for c in b])
+        check(agg, [b], [0, 1], [(O.COUNT_STAR, 0)])
     finally:
         agg.close()
