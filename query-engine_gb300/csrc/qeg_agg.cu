@@ -2158,8 +2158,9 @@ void AggState::consume(const qeg_column* cols, int ncols, const uint32_t* sel, u
   if (!table.get()) first_consume(staged, nrows, len, dsel);
   else if (packed && !can_pack(staged, len)) unpack();
   if (nrows > spill_cap) {  // a later, larger batch: the spill list must hold all of it
+    spill_cap = 0;
+    spill_rows.alloc(nrows * 4, ctx->stream);
     spill_cap = nrows;
-    spill_rows.alloc(spill_cap * 4, ctx->stream);
   }
   rows_seen += nrows;
   if (nrows == 0) return;

@@ -36,6 +36,7 @@ struct Error : std::runtime_error {
 
 inline void cuda_check(cudaError_t e, const char* what) {
   if (e == cudaSuccess) return;
+  cudaGetLastError();  // reported here, not by the next launch's check
   if (e == cudaErrorMemoryAllocation)
     throw Error(QEG_ERR_OOM, std::string(what) + ": out of device memory");
   throw Error(QEG_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
@@ -68,8 +69,8 @@ class DevBuf {
   void alloc(size_t bytes, cudaStream_t s) {
     release();
     stream_ = s;
-    bytes_ = bytes;
     if (bytes) QEG_CUDA(cudaMallocAsync(&ptr_, bytes, s));
+    bytes_ = bytes;  // (a failed allocation leaves an empty buffer)
   }
   void release() {
     if (ptr_) cudaFreeAsync(ptr_, stream_);

@@ -2679,7 +2679,8 @@ struct JoinState {
   DevBuf packed;
   int packed_words = 0, packed_mask = 0;
   std::vector<int> packed_off;
-  bool pack_rows(uint64_t count);
+  bool pack_refused = false;  // there was no memory for them
+  void pack_rows(uint64_t count);
   bool rows_ready = false;  // unique keys: `rows` holds the build row of every slot
   void ensure_rows();
 
@@ -3226,12 +3227,15 @@ void JoinState::ensure_rows() {
 
 // Packs the build columns into rows when an output of `count` rows pays for
 // the pass (it reads and writes every build row once; each output row then
-// saves a random access per column and validity byte) and a row fits 64
-// bytes. Returns whether packed rows are there.
-bool JoinState::pack_rows(uint64_t count) {
-  if (packed_words) return true;
+// saves a random access per column and validity byte), a row fits 64 bytes
+// and the output has one gather pass for all columns. Without memory for them
+// (up to 64 bytes per build row) the columns are gathered one by one.
+void JoinState::pack_rows(uint64_t count) {
+  if (packed_words || pack_refused) return;
   const int nc = static_cast<int>(btypes.size());
-  if (nc == 0 || nc > kMaxGatherCols || nbuild == 0 || count < 65536 || count * 2 < nbuild) return false;
+  if (ptypes.size() + btypes.size() > static_cast<size_t>(kMaxGatherCols) || nbuild == 0 || count < 65536 ||
+      count * 2 < nbuild)
+    return;
   packed_off.assign(nc, 0);
   int at = 0;
   for (int w : {8, 4, 1})
@@ -3242,7 +3246,7 @@ bool JoinState::pack_rows(uint64_t count) {
       }
   packed_mask = (at + 3) / 4 * 4;
   const int words = packed_mask + 4 <= 32 ? 4 : packed_mask + 4 <= 64 ? 8 : 0;
-  if (words == 0) return false;
+  if (words == 0) return;
   GatherK G{};
   G.ncols = nc;
   G.mask_off = packed_mask;
@@ -3253,14 +3257,19 @@ bool JoinState::pack_rows(uint64_t count) {
     G.c[c].off = packed_off[c];
     G.c[c].bit = c;
   }
-  packed.alloc(nbuild * words * 8, ctx->stream);
+  try {
+    packed.alloc(nbuild * words * 8, ctx->stream);
+  } catch (const Error& e) {
+    if (e.code != QEG_ERR_OOM) throw;
+    pack_refused = true;  // (not asked for again with every fetch)
+    return;
+  }
   const unsigned g = grid_for(ctx, nbuild, 256, 8);
   if (words == 4) pack_rows_kernel<4><<<g, 256, 0, ctx->stream>>>(G, nbuild, packed.get<uint64_t>());
   else pack_rows_kernel<8><<<g, 256, 0, ctx->stream>>>(G, nbuild, packed.get<uint64_t>());
   ctx->launches++;
   QEG_CUDA(cudaGetLastError());
   packed_words = words;
-  return true;
 }
 
 }  // namespace qeg
@@ -3667,8 +3676,16 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
       // start: probe columns are plain copies, made by the copy engines on a
       // side stream while the gather kernel fills the build columns.
       std::vector<char> copied(ncol, 0);
-      bool forked = false;
       DevBuf tmp_words;
+      // (Destroyed before flags and tmp_words: an error on the way must not
+      // leave copies under way into them or the caller's buffers.)
+      struct Fork {
+        qeg_ctx* ctx;
+        bool open = false;
+        ~Fork() {
+          if (open) cudaStreamSynchronize(ctx->side);
+        }
+      } fork{ctx};
       if (st.probe_identity && first % 64 == 0) {
         const uint64_t nw = (count + 63) / 64;
         auto copyable = [&](size_t c) { return !(st.ptypes[c] == QEG_STR && st.probe_staged[c].dev.code_map); };
@@ -3683,7 +3700,7 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
         }
         QEG_CUDA(cudaEventRecord(ctx->side_in, ctx->stream));
         QEG_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_in, 0));
-        forked = true;
+        fork.open = true;
         size_t itmp = 0;
         for (size_t c = 0; c < st.ptypes.size(); ++c) {
           if (!copyable(c)) continue;  // dictionary codes need translating: gathered below
@@ -3715,7 +3732,10 @@ qeg_status qeg_join_fetch(qeg_join* j, uint64_t first, uint64_t count, const qeg
           if (!copied[c]) gather_col(G.c[G.ncols++], c, outs[c].data, outs[c].validity);
         if (G.ncols > 0) launch_gather(G, first, gw);
       }
-      if (forked) QEG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->side_out, 0));
+      if (fork.open) {
+        QEG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->side_out, 0));
+        fork.open = false;
+      }
       for (size_t c = 0; c < ncol && ncol > static_cast<size_t>(kMaxGatherCols); ++c) {
         const bool pc = c < st.ptypes.size();
         const size_t bc = pc ? 0 : c - st.ptypes.size();

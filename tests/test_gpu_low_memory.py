@@ -1,0 +1,56 @@
+"""Calls that take memory for speed alone answer without it: joins whose build
+rows cannot be packed side by side."""
+import numpy as np
+import pytest
+import torch
+
+import oracle as O
+import qeg
+from mempool import limited_pool
+from util import to_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("device", [False, True])
+@pytest.mark.parametrize("join_type", [O.INNER, O.LEFT])
+def test_fetch_without_room_for_packed_rows(ctx, device, join_type):
+    rng = np.random.default_rng(2)
+    nb, n = 1 << 22, 2_400_000  # packed: 64 bytes a row, 256 MB
+    bkey = rng.permutation(nb) * 0x51ED270B7
+    build = [O.TCol(O.I64, bkey)] + [O.TCol(O.I64, rng.integers(0, 1 << 40, nb), rng.random(nb) > 0.1 if c else None)
+                                     for c in range(4)]
+    at = rng.integers(0, nb, n)
+    miss = rng.random(n) < 0.1
+    probe = [O.TCol(O.I64, np.where(miss, -1, bkey[at])), O.TCol(O.I32, np.arange(n, dtype=np.int32), rng.random(n) > 0.3)]
+    j = qeg.Join(ctx, [c.type for c in probe], [c.type for c in build], [0], [0], join_type)
+    try:
+        j.build([to_gpu(c, device=True) for c in build])
+        j.build_finish()
+        cols = [to_gpu(c, device=True) for c in probe]
+        m = j.probe(cols)
+        keep = np.arange(n) if join_type == O.LEFT else np.flatnonzero(~miss)
+        assert m == len(keep)
+        with limited_pool(224 << 20):
+            got = j.fetch_device() if device else j.fetch()
+            ctx.synchronize()
+        with pytest.raises(qeg.QegError):  # (the pool is as small as it says)
+            with limited_pool(32 << 20):
+                k = qeg.Join(ctx, [O.I64], [O.I64] * 5, [0], [0], O.INNER)
+                try:
+                    k.build([to_gpu(c, device=True) for c in build])
+                finally:
+                    k.close()
+                    ctx.synchronize()
+        for c, (v, w) in enumerate(got):
+            if device:
+                v, w = v[:m].cpu().numpy(), qeg.unpack_validity(w.cpu().numpy().view(np.uint64), m)
+            src = probe[c] if c < 2 else build[c - 2]
+            row = keep if c < 2 else at[keep]
+            ok = np.ones(len(src.values), bool) if src.valid is None else src.valid
+            ok = ok[row] if c < 2 else ok[row] & ~miss[keep]
+            assert np.array_equal(w, ok), c
+            assert np.array_equal(v[ok], src.values[row][ok]), c
+    finally:
+        j.close()
+        torch.cuda.synchronize()
