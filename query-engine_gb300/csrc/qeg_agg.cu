@@ -2514,8 +2514,22 @@ void AggState::consume_partitioned(const std::vector<StagedCol>& staged, uint64_
     read_words_and_error(ctx, total, 1, &pooled);
     Q.total = pooled;
   }
-  const size_t pool_bytes = std::max<uint64_t>(Q.total, 1) * kern.words * 8;
-  if (pool.bytes() < pool_bytes) pool.alloc(pool_bytes, ctx->stream);
+  // The pool takes 16 bytes or more per row that is not a heavy hitter's. An
+  // input that would otherwise go to the private tables and the global one
+  // does not depend on that memory: without it the batch goes there.
+  try {
+    const size_t pool_bytes = std::max<uint64_t>(Q.total, 1) * kern.words * 8;
+    if (pool.bytes() < pool_bytes) pool.alloc(pool_bytes, ctx->stream);
+    if (tails_cap == 0) alloc_tails(static_cast<uint64_t>(std::max(1.25 * est_groups, 4096.0)));
+  } catch (const Error& e) {
+    if (e.code != QEG_ERR_OOM) throw;
+    pool.release();
+    tails.release();
+    tails_cap = 0;
+    launch(P, nrows);
+    settle(staged, len);
+    return;
+  }
   Q.rows = pool.get<uint64_t>();
   {
     PrivK A = priv_layout(fkind.data(), nfields, smem_slots, skip, kPrivReps);
@@ -2540,10 +2554,6 @@ void AggState::consume_partitioned(const std::vector<StagedCol>& staged, uint64_
   priv_sums_for(A, grid);
   if (!part_counters.get()) part_counters.alloc(16, ctx->stream);
   if (part_failed.bytes() < np * 4) part_failed.alloc(np * 4, ctx->stream);
-  if (tails_cap == 0) {
-    tails_cap = static_cast<uint64_t>(std::max(1.25 * est_groups, 4096.0));
-    tails.alloc((tails_cap + 2) * row_words * 8, ctx->stream);
-  }
   PartB B{};
   B.counters = part_counters.get<unsigned long long>();
   B.failed = part_failed.get<uint32_t>();
@@ -2560,8 +2570,7 @@ void AggState::consume_partitioned(const std::vector<StagedCol>& staged, uint64_
     if (cnt[0] <= tails_cap) break;
     // More groups than the tail buffer holds: size it to the count and re-run
     // (the pass only reads the pool).
-    tails_cap = cnt[0] + cnt[0] / 8 + 4096;
-    tails.alloc((tails_cap + 2) * row_words * 8, ctx->stream);
+    alloc_tails(cnt[0] + cnt[0] / 8 + 4096);
   }
   ntails = cnt[0];
   // Two empty rows after the tails: the finalize pass reads a single-key
@@ -2594,6 +2603,13 @@ void AggState::consume_partitioned(const std::vector<StagedCol>& staged, uint64_
     grow(std::max<uint64_t>(cap * 2, next_pow2(2 * (inserted + nlist / 4))));
   }
   QEG_CUDA(cudaMemsetAsync(counters.get(), 0, 16, ctx->stream));
+}
+
+// Room for `rows` tail rows and the two empty ones behind them.
+void AggState::alloc_tails(uint64_t rows) {
+  tails_cap = 0;
+  tails.alloc((rows + 2) * row_words * 8, ctx->stream);
+  tails_cap = rows;
 }
 
 // The launch's blocks of F64 sums, one per CTA.

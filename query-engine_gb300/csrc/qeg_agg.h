@@ -196,6 +196,7 @@ struct AggState {
   bool part_eligible(const std::vector<StagedCol>& staged) const;
   int part_table_slots(uint32_t skip) const;
   std::vector<uint64_t> hot_table(int want, int S, int* count) const;
+  void alloc_tails(uint64_t rows);
   void preload_hot();
   void fit_private(const std::vector<StagedCol>& staged);
   void priv_sums_for(struct PrivK& A, uint64_t grid);

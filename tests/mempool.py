@@ -25,7 +25,6 @@ def limited_pool(limit, device=0):
     rt.cudaMemPoolCreate.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(PoolProps)]
     rt.cudaDeviceSetMemPool.argtypes = [ctypes.c_int, ctypes.c_void_p]
     rt.cudaDeviceGetMemPool.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_int]
-    rt.cudaMemPoolDestroy.argtypes = [ctypes.c_void_p]
     before, pool = ctypes.c_void_p(), ctypes.c_void_p()
     _ok(rt.cudaDeviceGetMemPool(ctypes.byref(before), device))
     props = PoolProps(1, 0, Location(1, device), None, limit)  # pinned to the device, no export handles
@@ -34,5 +33,5 @@ def limited_pool(limit, device=0):
     try:
         yield
     finally:
+        # (The pool itself stays: buffers from it are freed after this.)
         _ok(rt.cudaDeviceSetMemPool(device, before))
-        _ok(rt.cudaMemPoolDestroy(pool))  # (what was allocated from it stays usable until freed)

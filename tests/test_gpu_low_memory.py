@@ -1,5 +1,5 @@
 """Calls that take memory for speed alone answer without it: joins whose build
-rows cannot be packed side by side."""
+rows cannot be packed side by side, partitioned GROUP BYs without their pool."""
 import numpy as np
 import pytest
 import torch
@@ -54,3 +54,32 @@ def test_fetch_without_room_for_packed_rows(ctx, device, join_type):
     finally:
         j.close()
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("hot_keys", [0, 64])
+def test_partitioned_groupby_without_room_for_its_pool(ctx, hot_keys):
+    # The pool would take 16 bytes a row, 128 MB; everything else fits.
+    n, dom = 1 << 23, 100_000
+    g = torch.Generator(device="cuda").manual_seed(4)
+    a = qeg.Aggregate(ctx, [O.I64], [0], [(O.COUNT_STAR, 0)],
+                      qeg.agg_config(strategy=qeg.AGG_PARTITIONED, hot_keys=hot_keys, expected_groups=dom))
+    try:
+        want = torch.zeros(dom, dtype=torch.int64, device="cuda")
+        for limit in (112 << 20, 112 << 20, 0):  # twice without the pool, then with it
+            key = (dom ** torch.rand(n, device="cuda", dtype=torch.float64, generator=g)).long() - 1
+            want += torch.bincount(key, minlength=dom)
+            torch.cuda.synchronize()
+            if limit:
+                with limited_pool(limit):
+                    a.consume([qeg.Col(key)])
+                    ctx.synchronize()
+            else:
+                a.consume([qeg.Col(key)])
+        assert a.finish() == int((want > 0).sum())
+        (k, _), (c, _) = a.fetch()
+        assert a.stats()["strategy"] == qeg.AGG_PARTITIONED
+        got = np.zeros(dom, np.int64)
+        got[k] = c
+        assert np.array_equal(got, want.cpu().numpy())
+    finally:
+        a.close()
