@@ -37,6 +37,7 @@ namespace qeg {
 namespace {
 
 constexpr uint32_t kNullRow = 0xffffffffu;  // ops/join_internal.h:31
+constexpr uint64_t kNoSlot = ~0ull;
 // Hashed single-key tables of at least this many bytes get a Bloom filter of
 // kBloomBitsPerKey bits per build row: 16 bits and four bits per key in one
 // 32-bit word give a false positive rate of about 0.8%, in 32 MB for 16M build
@@ -418,6 +419,7 @@ struct ProbeK {
   uint32_t* counts;    // per probe row output rows
   const uint64_t* starts;
   uint32_t* match;     // per probe row: build row (unique build keys) or slot
+  uint64_t* match64;   // repeated build keys, tables of 2^32-1 slots or more: the slot (kNoSlot: none)
   uint32_t* out_probe;
   uint32_t* out_build;
   unsigned long long* acc;  // sink: [0] count, [1] sum, [2] any payload
@@ -1610,7 +1612,7 @@ __global__ void __launch_bounds__(256) build_rows_kernel(const __grid_constant__
 // One lookup per probe row. Unique build keys (P.T.unique): match[p] is the
 // build row or kNullRow, and an inner join counts the matches of every
 // kProbeChunk rows (chunk c: rows of one warp, in order). Repeated keys:
-// counts[p] output rows and the slot in match[p] (kNullRow: none).
+// counts[p] output rows and the slot in match[p] (kNullRow: none) or match64[p].
 constexpr int kProbeChunk = 32 * kProbeU;  // (64)
 template <int NK>
 __global__ void __launch_bounds__(256) probe_match_kernel(const __grid_constant__ ProbeK P) {
@@ -1645,7 +1647,8 @@ __global__ void __launch_bounds__(256) probe_match_kernel(const __grid_constant_
 #pragma unroll
       for (int u = 0; u < kProbeU; ++u) {
         if (!live[u]) continue;
-        P.match[p[u]] = n[u] ? static_cast<uint32_t>(slot[u]) : kNullRow;
+        if (P.match64) P.match64[p[u]] = n[u] ? static_cast<uint64_t>(slot[u]) : kNoSlot;
+        else P.match[p[u]] = n[u] ? static_cast<uint32_t>(slot[u]) : kNullRow;
         P.counts[p[u]] = n[u] == 0 && P.left ? 1 : n[u];
       }
     }
@@ -1685,8 +1688,8 @@ __global__ void probe_emit_kernel(const __grid_constant__ ProbeK P) {
     const uint32_t m = P.counts[p];
     if (m == 0) continue;
     const uint64_t o = P.starts[p];
-    const uint32_t s = P.match[p];
-    if (s == kNullRow) {  // LEFT join, unmatched: one row, build side NULL
+    const uint64_t s = P.match64 ? P.match64[p] : P.match[p] == kNullRow ? kNoSlot : P.match[p];
+    if (s == kNoSlot) {  // LEFT join, unmatched: one row, build side NULL
       P.out_probe[o] = static_cast<uint32_t>(p);
       P.out_build[o] = kNullRow;
       continue;
@@ -3588,13 +3591,17 @@ qeg_status qeg_join_probe(qeg_join* j, const qeg_column* cols, int ncols, uint64
       return;
     }
     st.ensure_csr();
-    require(st.slots() < kNullRow, "join table too large");
-    DevBuf slot(n * 4, ctx->stream);
+    // Slots of a probe batch as 32-bit numbers while the table has fewer than
+    // 2^32-1 (half the bytes); QEG_JOIN_WIDE_SLOTS=1 takes 64-bit ones always
+    // (for tests: a table that needs them has over 2^30 build rows).
+    const bool wide = st.slots() >= kNullRow || getenv("QEG_JOIN_WIDE_SLOTS") != nullptr;
+    DevBuf slot(n * (wide ? 8 : 4), ctx->stream);
     st.counts.alloc(n * 4, ctx->stream);
     st.starts.alloc((n + 1) * 8, ctx->stream);
     ProbeK P = probe_params(st, n);
     P.counts = st.counts.get<uint32_t>();
-    P.match = slot.get<uint32_t>();
+    if (wide) P.match64 = slot.get<uint64_t>();
+    else P.match = slot.get<uint32_t>();
     match<<<g, 256, 0, ctx->stream>>>(P);
     ctx->launches++;
     QEG_CUDA(cudaGetLastError());
