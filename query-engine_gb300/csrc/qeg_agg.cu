@@ -124,52 +124,65 @@ __device__ __forceinline__ uint64_t home_slot(uint64_t h, uint64_t cap) {
 // where want[u]) from their home slots s[u], whose key words were last read as
 // cur[u]: the row of each, or nullptr when it could not be placed within the
 // probe limit. Linear probing. A key word never changes once set, so a stale
-// non-empty value stays correct. Past the home slot's load every probe is one
-// compare-and-swap, which finds the key, claims an empty slot or moves on: a
-// single memory round trip per probe, taken by all lanes and all U keys
-// together. (Looking first and claiming in a branch of its own made the
-// lanes of a warp wait out each other's round trips, up to eight per row:
-// 29,000 clocks per 64 rows of a Zipf(1.1) column, whose rows miss the
-// private tables and mostly L2.)
+// non-empty value stays correct. Behind the home slot a few slots are loaded
+// per step, for all U keys together, and examined in order; only one that
+// reads as empty is claimed by a compare-and-swap. (A compare-and-swap per
+// probe is one round trip less for an insert, but an atomic for every look at
+// a taken slot: 256M Zipf(1.1) rows over 64M keys, 16.6M groups, forced through
+// the private tables 33.9 ms, now 19.0; through the global table alone 107,
+// now 65.) One key takes four slots per step, two keys two each: four would spill
+// registers at 1024 threads (64M uniform rows over 20k groups: 2.31 ms with one
+// or two, 2.80 with four).
 template <int U>
 __device__ __forceinline__ void global_rows1(const AggK& P, bool (&want)[U], const uint64_t (&k)[U], uint64_t (&s)[U],
                                              const uint64_t (&cur)[U], uint64_t* (&r)[U],
                                              unsigned long long& inserted, int limit) {
+  constexpr int kLook = U == 1 ? 4 : 2;
   const int W = P.row_words;
+  auto claim = [&](uint64_t* at, uint64_t key) -> bool {  // whether the slot is the key's now
+    const unsigned long long old =
+        atomicCAS(reinterpret_cast<unsigned long long*>(at), 0ull, static_cast<unsigned long long>(key));
+    inserted += old == 0;
+    return old == 0 || old == key;
+  };
   bool any = false;
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     r[u] = nullptr;
     if (!want[u]) continue;
-    if (cur[u] == k[u]) {
-      r[u] = P.table + s[u] * W;
+    uint64_t* const at = P.table + s[u] * W;
+    if (cur[u] == k[u] || (cur[u] == 0 && claim(at, k[u]))) {
+      r[u] = at;
       want[u] = false;
     } else {
-      if (cur[u] != 0 && ++s[u] == P.cap) s[u] = 0;
+      if (++s[u] == P.cap) s[u] = 0;
       any = true;
     }
   }
-  for (int t = 0; any && t < limit; ++t) {
-    unsigned long long old[U];
+  for (int t = 1; any && t < limit; t += kLook) {
+    uint64_t w[U][kLook];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      old[u] = 0;
-      if (want[u])
-        old[u] = atomicCAS(reinterpret_cast<unsigned long long*>(P.table + s[u] * W), 0ull,
-                           static_cast<unsigned long long>(k[u]));
-    }
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int j = 0; j < kLook; ++j) {
+        w[u][j] = 0;
+        if (want[u]) w[u][j] = ld_relaxed(P.table + (s[u] + j < P.cap ? s[u] + j : s[u] + j - P.cap) * W);
+      }
     any = false;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (!want[u]) continue;
-      if (old[u] == 0 || old[u] == k[u]) {
-        inserted += old[u] == 0;
-        r[u] = P.table + s[u] * W;
-        want[u] = false;
-      } else {
-        if (++s[u] == P.cap) s[u] = 0;
-        any = true;
+#pragma unroll
+      for (int j = 0; j < kLook; ++j) {
+        if (!want[u]) continue;
+        uint64_t* const at = P.table + s[u] * W;
+        if (w[u][j] == k[u] || (w[u][j] == 0 && claim(at, k[u]))) {
+          r[u] = at;
+          want[u] = false;
+        } else if (++s[u] == P.cap) {
+          s[u] = 0;
+        }
       }
+      any |= want[u];
     }
   }
 }
@@ -592,6 +605,7 @@ __global__ void __launch_bounds__(1024) agg_private_kernel(const __grid_constant
   unsigned before = 0;             // the CTA's misses in the window before the last flush
   int wait = 0, backoff = 0;       // windows until the next flush may happen
   int judge = 0;                   // windows until the last flush is judged
+  unsigned decision = 0;           // windows whose misses were summed
   const DevCol& kc = P.key[0];
   const uint64_t per = ((P.nrows + gridDim.x - 1) / gridDim.x + 31) & ~31ull;
   const uint64_t lo = min(per * blockIdx.x, P.nrows), hi = min(lo + per, P.nrows);
@@ -671,24 +685,32 @@ __global__ void __launch_bounds__(1024) agg_private_kernel(const __grid_constant
       tracked = inserted;
     }
     if (insert && (step & (kPrivWindow - 1)) == kPrivWindow - 1) {
+      if (judge > 1 || (judge == 0 && wait > 0)) {
+        // Nothing to decide: no barrier.
+        if (judge > 1) --judge;
+        else --wait;
+        missed = 0;
+        continue;
+      }
       // The window's misses, summed over the CTA (three sums in turn: the one
       // cleared here is next used after another barrier).
-      unsigned* sum = &s_miss[(step / kPrivWindow) % 3];
+      unsigned* sum = &s_miss[decision % 3];
       // Not once the global table is full: a flush would search it in vain for
       // most groups, and its refill would spill.
       if (lane == 0 && missed && !full) atomicAdd(sum, missed);
       missed = 0;
       __syncthreads();
       const unsigned m = *sum;
-      if (threadIdx.x == 0) s_miss[(step / kPrivWindow + 2) % 3] = 0;
+      if (threadIdx.x == 0) s_miss[(decision + 2) % 3] = 0;
+      ++decision;
       // A flush is judged by the second window after it: in the first the
       // refill alone keeps the misses low.
-      if (judge > 0 && --judge == 0) {
+      if (judge > 0) {
+        judge = 0;
         backoff = m < before - before / 5 ? 0 : min(2 * backoff + 1, 63);
         wait = backoff;
       }
-      if (judge > 0) {
-      } else if (wait > 0) {
+      if (wait > 0) {
         --wait;
       } else if (m > span * kPrivWindow / 4) {
         priv_flush1(keys, T, A, P, rep, s_rslot, &s_nrep, false, inserted);

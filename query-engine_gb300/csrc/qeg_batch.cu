@@ -63,9 +63,9 @@ struct BatchK {
 };
 
 // Hash of a batch key word, and a key's row in its query's table: found or
-// claimed, or nullptr (the table is too full; the query is re-run). Past the
-// home slot's look every probe is one compare-and-swap (see global_rows1 in
-// qeg_agg.cu).
+// claimed, or nullptr (the table is too full; the query is re-run). Behind the
+// home slot a few slots are loaded per step, and only one that reads as empty
+// is claimed (see global_rows1 in qeg_agg.cu).
 __device__ __forceinline__ uint64_t batch_hash(uint64_t k) {
   uint64_t x = k * 0x9E3779B97F4A7C15ull;
   x ^= x >> 32;
@@ -74,7 +74,13 @@ __device__ __forceinline__ uint64_t batch_hash(uint64_t k) {
 template <int U>
 __device__ __forceinline__ void batch_global_rows(const BatchK& P, const BatchQ& Q, bool (&want)[U],
                                                   const uint64_t (&k)[U], const uint64_t (&h)[U], uint64_t* (&r)[U]) {
+  constexpr int kLook = U == 1 ? 4 : 2;
   uint64_t* T = P.arena + Q.table_off * P.W;
+  auto claim = [](uint64_t* at, uint64_t key) -> bool {  // whether the slot is the key's now
+    const unsigned long long old =
+        atomicCAS(reinterpret_cast<unsigned long long*>(at), 0ull, static_cast<unsigned long long>(key));
+    return old == 0 || old == key;
+  };
   uint64_t s[U];
   unsigned long long cur[U];
   bool any = false;
@@ -87,31 +93,41 @@ __device__ __forceinline__ void batch_global_rows(const BatchK& P, const BatchQ&
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     if (!want[u]) continue;
-    if (cur[u] == k[u]) {
-      r[u] = T + s[u] * P.W;
+    uint64_t* const at = T + s[u] * P.W;
+    if (cur[u] == k[u] || (cur[u] == 0 && claim(at, k[u]))) {
+      r[u] = at;
       want[u] = false;
     } else {
-      if (cur[u] != 0 && ++s[u] == Q.cap) s[u] = 0;
+      if (++s[u] == Q.cap) s[u] = 0;
       any = true;
     }
   }
-  for (int t = 0; any && t < 128; ++t) {
+  for (int t = 1; any && t < 128; t += kLook) {
+    unsigned long long w[U][kLook];
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (want[u])
-        cur[u] = atomicCAS(reinterpret_cast<unsigned long long*>(T + s[u] * P.W), 0ull,
-                           static_cast<unsigned long long>(k[u]));
+#pragma unroll
+      for (int j = 0; j < kLook; ++j) {
+        w[u][j] = 0;
+        if (want[u])
+          w[u][j] = *reinterpret_cast<volatile unsigned long long*>(
+              T + (s[u] + j < Q.cap ? s[u] + j : s[u] + j - Q.cap) * P.W);
+      }
     any = false;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (!want[u]) continue;
-      if (cur[u] == 0 || cur[u] == k[u]) {
-        r[u] = T + s[u] * P.W;
-        want[u] = false;
-      } else {
-        if (++s[u] == Q.cap) s[u] = 0;
-        any = true;
+#pragma unroll
+      for (int j = 0; j < kLook; ++j) {
+        if (!want[u]) continue;
+        uint64_t* const at = T + s[u] * P.W;
+        if (w[u][j] == k[u] || (w[u][j] == 0 && claim(at, k[u]))) {
+          r[u] = at;
+          want[u] = false;
+        } else if (++s[u] == Q.cap) {
+          s[u] = 0;
+        }
       }
+      any |= want[u];
     }
   }
 }
