@@ -1993,8 +1993,8 @@ int AggState::priv_max_slots(uint32_t skip) const {
   return slots;
 }
 
-// Single key, private tables: one CTA per SM. The table has as many slots as
-// the launch gives each CTA rows, within [256, smem_slots]: clearing and
+// Single key, private tables: 1024 threads per SM. The table has as many slots
+// as the launch gives each CTA rows, within [256, smem_slots]: clearing and
 // flushing a table that no CTA can fill costs a small launch more than its
 // rows.
 void AggState::launch_private1(const AggK& P0, uint64_t nrows) {
@@ -2014,20 +2014,29 @@ void AggState::launch_private1(const AggK& P0, uint64_t nrows) {
   else if (nv <= 4) kern = agg_private_kernel<4, kGenericSpec>;
   else kern = agg_private_kernel<8, kGenericSpec>;
   const int block = block_threads();
-  // A few thousand rows per CTA at least, so the flush stays small.
-  const uint64_t grid = std::max<uint64_t>(
-      1, std::min<uint64_t>((nrows + 4095) / 4096, static_cast<uint64_t>(ctx->sms)));
-  int slots = 256;
-  while (slots < smem_slots && static_cast<uint64_t>(slots) * grid < nrows) slots *= 2;
-  if (P.nhot > 0) slots = smem_slots;  // preloaded
   uint32_t skip = 0;
   for (int c = 0; c < nv; ++c)
     if (P.val[c].all_valid) skip |= null_field(c);
-  slots = std::min({slots, smem_slots, priv_max_slots(skip)});
+  const int most = std::min(smem_slots, priv_max_slots(skip));
+  // A few thousand rows per CTA at least, so the flush stays small. A CTA of
+  // fewer than 1024 threads shares its SM with others as far as their tables
+  // (and the partial-row list) allow: 64M Zipf(1.1) rows over 100k keys, 1024
+  // slots, 256 threads 4.6 ms with one CTA per SM, 1.8 now.
+  const size_t full = priv_layout(fkind.data(), nfields, most, skip, kPrivReps).bytes;
+  const uint64_t per_sm = std::max<uint64_t>(
+      1, std::min<uint64_t>({static_cast<uint64_t>(1024 / block),
+                             static_cast<uint64_t>(blocks_per_sm(reinterpret_cast<const void*>(kern), block, full)),
+                             part_cap / (static_cast<uint64_t>(ctx->sms) * (most + 2))}));
+  const uint64_t grid = std::max<uint64_t>(
+      1, std::min<uint64_t>((nrows + 4095) / 4096, static_cast<uint64_t>(ctx->sms) * per_sm));
+  int slots = 256;
+  while (slots < most && static_cast<uint64_t>(slots) * grid < nrows) slots *= 2;
+  if (P.nhot > 0) slots = smem_slots;  // preloaded
+  slots = std::min(slots, most);
   PrivK A = priv_layout(fkind.data(), nfields, slots, skip, kPrivReps);
   priv_sums_for(A, grid);
-  const int per_sm = blocks_per_sm(reinterpret_cast<const void*>(kern), block, A.bytes);
-  require(per_sm > 0, "aggregate kernel does not fit on an SM with this configuration");
+  require(blocks_per_sm(reinterpret_cast<const void*>(kern), block, A.bytes) > 0,
+          "aggregate kernel does not fit on an SM with this configuration");
   kern<<<(unsigned)grid, block, A.bytes, ctx->stream>>>(P, A);
   ctx->launches++;
   QEG_CUDA(cudaGetLastError());
@@ -2361,8 +2370,10 @@ void AggState::first_consume(const std::vector<StagedCol>& staged, uint64_t nrow
   } else {
     smem_slots = 0;
   }
-  // At most two private tables per SM; the composite tables run more CTAs.
-  part_cap = static_cast<uint64_t>(ctx->sms) * (mode == 1 ? 2 : 32) * (smem_slots + 2) + 64;
+  // At most 2 private tables per SM (1024 threads in all, so more of smaller
+  // CTAs, each with fewer slots); the composite tables run more CTAs.
+  const int tables = mode == 1 ? std::max(2, std::min(1024 / block_threads(), 16384 / (smem_slots + 2))) : 32;
+  part_cap = static_cast<uint64_t>(ctx->sms) * tables * (smem_slots + 2) + 64;
   spill_parts.alloc(part_cap * row_words * 8, ctx->stream);
   if (go_part && smem_slots > 0) setup_partitioned(nrows);
 }
