@@ -59,7 +59,7 @@ struct PipeK {
   // The same as u16 group ids (0xffff: no match, 0xfffe: several) when the
   // groups number at most 65533, for the trades kernel's shared-memory copy.
   const uint16_t* kf16;
-  const uint32_t* glist;   // group ids
+  const uint32_t* glist;   // group ids (kfirst for unique build keys)
   DevCol val[kPipeMaxVals];
   int nvals;
   uint8_t fkind[kMaxFields];
@@ -809,27 +809,28 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
     // Group of each join value's build row, while every value has one row.
     constexpr uint32_t kNoGroup = 0xffffffffu;
     std::vector<uint32_t> vgroup(vrange, kNoGroup);
-    bool single = true;
-    for (size_t i = 0; i < bval.size() && single; ++i) {
+    bool unique = true;
+    for (size_t i = 0; i < bval.size() && unique; ++i) {
       uint32_t& g = vgroup[static_cast<size_t>(bval[i] - vmin)];
-      single = g == kNoGroup;
+      unique = g == kNoGroup;
       g = bgrp[i];
     }
     // Translation of the probe keys. kfirst: the group of a key that matches
     // exactly one build row, kNoGroup for none, else the key's slot with the
     // top bit set. Every key's groups are glist[kstart[s]...] (kcount[s] of
-    // them): the shared-state kernel reads these alone.
+    // them): the shared-state kernel reads these alone. Unique build keys need
+    // no list: kfirst is theirs. single: no probe key matches several rows.
     const uint64_t nslots = std::max<uint64_t>(domain, 1);
     std::vector<uint32_t> kfirst(nslots, kNoGroup), kstart, kcount, glist;
     auto slot_value = [&](uint64_t sl) {
       return kt == QEG_STR ? static_cast<int64_t>(pmap[sl]) : kmin + static_cast<int64_t>(sl);
     };
-    if (single) {
+    bool single = true;
+    if (unique) {
       for (uint64_t sl = 0; sl < domain; ++sl) {
         const int64_t v = slot_value(sl);
         if (v >= vmin && v <= vmax) kfirst[sl] = vgroup[static_cast<size_t>(v - vmin)];
       }
-      glist = kfirst;
       kstart.resize(nslots);
       kcount.resize(nslots);
       for (uint64_t sl = 0; sl < nslots; ++sl) {
@@ -856,6 +857,7 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
         kcount[sl] = vstart[i + 1] - vstart[i];
         if (kcount[sl] == 1) kfirst[sl] = glist[kstart[sl]];
         else if (kcount[sl] > 1) kfirst[sl] = 0x80000000u | static_cast<uint32_t>(sl);
+        single = single && kcount[sl] <= 1;
       }
     }
 
@@ -963,7 +965,7 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
     // The translation tables go to the device in one copy from the context's
     // page-locked buffer into one device buffer: kstart, kcount, kfirst,
     // glist (u32 each), then kf16 (u16); the state is zeroed beside them.
-    const size_t n_kst = kstart.size(), n_kfi = kfirst.size(), n_gl = std::max<size_t>(glist.size(), 1);
+    const size_t n_kst = kstart.size(), n_kfi = kfirst.size(), n_gl = unique ? 0 : std::max<size_t>(glist.size(), 1);
     const size_t o_kst = 0, o_kct = o_kst + n_kst * 4, o_kfi = o_kct + n_kst * 4, o_gl = o_kfi + n_kfi * 4;
     const size_t o_k16 = (o_gl + n_gl * 4 + 15) & ~size_t{15};
     const size_t tbl_bytes = o_k16 + ((std::max<size_t>(kf16.size(), 1) * 2 + 15) & ~size_t{15});
@@ -981,7 +983,7 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
     P.kcount = reinterpret_cast<const uint32_t*>(dt + o_kct);
     P.kfirst = reinterpret_cast<const uint32_t*>(dt + o_kfi);
     P.kf16 = kf16.empty() ? nullptr : reinterpret_cast<const uint16_t*>(dt + o_k16);
-    P.glist = reinterpret_cast<const uint32_t*>(dt + o_gl);
+    P.glist = unique ? P.kfirst : reinterpret_cast<const uint32_t*>(dt + o_gl);
     P.state = dstate.get<unsigned long long>();
     const int block = 512;
     // The kernel for this field set: COUNT(*) with SUM/AVG over an F64 column
