@@ -253,11 +253,13 @@ void fetch_columns(qeg_ctx* ctx, const FetchCol* cols, int ncols, uint64_t first
   // kSmallFetch bytes about as much in all.
   constexpr size_t kSmallFetch = 256 << 10;
   // Device words go straight to the caller when they are 8-byte aligned.
-  std::vector<bool> dev_data(ncols), dev_words(ncols), copy_words(ncols);
+  // Memory of another device than the context's goes by copies.
+  std::vector<bool> dev_data(ncols), dev_words(ncols), copy_words(ncols), far_data(ncols);
   size_t host_bytes = 0;
   for (int c = 0; c < ncols; ++c) {
     dev_data[c] = outs[c].data && is_device_ptr(outs[c].data);
     dev_words[c] = outs[c].validity && is_device_ptr(outs[c].validity);
+    far_data[c] = dev_data[c] && !kernel_reaches(outs[c].data, ctx->device);
     if (outs[c].data && !dev_data[c]) host_bytes += (count * cols[c].width + 15) / 16 * 16;
     if (outs[c].validity && !dev_words[c]) host_bytes += (nw * 8 + 15) / 16 * 16;
   }
@@ -265,7 +267,9 @@ void fetch_columns(qeg_ctx* ctx, const FetchCol* cols, int ncols, uint64_t first
   bool any_copy = false;
   for (int c = 0; c < ncols; ++c) {
     copy_words[c] = outs[c].validity &&
-                    (dev_words[c] ? reinterpret_cast<uintptr_t>(outs[c].validity) % 8 != 0 : !small);
+                    (dev_words[c] ? reinterpret_cast<uintptr_t>(outs[c].validity) % 8 != 0 ||
+                                        !kernel_reaches(outs[c].validity, ctx->device)
+                                  : !small);
     any_copy = any_copy || copy_words[c];
   }
   uint8_t* pin = static_cast<uint8_t*>(ctx->pinned_in.reserve(flag_bytes + (small ? host_bytes : 0)));
@@ -282,13 +286,13 @@ void fetch_columns(qeg_ctx* ctx, const FetchCol* cols, int ncols, uint64_t first
     P.vals[c] = static_cast<const uint8_t*>(cols[c].vals) + first * cols[c].width;
     P.valid[c] = cols[c].valid + first;
     P.width[c] = static_cast<uint8_t>(cols[c].width);
-    if (dev_data[c]) {
+    if (dev_data[c] && !far_data[c]) {
       P.dst[c] = static_cast<uint8_t*>(outs[c].data);
-    } else if (outs[c].data && small) {
+    } else if (outs[c].data && !dev_data[c] && small) {
       P.dst[c] = pin_data[c] = at;
       at += (bytes + 15) / 16 * 16;
     } else if (outs[c].data) {
-      QEG_CUDA(cudaMemcpyAsync(outs[c].data, P.vals[c], bytes, cudaMemcpyDeviceToHost, ctx->stream));
+      QEG_CUDA(cudaMemcpyAsync(outs[c].data, P.vals[c], bytes, cudaMemcpyDefault, ctx->stream));
     }
     if (copy_words[c]) {
       P.words[c] = staged.get<uint64_t>() + nw * c;

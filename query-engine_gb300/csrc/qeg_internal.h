@@ -114,6 +114,17 @@ inline bool is_device_ptr(const void* p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// Whether a kernel on `device` may read and write p: device memory of that device, or
+// managed memory. Another device's memory is reached by copies.
+inline bool kernel_reaches(const void* p, int device) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeManaged || (a.type == cudaMemoryTypeDevice && a.device == device);
+}
+
 struct Mlp;
 
 }  // namespace qeg

@@ -651,13 +651,15 @@ qeg_status qeg_filter_join_agg(qeg_ctx* ctx, const qeg_column* probe, int nprobe
     }
     uint8_t* fetched = static_cast<uint8_t*>(ctx->pinned_in.reserve(std::max<size_t>(fetch_bytes, 16)));
     // Device arrays: one kernel writes all of them into the page-locked buffer
-    // (a copy command each costs more than its bytes); large ones are copied.
+    // (a copy command each costs more than its bytes); large ones, and those of
+    // another device, are copied.
     CollectK C{};
     for (const Fetch& f : fetches) {
       if (f.bytes == 0) continue;
       if (!f.dev) {
         std::memcpy(fetched + f.off, f.src, f.bytes);
-      } else if (f.bytes <= kCollectBytes && reinterpret_cast<uintptr_t>(f.src) % 4 == 0 && f.bytes % 4 == 0) {
+      } else if (f.bytes <= kCollectBytes && reinterpret_cast<uintptr_t>(f.src) % 4 == 0 && f.bytes % 4 == 0 &&
+                 kernel_reaches(f.src, ctx->device)) {
         C.src[C.n] = static_cast<const uint32_t*>(f.src);
         C.dst[C.n] = reinterpret_cast<uint32_t*>(fetched + f.off);
         C.words[C.n++] = static_cast<uint32_t>(f.bytes / 4);
