@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(256) build_insert1_kernel(const __grid_constan
   unsigned long long fresh = 0;
   uint32_t dup = 0;
   const uint64_t step = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  const uint64_t limit = P.ovf ? min(P.probe_limit, P.T.cap) : P.T.cap;
+  const uint32_t limit = static_cast<uint32_t>((P.ovf ? min(P.probe_limit, P.T.cap) : P.T.cap) / 4);  // buckets
   unsigned long long* const slots = reinterpret_cast<unsigned long long*>(P.T.keys);
   for (uint64_t r0 = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; r0 < P.n; r0 += step * kInsertU) {
     uint64_t k[kInsertU], s[kInsertU];
@@ -304,7 +304,9 @@ __global__ void __launch_bounds__(256) build_insert1_kernel(const __grid_constan
       any |= look[u];
     }
     int from[kInsertU] = {};
-    for (uint64_t t = 0; any && t < limit; ++t) {
+    uint32_t seen[kInsertU] = {};  // buckets full of other keys
+    bool failed = false;
+    while (any) {  // (every step settles a row or moves it on by a slot or a bucket)
       uint64_t w[kInsertU][4], x[kInsertU];
       int pos[kInsertU];
 #pragma unroll
@@ -333,17 +335,25 @@ __global__ void __launch_bounds__(256) build_insert1_kernel(const __grid_constan
           look[u] = false;
           continue;
         }
-        any = true;
         from[u] = pos[u] + 1;  // (taken by another key in the meantime)
         if (pos[u] >= 3) {
           from[u] = 0;
           s[u] = (s[u] + 4) & (P.T.cap - 1);
+          if (++seen[u] == limit) {
+            look[u] = false;
+            failed = true;
+            continue;
+          }
         }
+        any = true;
       }
     }
-    if (any) {
-      if (P.ovf) atomicExch(P.ovf, 1u);  // the table is too small: the host rebuilds it
-      else atomicOr(P.err, kDevSpillOverflow);
+    if (failed) {
+      if (P.ovf) {
+        atomicExch(P.ovf, 1u);  // the table is too small: the host rebuilds it
+        break;
+      }
+      atomicOr(P.err, kDevSpillOverflow);
     }
   }
   // One atomic per CTA: one per warp queues up at the word.
