@@ -531,11 +531,12 @@ constexpr int priv_rows() {  // rows per thread in flight (registers)
 // of the CTA calls it). A row that finds no place there stays for the next
 // flush, or goes to the partial-row list at the final one. CTAs start at
 // different slots, so they do not merge the same group at the same time.
+template <bool SSUM = false>
 __device__ __forceinline__ void priv_flush1(uint64_t* keys, const PrivT& T, const PrivK& A, const AggK& P, uint8_t* rep,
                                             uint16_t* rslot, unsigned* nrep, bool final,
                                             unsigned long long& inserted) {
   priv_fence();
-  priv_fold(T, A, rslot, *nrep, P.fkind, P.nfields);
+  priv_fold<SSUM>(T, A, rslot, *nrep, P.fkind, P.nfields);
   priv_fence();
   const int S = A.slots, W = P.row_words;
   const int rot = static_cast<int>((blockIdx.x * 97u) % static_cast<unsigned>(S + 2));
@@ -543,7 +544,7 @@ __device__ __forceinline__ void priv_flush1(uint64_t* keys, const PrivT& T, cons
     int sr = i + rot;
     if (sr >= S + 2) sr -= S + 2;
     rep[sr] = 0;
-    if (priv_load(T, A, 0, F_ROWS, sr) == 0) continue;
+    if (priv_load<SSUM>(T, A, 0, F_ROWS, sr) == 0) continue;
     const uint64_t k = sr < S ? keys[sr] : 0;
     uint64_t* dst = global_row1(P, sr != S + 1, k, key_hash1(k), inserted, P.probe_limit);
     if (dst) {
@@ -551,14 +552,14 @@ __device__ __forceinline__ void priv_flush1(uint64_t* keys, const PrivT& T, cons
       for (int f = 0; f < P.nfields; ++f) {
         if ((A.skip >> f) & 1u) continue;
         const uint8_t kind = P.fkind[f];
-        field_red<kRowGlobal>(dst + 1 + f, kind, priv_load(T, A, f, kind, sr));
+        field_red<kRowGlobal>(dst + 1 + f, kind, priv_load<SSUM>(T, A, f, kind, sr));
       }
     } else if (final) {
       const unsigned long long j = atomicAdd(P.counters + 1, 1ull);
       if (j < P.part_cap) {
         P.spill_parts[j * W] = k;
         for (int f = 0; f < P.nfields; ++f)
-          P.spill_parts[j * W + 1 + f] = ((A.skip >> f) & 1u) ? 0 : priv_load(T, A, f, P.fkind[f], sr);
+          P.spill_parts[j * W + 1 + f] = ((A.skip >> f) & 1u) ? 0 : priv_load<SSUM>(T, A, f, P.fkind[f], sr);
       } else {
         atomicOr(P.err, kDevSpillOverflow);
       }
@@ -567,14 +568,14 @@ __device__ __forceinline__ void priv_flush1(uint64_t* keys, const PrivT& T, cons
     }
     if (final) continue;
     for (int f = 0; f < P.nfields; ++f)
-      if (!((A.skip >> f) & 1u)) priv_clear(T, A, f, P.fkind[f], sr);
+      if (!((A.skip >> f) & 1u)) priv_clear<SSUM>(T, A, f, P.fkind[f], sr);
     if (sr < S) keys[sr] = 0;
   }
   if (threadIdx.x == 0) *nrep = 0;
   __syncthreads();
 }
 
-template <int NV, uint32_t SPEC>
+template <int NV, uint32_t SPEC, bool SSUM = false>
 __global__ void __launch_bounds__(1024) agg_private_kernel(const __grid_constant__ AggK P,
                                                            const __grid_constant__ PrivK A) {
   constexpr int kPrivU = priv_rows<NV>();
@@ -661,7 +662,7 @@ __global__ void __launch_bounds__(1024) agg_private_kernel(const __grid_constant
     for (int u = 0; u < kPrivU; ++u) {
       if (slot[u] >= 0) {
         const int id = rep[slot[u]];
-        priv_apply<SPEC, NV>(T, A, id ? S + 2 + (id - 1) * 32 + static_cast<int>(lane) : slot[u], P.fkind, P.fcol,
+        priv_apply<SPEC, NV, SSUM>(T, A, id ? S + 2 + (id - 1) * 32 + static_cast<int>(lane) : slot[u], P.fkind, P.fcol,
                              P.nfields, vv[u], vb[u]);
       }
     }
@@ -713,13 +714,13 @@ __global__ void __launch_bounds__(1024) agg_private_kernel(const __grid_constant
       if (wait > 0) {
         --wait;
       } else if (m > span * kPrivWindow / 4) {
-        priv_flush1(keys, T, A, P, rep, s_rslot, &s_nrep, false, inserted);
+        priv_flush1<SSUM>(keys, T, A, P, rep, s_rslot, &s_nrep, false, inserted);
         before = m;
         judge = 2;
       }
     }
   }
-  priv_flush1(keys, T, A, P, rep, s_rslot, &s_nrep, true, inserted);
+  priv_flush1<SSUM>(keys, T, A, P, rep, s_rslot, &s_nrep, true, inserted);
   // Occupancy accounting: one atomic per warp.
   for (int o = 16; o > 0; o >>= 1) inserted += __shfl_down_sync(0xffffffffu, inserted, o);
   if (lane == 0 && inserted) atomicAdd(P.counters + 2, inserted);
@@ -1987,9 +1988,11 @@ uint32_t AggState::null_field(int c) const {
 
 // Most slots of a private table (a power of two, at most 8192) that shared
 // memory holds beside the kernel's static variables.
-int AggState::priv_max_slots(uint32_t skip) const {
+int AggState::priv_max_slots(uint32_t skip, bool ssum) const {
   int slots = 64;
-  while (slots < 8192 && priv_layout(fkind.data(), nfields, slots * 2, skip, kPrivReps).bytes + 1024 <= ctx->smem_optin) slots *= 2;
+  while (slots < 8192 &&
+         priv_layout(fkind.data(), nfields, slots * 2, skip, kPrivReps, ssum).bytes + 1024 <= ctx->smem_optin)
+    slots *= 2;
   return slots;
 }
 
@@ -2002,27 +2005,39 @@ void AggState::launch_private1(const AggK& P0, uint64_t nrows) {
   void (*kern)(AggK, PrivK) = nullptr;
   const int nv = static_cast<int>(val_cols.size());
   const uint32_t spec = field_spec(P);
-  if (spec == kSpecIntF64) kern = agg_private_kernel<2, kSpecIntF64>;
-  else if (spec == kSpecIntF64Nulls) kern = agg_private_kernel<2, kSpecIntF64Nulls>;
-  else if (spec == kSpecF64) kern = agg_private_kernel<1, kSpecF64>;
-  else if (spec == kSpecF64Nulls) kern = agg_private_kernel<1, kSpecF64Nulls>;
-  else if (spec == kSpecCount) kern = agg_private_kernel<1, kSpecCount>;
-  else if (spec == kSpecIntSumF64Stats) kern = agg_private_kernel<2, kSpecIntSumF64Stats>;
-  else if (spec == kSpecIntSumF64StatsNulls) kern = agg_private_kernel<2, kSpecIntSumF64StatsNulls>;
-  else if (nv <= 1) kern = agg_private_kernel<1, kGenericSpec>;
-  else if (nv <= 2) kern = agg_private_kernel<2, kGenericSpec>;
-  else if (nv <= 4) kern = agg_private_kernel<4, kGenericSpec>;
-  else kern = agg_private_kernel<8, kGenericSpec>;
+  auto pick = [&](auto ssum) -> void (*)(AggK, PrivK) {
+    constexpr bool kS = decltype(ssum)::value;
+    if (spec == kSpecIntF64) return agg_private_kernel<2, kSpecIntF64, kS>;
+    if (spec == kSpecIntF64Nulls) return agg_private_kernel<2, kSpecIntF64Nulls, kS>;
+    if (spec == kSpecF64) return agg_private_kernel<1, kSpecF64, kS>;
+    if (spec == kSpecF64Nulls) return agg_private_kernel<1, kSpecF64Nulls, kS>;
+    if (spec == kSpecCount) return agg_private_kernel<1, kSpecCount>;
+    if (spec == kSpecIntSumF64Stats) return agg_private_kernel<2, kSpecIntSumF64Stats, kS>;
+    if (spec == kSpecIntSumF64StatsNulls) return agg_private_kernel<2, kSpecIntSumF64StatsNulls, kS>;
+    if (nv <= 1) return agg_private_kernel<1, kGenericSpec, kS>;
+    if (nv <= 2) return agg_private_kernel<2, kGenericSpec, kS>;
+    if (nv <= 4) return agg_private_kernel<4, kGenericSpec, kS>;
+    return agg_private_kernel<8, kGenericSpec, kS>;
+  };
+  // F64 sums in shared memory (qeg_privagg.cuh) when the estimate puts the
+  // global table beyond half of L2, as for the partitioned passes. A window's
+  // groups come and go, so its tables hold most rows whatever the estimate.
+  // (512M Zipf(1.1) rows over 64M keys, 25M groups: 32.5 ms with the sums at L2,
+  // 30.7 here; 64M rows over 50k pairs of keys the other way round, 3.0 and 6.5.)
+  const bool ssum = bucket_width == 0 && P.nhot == 0 && spec != kSpecCount &&
+                    std::find(fkind.begin(), fkind.end(), F_SUMF) != fkind.end() &&
+                    est_groups / kTargetLoad * row_words * 8.0 >= static_cast<double>(kPartMinTableBytes);
+  kern = ssum ? pick(std::true_type{}) : pick(std::false_type{});
   const int block = block_threads();
   uint32_t skip = 0;
   for (int c = 0; c < nv; ++c)
     if (P.val[c].all_valid) skip |= null_field(c);
-  const int most = std::min(smem_slots, priv_max_slots(skip));
+  const int most = std::min(smem_slots, priv_max_slots(skip, ssum));
   // A few thousand rows per CTA at least, so the flush stays small. A CTA of
   // fewer than 1024 threads shares its SM with others as far as their tables
   // (and the partial-row list) allow: 64M Zipf(1.1) rows over 100k keys, 1024
   // slots, 256 threads 4.6 ms with one CTA per SM, 1.8 now.
-  const size_t full = priv_layout(fkind.data(), nfields, most, skip, kPrivReps).bytes;
+  const size_t full = priv_layout(fkind.data(), nfields, most, skip, kPrivReps, ssum).bytes;
   const uint64_t per_sm = std::max<uint64_t>(
       1, std::min<uint64_t>({static_cast<uint64_t>(1024 / block),
                              static_cast<uint64_t>(blocks_per_sm(reinterpret_cast<const void*>(kern), block, full)),
@@ -2033,7 +2048,7 @@ void AggState::launch_private1(const AggK& P0, uint64_t nrows) {
   while (slots < most && static_cast<uint64_t>(slots) * grid < nrows) slots *= 2;
   if (P.nhot > 0) slots = smem_slots;  // preloaded
   slots = std::min(slots, most);
-  PrivK A = priv_layout(fkind.data(), nfields, slots, skip, kPrivReps);
+  PrivK A = priv_layout(fkind.data(), nfields, slots, skip, kPrivReps, ssum);
   priv_sums_for(A, grid);
   require(blocks_per_sm(reinterpret_cast<const void*>(kern), block, A.bytes) > 0,
           "aggregate kernel does not fit on an SM with this configuration");

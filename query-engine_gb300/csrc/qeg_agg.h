@@ -181,7 +181,7 @@ struct AggState {
   size_t smem_bytes(int block) const;
   int block_threads() const;
   uint32_t null_field(int c) const;
-  int priv_max_slots(uint32_t skip) const;
+  int priv_max_slots(uint32_t skip, bool ssum = false) const;
   void set_field_columns(AggK& P) const;
   uint32_t field_spec(const AggK& P) const;  // qeg_warpagg.cuh field-set code
   void launch(const AggK& P, uint64_t nrows);

@@ -21,6 +21,10 @@ namespace qeg {
 // throughput whatever the spread, and no time of the SM. 64-bit integer sums
 // are added as two 32-bit halves with a carry: the 64-bit shared add is such
 // a loop too (352 clocks over 8 words, 32-bit adds take 3).
+// Where most rows miss the private tables anyway and update a global table far
+// beyond L2, those reductions are what bounds the launch (about 50 G/s there),
+// and the hits' sums must not add to them: SSUM tables keep the F64 sums in
+// shared memory, in fewer slots.
 // ---------------------------------------------------------------------------
 constexpr int kPrivReps = 16;
 
@@ -38,8 +42,8 @@ struct PrivK {
 // Lays out a table of `slots` slots for the given fields. `skip` has a bit for
 // every field that no row of the launch changes (NULL counts of columns
 // without NULLs): these have no array; `reps` is the number of slots that may
-// have replica rows.
-inline PrivK priv_layout(const uint8_t* fkind, int nfields, int slots, uint32_t skip, int reps) {
+// have replica rows; `ssum` puts F64 sums into shared memory too.
+inline PrivK priv_layout(const uint8_t* fkind, int nfields, int slots, uint32_t skip, int reps, bool ssum = false) {
   PrivK A{};
   A.slots = slots;
   A.rows = slots + 2 + 32 * reps;
@@ -47,12 +51,12 @@ inline PrivK priv_layout(const uint8_t* fkind, int nfields, int slots, uint32_t 
   for (int pass = 0; pass < 2; ++pass)  // 8-byte fields first
     for (int f = 0; f < nfields; ++f) {
       const uint32_t size = fkind[f] <= F_NULLS ? 4 : 8;
-      if (fkind[f] == F_SUMF || (size == 4) != (pass == 1) || ((skip >> f) & 1u)) continue;
+      if ((fkind[f] == F_SUMF && !ssum) || (size == 4) != (pass == 1) || ((skip >> f) & 1u)) continue;
       A.foff[f] = at;
       at += size * static_cast<uint32_t>(A.rows);
     }
   for (int f = 0; f < nfields; ++f)
-    if (fkind[f] == F_SUMF) {
+    if (fkind[f] == F_SUMF && !ssum) {
       A.foff[f] = A.sum_bytes;
       A.sum_bytes += 8 * static_cast<uint32_t>(A.rows);
     }
@@ -112,16 +116,19 @@ __device__ __forceinline__ int hot_slot(const uint64_t* keys, int slots, uint64_
 }
 
 // Merges one contribution x into field f (of kind `kind`) of private row `row`.
+template <bool SSUM = false>
 __device__ __forceinline__ void priv_red(const PrivT& T, const PrivK& A, int f, uint8_t kind, int row, uint64_t x) {
   if (!x) return;  // zero is the identity of every field
-  if (kind == F_SUMF) {
+  if (kind == F_SUMF && !SSUM) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(T.sums + A.foff[f] + static_cast<uint32_t>(row) * 8u),
                  "d"(__longlong_as_double(static_cast<long long>(x)))
                  : "memory");
     return;
   }
   const uint32_t a = T.base + A.foff[f] + static_cast<uint32_t>(row) * (kind <= F_NULLS ? 4u : 8u);
-  if (kind <= F_NULLS) {
+  if (kind == F_SUMF) {
+    asm volatile("red.shared.add.f64 [%0], %1;" ::"r"(a), "d"(__longlong_as_double(static_cast<long long>(x))) : "memory");
+  } else if (kind <= F_NULLS) {
     asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(static_cast<uint32_t>(x)) : "memory");
   } else if (kind == F_SUMI) {
     const uint32_t lo = static_cast<uint32_t>(x);
@@ -134,9 +141,10 @@ __device__ __forceinline__ void priv_red(const PrivT& T, const PrivK& A, int f, 
   }
 }
 
+template <bool SSUM = false>
 __device__ __forceinline__ uint64_t priv_load(const PrivT& T, const PrivK& A, int f, uint8_t kind, int row) {
   uint64_t v;
-  if (kind == F_SUMF) {  // from L2, where the reductions land
+  if (kind == F_SUMF && !SSUM) {  // from L2, where the reductions land
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];"
                  : "=l"(v)
                  : "l"(T.sums + A.foff[f] + static_cast<uint32_t>(row) * 8u)
@@ -153,8 +161,9 @@ __device__ __forceinline__ uint64_t priv_load(const PrivT& T, const PrivK& A, in
   return v;
 }
 
+template <bool SSUM = false>
 __device__ __forceinline__ void priv_clear(const PrivT& T, const PrivK& A, int f, uint8_t kind, int row) {
-  if (kind == F_SUMF) {
+  if (kind == F_SUMF && !SSUM) {
     *reinterpret_cast<volatile uint64_t*>(T.sums + A.foff[f] + static_cast<uint32_t>(row) * 8u) = 0;
     return;
   }
@@ -175,17 +184,17 @@ __device__ __forceinline__ PrivT priv_init(uint64_t* sm, const PrivK& A) {
 }
 
 // Adds one input row to private row `row`.
-template <uint32_t SPEC, int NV>
+template <uint32_t SPEC, int NV, bool SSUM = false>
 __device__ __forceinline__ void priv_apply(const PrivT& T, const PrivK& A, int row, const uint8_t* fkind,
                                            const uint8_t* fcol, int nfields, const bool (&vv)[kMaxVals],
                                            const uint64_t (&vb)[kMaxVals]) {
-  priv_red(T, A, 0, F_ROWS, row, 1);
+  priv_red<SSUM>(T, A, 0, F_ROWS, row, 1);
   if constexpr (SPEC != kGenericSpec) {
 #pragma unroll
     for (int i = 1; i <= spec_n(SPEC); ++i) {
       const uint8_t kind = static_cast<uint8_t>(spec_kind(SPEC, i));
       const int col = spec_col(SPEC, i) < NV ? spec_col(SPEC, i) : 0;
-      if (kind != 0) priv_red(T, A, i, kind, row, field_contrib(kind, vv[col], vb[col]));
+      if (kind != 0) priv_red<SSUM>(T, A, i, kind, row, field_contrib(kind, vv[col], vb[col]));
     }
   } else {
 #pragma unroll 1
@@ -201,7 +210,7 @@ __device__ __forceinline__ void priv_apply(const PrivT& T, const PrivK& A, int r
         }
       }
       const uint64_t x = field_contrib(kind, v, b);
-      if (x) priv_red(T, A, i, kind, row, x);
+      if (x) priv_red<SSUM>(T, A, i, kind, row, x);
     }
   }
 }
@@ -258,6 +267,7 @@ __device__ __forceinline__ void priv_promote(int slot, uint8_t* rep, uint16_t* r
 // Adds the replica rows to their slots' rows and clears them. All threads of
 // the CTA call it, after a barrier; priv_fence() must follow before the slots'
 // rows are read.
+template <bool SSUM = false>
 __device__ __forceinline__ void priv_fold(const PrivT& T, const PrivK& A, const uint16_t* rslot, unsigned nrep,
                                           const uint8_t* fkind, int nfields) {
   const int n = static_cast<int>(min(nrep, static_cast<unsigned>(kPrivReps))) * 32;
@@ -266,8 +276,8 @@ __device__ __forceinline__ void priv_fold(const PrivT& T, const PrivK& A, const 
     for (int f = 0; f < nfields; ++f) {
       if ((A.skip >> f) & 1u) continue;
       const uint8_t kind = fkind[f];
-      priv_red(T, A, f, kind, slot, priv_load(T, A, f, kind, row));
-      priv_clear(T, A, f, kind, row);
+      priv_red<SSUM>(T, A, f, kind, slot, priv_load<SSUM>(T, A, f, kind, row));
+      priv_clear<SSUM>(T, A, f, kind, row);
     }
   }
 }
