@@ -1904,11 +1904,7 @@ AggK AggState::kparams(const std::vector<StagedCol>& staged, const uint32_t* sel
   P.nkeys = static_cast<int>(keys.size());
   for (size_t j = 0; j < keys.size(); ++j) P.key[j] = key_col(staged, j);
   P.nvals = static_cast<int>(val_cols.size());
-  for (size_t c = 0; c < val_cols.size(); ++c) {
-    P.val[c] = staged[val_cols[c]].dev;
-    P.cfirst[c] = static_cast<uint8_t>(cfirst[c]);
-    P.cnf[c] = static_cast<uint8_t>(cnf[c]);
-  }
+  for (size_t c = 0; c < val_cols.size(); ++c) P.val[c] = staged[val_cols[c]].dev;
   P.nfields = nfields;
   for (int f = 0; f < nfields; ++f) P.fkind[f] = fkind[f];
   set_field_columns(P);
@@ -1962,9 +1958,9 @@ void AggState::set_field_columns(AggK& P) const {
     for (int k = 0; k < cnf[c]; ++k) P.fcol[cfirst[c] + k] = static_cast<uint8_t>(c);
 }
 
-// 1024-thread CTAs for the single-key private-table strategy (one CTA per SM
-// with a 2048-slot table: measured 1.28x faster than 512 threads on a 512M-row
-// Zipf(1.1) GROUP BY), 512 otherwise.
+// 1024-thread CTAs for the single-key private-table strategy (64M Zipf(1.1) rows
+// over 100k keys, the largest tables: 1.72 ms, 2.82 with 512 threads; 1024
+// slots: 1.68 and 1.71), 512 otherwise.
 int AggState::block_threads() const {
   if (cfg.block_threads > 0) return cfg.block_threads;
   return (mode == 1 && (strategy == QEG_AGG_SMEM || strategy == QEG_AGG_PARTITIONED)) ? 1024 : 512;
@@ -2166,10 +2162,6 @@ AggK AggState::kparams_base() const {
   AggK P{};
   P.nkeys = static_cast<int>(keys.size());
   P.nvals = static_cast<int>(val_cols.size());
-  for (size_t c = 0; c < val_cols.size(); ++c) {
-    P.cfirst[c] = static_cast<uint8_t>(cfirst[c]);
-    P.cnf[c] = static_cast<uint8_t>(cnf[c]);
-  }
   P.nfields = nfields;
   for (int f = 0; f < nfields; ++f) P.fkind[f] = fkind[f];
   set_field_columns(P);
@@ -2296,12 +2288,11 @@ void AggState::first_consume(const std::vector<StagedCol>& staged, uint64_t nrow
     want = static_cast<uint64_t>(std::max(kEstimateHeadroom * est_groups / kTargetLoad, 1024.0));
   }
   // Partitioned strategy: asked for, or chosen when the estimate puts the
-  // global table far beyond L2 (every row would be a random DRAM round trip
-  // there) and the key column has no heavy head. With a heavy head the
-  // CTA-private tables absorb most rows and the rest reach the global table:
-  // on GB300, 512M Zipf(1.1) rows over 64M keys take 28.0 ms that way against
-  // 31.3 ms partitioned. Its global table only takes the private tables'
-  // flushes, so it starts small.
+  // global table far beyond L2, where every row that misses the private tables
+  // costs its reductions on random lines: 512M Zipf(1.1) rows over 64M keys
+  // take 14.1 ms partitioned and 30.7 ms through the private tables, 48M
+  // uniform rows over 10M keys 3.3 ms and (global table alone) 8.2. Its global
+  // table only takes the private tables' flushes, so it starts small.
   bool go_part = false;
   const double part_most = kPartMaxFill * part_table_slots(0) * static_cast<double>(1u << kPartMaxBits);
   if (mode == 1 && part_eligible(staged)) {

@@ -37,8 +37,6 @@ struct AggK {
   int nkeys, nvals, nfields, row_words;
   uint8_t fkind[kMaxFields];
   uint8_t fcol[kMaxFields];  // value column of each field (field 0: rows)
-  uint8_t cfirst[kMaxVals];
-  uint8_t cnf[kMaxVals];
   uint64_t* table;
   uint64_t cap;  // slots; a key's first slot is mulhi(hash, cap)
   const uint32_t* sel;

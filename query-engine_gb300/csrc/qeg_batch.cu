@@ -386,7 +386,7 @@ struct BatchState {
   std::vector<float> hot;
   std::vector<int32_t> slots;   // per query: CTA-private table slots (0 = global table only)
   std::vector<uint64_t> chunk;  // per query: rows per work item
-  std::vector<int32_t> peer;    // per query: warp peer aggregation
+  std::vector<int32_t> peer;    // per query: many rows of a warp share a group
   StagedCol key, val;
   uint32_t nq = 0;
   int block = 512;

@@ -3930,10 +3930,9 @@ qeg_status qeg_join_probe_count_sum(qeg_join* j, const qeg_column* probe_key, co
       }
       const bool k8 = type_width(kt) == 8, v8 = type_width(vt) == 8, dense = st.strategy == QEG_JOIN_DENSE;
       // Hashed tables: QEG_JOIN_SWEEPS=n > 1 probes in n sweeps over windows of
-      // the table (opt-in: on GB300 the 16M-key table's 64 MB windows reach a
-      // 73% L2 hit rate and each sweep re-reads the 2 GB key column, so 256M
-      // probes take 5.8 ms in 2 sweeps and 6.8 ms in 4, against 3.8 ms for
-      // the direct probe below).
+      // the table (opt-in: each sweep re-reads the 2 GB key column, so 256M
+      // probes of a 16M-key table take 3.8 ms in 2 sweeps and 4.4 ms in 4,
+      // against 3.5 ms for the direct probe below).
       if (st.strategy == QEG_JOIN_HASH && lean_sizes_ok(n)) {
         uint64_t sweeps = 1;
         if (const char* e = getenv("QEG_JOIN_SWEEPS")) sweeps = std::max(1, atoi(e));
@@ -3972,8 +3971,8 @@ qeg_status qeg_join_probe_count_sum(qeg_join* j, const qeg_column* probe_key, co
       };
       // The TMA-staged kernel (one block of kTmaThreads per SM, a kStages ring
       // of shared-memory tiles) is opt-in (QEG_SINK_TMA=1): on GB300 the
-      // register-pipelined kernel reads the probe side faster (1.05 ms against
-      // 1.38 ms for 256M dense-table probes; 5.9 against 10.4 ms hashed).
+      // register-pipelined kernel reads the probe side faster (0.88 ms against
+      // 1.36 ms for 256M dense-table probes; 4.7 against 6.2 ms hashed).
       auto al16 = [](const void* p) { return p == nullptr || reinterpret_cast<uintptr_t>(p) % 16 == 0; };
       const char* tma_env = getenv("QEG_SINK_TMA");
       // The lean kernel is the default. Dense table with unique build keys: 32
@@ -3981,11 +3980,11 @@ qeg_status qeg_join_probe_count_sum(qeg_join* j, const qeg_column* probe_key, co
       // probe side at 96% of the measured HBM copy bandwidth on GB300. The
       // same kernel with the next tile's loads issued early, or at 6 CTAs per
       // SM, measured 88-96%; the 64-register pipelined kernel with 128-row
-      // warp tiles (4 CTAs per SM) 73%, and 81% at 6 CTAs per SM (40
+      // warp tiles (4 CTAs per SM) 72%, and 81% at 6 CTAs per SM (40
       // registers, spilling). Hashed tables: 40 registers at 6 CTAs per SM
-      // (the probe loop spills 76 B at 32 registers) probe 256M rows against
-      // 16M unique keys in 4.4 ms, against 5.5 ms at 8 CTAs and 5.6 ms for the
-      // pipelined kernel. QEG_SINK_PIPE=0|1|2|4|8 picks one for measurement.
+      // probe 256M rows against 16M unique keys in 3.5 ms, 4.7 ms at 8 CTAs
+      // (spills at 32 registers), 3.1 at 4 CTAs and 4.7 for the pipelined
+      // kernel. QEG_SINK_PIPE=0|1|2|4|8 picks one for measurement.
       const bool lean_ok = n / 64 < (uint64_t{1} << 31);
       const bool bloomed = st.bloom.get() != nullptr;
       // CTAs per SM of the hashed sink (QEG_SINK_HASH_MINB=4|6|8, for measurement).

@@ -1,5 +1,6 @@
-// qeg_warpagg.cuh -- warp-level peer aggregation shared by the GROUP BY
-// kernels (qeg_agg.cu, qeg_batch.cu).
+// qeg_warpagg.cuh -- warp-level peer aggregation (qeg_agg.cu's kernels without
+// private tables and its composite ones, qeg_pipeline.cu), and the aggregate
+// fields' operations and field-set codes that every GROUP BY kernel uses.
 #pragma once
 
 #include "qeg_agg.h"
