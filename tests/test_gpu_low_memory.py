@@ -57,15 +57,18 @@ def test_fetch_without_room_for_packed_rows(ctx, device, join_type):
 
 
 @pytest.mark.parametrize("hot_keys", [0, 64])
-def test_partitioned_groupby_without_room_for_its_pool(ctx, hot_keys):
-    # The pool would take 16 bytes a row, 128 MB; everything else fits.
+@pytest.mark.parametrize("expected,mb", [(100_000, 112), (12_000_000, 288)])
+def test_partitioned_groupby_without_room_for_its_pool(ctx, hot_keys, expected, mb):
+    # The pool would take 16 bytes a row, up to 128 MB; the rest fits. Or the
+    # pool fits and the tail rows, 16 bytes for 1.25 of the expected groups, do
+    # not (240 MB).
     n, dom = 1 << 23, 100_000
     g = torch.Generator(device="cuda").manual_seed(4)
     a = qeg.Aggregate(ctx, [O.I64], [0], [(O.COUNT_STAR, 0)],
-                      qeg.agg_config(strategy=qeg.AGG_PARTITIONED, hot_keys=hot_keys, expected_groups=dom))
+                      qeg.agg_config(strategy=qeg.AGG_PARTITIONED, hot_keys=hot_keys, expected_groups=expected))
     try:
         want = torch.zeros(dom, dtype=torch.int64, device="cuda")
-        for limit in (112 << 20, 112 << 20, 0):  # twice without the pool, then with it
+        for limit in (mb << 20, mb << 20, 0):  # twice without that memory, then with it
             key = (dom ** torch.rand(n, device="cuda", dtype=torch.float64, generator=g)).long() - 1
             want += torch.bincount(key, minlength=dom)
             torch.cuda.synchronize()
