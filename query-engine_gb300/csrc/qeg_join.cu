@@ -3036,6 +3036,7 @@ void JoinState::asof_sort() {
   const bool in_a = R.lo == A.lo;
   ats = in_a ? std::move(a_lo) : std::move(b_lo);
   arow = in_a ? std::move(a_val) : std::move(b_val);
+  if (!amerge || aprobe_unsorted) bslot.release();  // (the merge's alone from here on)
   check_device_error(ctx);  // synchronises the stream
 }
 
@@ -3350,8 +3351,15 @@ bool JoinState::asof_merge(uint64_t n) {
   const int per_sm = std::max(1, blocks_per_sm(reinterpret_cast<const void*>(merge), 256, smem));
   const unsigned slices = static_cast<unsigned>(std::max<uint64_t>(
       1, std::min<uint64_t>((n + nbuild) / kAsofMinSlice, static_cast<uint64_t>(ctx->sms) * per_sm)));
-  DevBuf split((slices + 1) * 8, ctx->stream), heads(static_cast<uint64_t>(slices) * aslots * 4, ctx->stream),
-      flags(8, ctx->stream);
+  DevBuf split, heads, flags;
+  try {
+    split.alloc((slices + 1) * 8, ctx->stream);
+    heads.alloc(static_cast<uint64_t>(slices) * aslots * 4, ctx->stream);
+    flags.alloc(8, ctx->stream);
+  } catch (const Error& e) {  // the search needs none of it
+    if (e.code != QEG_ERR_OOM) throw;
+    return false;
+  }
   P.split = split.get<uint2>();
   P.heads = heads.get<uint32_t>();
   P.unsorted = flags.get<uint32_t>();

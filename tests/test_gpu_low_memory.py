@@ -1,5 +1,6 @@
 """Calls that take memory for speed alone answer without it: joins whose build
-rows cannot be packed side by side, partitioned GROUP BYs without their pool."""
+rows cannot be packed side by side, partitioned GROUP BYs without their pool, as-of joins without the
+merge's scratch."""
 import numpy as np
 import pytest
 import torch
@@ -7,6 +8,7 @@ import torch
 import oracle as O
 import qeg
 from mempool import limited_pool
+from test_gpu_asof_merge import expected
 from util import to_gpu
 
 pytestmark = pytest.mark.gpu
@@ -86,3 +88,29 @@ def test_partitioned_groupby_without_room_for_its_pool(ctx, hot_keys, expected, 
         assert np.array_equal(got, want.cpu().numpy())
     finally:
         a.close()
+
+
+def test_asof_without_room_for_the_merge(ctx):
+    # 16,000 slots and as many slices as fill the GPU take about 30 MB; the probe
+    # batch's own buffers 8 MB. The build side was sorted by an earlier batch.
+    rng = np.random.default_rng(6)
+    nb, n, nsym = 100_000, 2_000_000, 16_000
+    bts, pts = np.sort(rng.integers(0, 1 << 30, nb)), np.sort(rng.integers(0, 1 << 30, n))
+    bkey, pkey = rng.integers(0, nsym, nb).astype(np.int32), rng.integers(0, nsym, n).astype(np.int32)
+    exp = expected(bkey.astype(np.int64), bts, pkey.astype(np.int64), pts, None)
+    j = qeg.AsofJoin(ctx, [O.I32, O.TS], [O.I32, O.TS, O.I64], [0], [0], 1, 1, O.LEFT)
+    try:
+        j.build([qeg.Col(bkey), qeg.Col(bts, None, qeg.TS), qeg.Col(np.arange(nb))])
+        j.build_finish()
+        assert j.probe([qeg.Col(pkey[:50_000]), qeg.Col(pts[:50_000], None, qeg.TS)]) == 50_000  # (fewer rows: the search)
+        cols = [to_gpu(O.TCol(O.I32, pkey), device=True), to_gpu(O.TCol(O.TS, pts), device=True)]
+        with limited_pool(32 << 20):
+            assert j.probe(cols) == n
+            ctx.synchronize()
+        v, ok = j.fetch()[-1]
+        assert np.array_equal(np.where(ok, v, -1), exp)
+        assert j.probe(cols) == n  # with memory again
+        v, ok = j.fetch()[-1]
+        assert np.array_equal(np.where(ok, v, -1), exp)
+    finally:
+        j.close()
